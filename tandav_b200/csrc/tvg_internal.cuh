@@ -180,6 +180,7 @@ struct tvg_context {
 
 	// Ewald tables (Float, divided by box^2) and raw FP64
 	void *ewald_f[4] = { nullptr, nullptr, nullptr, nullptr };
+	void *ewald_xyz = nullptr;         // the plain walk's interleaved Ewald tables (32 B per entry)
 	double *ewald_raw = nullptr;
 	float *ewald32 = nullptr;          // FP32 copy for the group form (FP64 builds)
 	float *ewald_ext = nullptr;        // (Tx, Ty, Tz, 0) on 68^3 points, x = 0.5 i / 64, i = -1..66
