@@ -357,7 +357,8 @@ int tvg_walk_quad_interactions(tvg_context *ctx, double *quad_interactions);
  * acc_direct and acc_tree (3 * n_targets doubles, x block then y then z) hold
  * the direct sum and the resident Grav_Acc; err[4] = rms, 99th percentile
  * (nearest rank), mean and max of |a_tree - a_direct| / |a_direct|.
- * Allocates and frees its own device scratch. */
+ * Keeps up to 64 MB of device scratch in the context; a larger call allocates
+ * and frees its own. */
 int tvg_forcetest(tvg_context *ctx, uint32_t parts, int64_t n_targets, const int64_t *targets,
                   double *acc_direct, double *acc_tree, double *err);
 

@@ -248,6 +248,10 @@ struct tvg_context {
 	tvg_graph_entry *graphs[2] = { nullptr, nullptr };
 	uint64_t graph_warm_key = 0;
 
+	// tvg_forcetest's device memory (at most 64 MB kept)
+	void *ft_ws = nullptr;
+	size_t ft_bytes = 0;
+
 	// timings
 	cudaEvent_t ev[16];
 	double phase_ms[8] = { 0 };

@@ -652,9 +652,9 @@ __device__ void walk_ewald(const PlainCtx<F> &c, const Lanes<S> &l, bool have, c
 }
 
 // A warp walks together when its targets lie within this many particles of
-// the order. Measured, ms together / lane by lane, every 16th particle active:
-// halo of 400,000, FP64: 7.4 / 12.6; box of 50^3, FP32 gravity: 44 / 76. Every
-// 64th: lane by lane 16.4 against 14.1 ms of the old walk's for 6250 targets.
+// the order. Walked together, every 8th particle of a 50^3 box (FP32 gravity)
+// takes 16 ms against 80 ms of the walk per thread; lane by lane, every 64th
+// takes 21 against 80 ms, and of a halo of 400,000 (FP64) 2.1 against 14 ms.
 #ifndef PLAIN_SPREAD
 #define PLAIN_SPREAD 512
 #endif

@@ -119,3 +119,26 @@ def test_forcetest_error_statistics():
     assert err["mean"] == pytest.approx(e.mean(), rel=1e-12)
     assert err["max"] == es[-1]
     assert err["rms"] < 5e-2
+
+
+@pytest.mark.parametrize("box", [1000.0, 0.0])
+@pytest.mark.parametrize("n", [1, 23, 129, 3001])
+def test_forcetest_any_number_of_targets(box, n):
+    """How the targets are dealt over threads and blocks follows from their
+    number (powers of two up to 128 share a block's sources, from four per SM
+    on a block sums k-space for four): every target's direct sum must be the
+    one it has among all targets. The sums' order differs, so FP64 round-off of
+    n terms and 28,000 waves, well below 1e-10 of the largest force."""
+    p = ics.random_box(max(n, 2), box=1000.0, seed=n, clumps=3)
+    pos, mass = p.pos[:, :n], p.mass[:n]
+    with G.GravityContext(4096, float_bytes=8, periodic=box > 0, boxsize=box, softening=p.softening) as ctx:
+        ctx.upload(pos, mass)
+        full, _, _ = ctx.forcetest(np.arange(n))
+        scale = np.abs(full).max() + 1e-30
+        for nt in (1, 2, 3, 64, 65, 127, 128, 129, 591, 593):
+            if nt > n:
+                continue
+            t = np.random.default_rng(nt).choice(n, nt, replace=False)
+            ad, at, _ = ctx.forcetest(t)
+            assert np.abs(ad - full[:, t]).max() < 1e-10 * scale, nt
+            assert not at.any()
