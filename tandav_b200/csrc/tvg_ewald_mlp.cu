@@ -20,9 +20,9 @@
 // targets T(x) by the Ewald sum of the table generator (tvg_ewald_sum.cuh)
 // minus the analytic part; the normal equations of the cubic fit summed in
 // FP64 (fixed-order block sums) and solved on the host (Cholesky); then the
-// network's FP32 minibatch mean-square loss on the normalised rest: one
-// thread per sample runs forward and backward, gradients are summed over the
-// warp by shuffles into one slot per warp, then over the slots in fixed order
+// network's FP32 minibatch mean-square loss on the normalised rest: tiles of 64
+// samples run forward and backward in shared memory, the gradients summed as
+// matrix products into one slot per block, then over the slots in fixed order
 // (deterministic), then Adam.
 //
 // Inference: BF16 weights (rounded once after training), FP32 arithmetic and
@@ -32,6 +32,7 @@
 // the caller gives.
 #include <math.h>
 
+#include <algorithm>
 #include <cmath>
 #include <stdlib.h>
 
@@ -138,105 +139,224 @@ __device__ __forceinline__ float warp_sum(float v)
 	return v;
 }
 
-// the warp's sum of v for parameter e lands in slot[e] (lane e % 32 writes)
-__device__ __forceinline__ void put(float *slot, int e, float v)
-{
-	const float s = warp_sum(v);
-	if ((threadIdx.x & 31) == (e & 31)) slot[e] = s;
-}
+// Forward and backward of tiles of MT samples, gradients summed over a block's
+// tiles in registers and written to the block's slot. Per sample the network is
+// three 64 x 64 products (W2 a1, W2^T dz2 and the outer product dz2 a1^T), FP32 FMA
+// bound: two threads share a sample (32 neurons each) for the first two, and
+// the outer products of a tile are one 64 x 64 x MT product with an 8 x 4 tile of
+// dW2 a thread, so that a weight gradient costs one FMA a sample (a warp's
+// butterfly sum of every parameter took 10 instructions: 123 us for 16,384
+// samples, 26 us now). Samples past n contribute zero.
+#define MT 64
+#define MT_THREADS 128
+#define MT_LD 68                // row stride: 16-byte rows, conflict-free by quarter warps
+struct MlpTile {
+	float w2[MLP_H * MLP_H];
+	float a1[MT * MT_LD], a2[MT * MT_LD], dz2[MT * MT_LD], dz1[MT * MT_LD];
+	float w1[3 * MLP_H], b1[MLP_H], b2[MLP_H], w3[3 * MLP_H], b3[4];
+	float v[MT][4], dy[MT][4], out[2][MT][4];
+};
 
-// forward + backward of one sample per thread; per-warp gradient slots and
-// per-warp loss sums. Samples past n contribute zero.
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(MT_THREADS)
 k_mlp_grad(int64_t n, const float *__restrict__ x, const float *__restrict__ y,
            const float *__restrict__ prm, float inv_norm, float *slots, float *loss_slots)
 {
-	__shared__ float P[MLP_NPARAM];
-	for (int e = threadIdx.x; e < MLP_NPARAM; e += blockDim.x) P[e] = prm[e];
-	__syncthreads();
-	const float *W1 = P + MLP_W1, *B1 = P + MLP_B1, *W2 = P + MLP_W2, *B2 = P + MLP_B2,
-	            *W3 = P + MLP_W3, *B3 = P + MLP_B3;
-	const int64_t s = blockIdx.x * (int64_t) blockDim.x + threadIdx.x;
-	const bool have = s < n;
-	const int64_t gw = s >> 5;
-	float *slot = slots + gw * MLP_NNET;
-	float v[3] = { 0.f, 0.f, 0.f }, t[3] = { 0.f, 0.f, 0.f };
-	if (have) {
+	extern __shared__ __align__(16) unsigned char mlp_smem[];
+	MlpTile &T = *(MlpTile *) mlp_smem;
+	const int tid = threadIdx.x, s = tid & (MT - 1), half = tid / MT, j0 = half * (MLP_H / 2);
+	for (int e = tid; e < MLP_H * MLP_H; e += MT_THREADS) T.w2[e] = prm[MLP_W2 + e];
+	for (int e = tid; e < 3 * MLP_H; e += MT_THREADS) {
+		T.w1[e] = prm[MLP_W1 + e];
+		T.w3[e] = prm[MLP_W3 + e];
+	}
+	if (tid < MLP_H) {
+		T.b1[tid] = prm[MLP_B1 + tid];
+		T.b2[tid] = prm[MLP_B2 + tid];
+	}
+	if (tid < 3) T.b3[tid] = prm[MLP_B3 + tid];
+	// this thread's parameters: an 8 x 4 tile of dW2; of neuron `s` of layer 2
+	// (half 0) or 1 (half 1) the bias and three weights; db3 of component tid
+	const int tj = 8 * (tid / 16), ti = 4 * (tid % 16);
+	float g2[8][4], gs[4] = { 0.f, 0.f, 0.f, 0.f }, g3 = 0.f, loss = 0.f;
+#pragma unroll
+	for (int a = 0; a < 8; a++)
+#pragma unroll
+		for (int b = 0; b < 4; b++) g2[a][b] = 0.f;
+	const int64_t ntile = (n + MT - 1) / MT;
+	for (int64_t tile = blockIdx.x; tile < ntile; tile += gridDim.x) {
+		const int64_t q = tile * MT + s;
+		const bool have = q < n;
+		float v[3], t[3];
+#pragma unroll
 		for (int d = 0; d < 3; d++) {
-			v[d] = 4.f * x[3 * s + d] - 1.f;
-			t[d] = y[3 * s + d];
+			v[d] = have ? 4.f * x[3 * q + d] - 1.f : 0.f;
+			t[d] = have ? y[3 * q + d] : 0.f;
 		}
-	}
-	float a1[MLP_H];
+		__syncthreads();          // the weights, and the previous tile's last readers
+		if (half == 0)
 #pragma unroll
-	for (int j = 0; j < MLP_H; j++)
-		a1[j] = tanhf(B1[j] + W1[3 * j] * v[0] + W1[3 * j + 1] * v[1] + W1[3 * j + 2] * v[2]);
-	float out[3] = { B3[0], B3[1], B3[2] };
-	for (int j = 0; j < MLP_H; j++) {
-		float z = B2[j];
+			for (int d = 0; d < 3; d++) T.v[s][d] = v[d];
+#pragma unroll 8
+		for (int j = j0; j < j0 + MLP_H / 2; j += 4) {
+			float a[4];
 #pragma unroll
-		for (int i = 0; i < MLP_H; i++) z = fmaf(W2[MLP_H * j + i], a1[i], z);
-		const float a2 = tanhf(z);
-		out[0] = fmaf(W3[j], a2, out[0]);
-		out[1] = fmaf(W3[MLP_H + j], a2, out[1]);
-		out[2] = fmaf(W3[2 * MLP_H + j], a2, out[2]);
-	}
-	float dy[3], l = 0.f;
-	for (int d = 0; d < 3; d++) {
-		const float r = have ? out[d] - t[d] : 0.f;
-		l += r * r;
-		dy[d] = 2.f * r * inv_norm;
-	}
-	l = warp_sum(l);
-	if ((threadIdx.x & 31) == 0) loss_slots[gw] = l;
-	put(slot, MLP_B3 + 0, dy[0]);
-	put(slot, MLP_B3 + 1, dy[1]);
-	put(slot, MLP_B3 + 2, dy[2]);
-	float dh1[MLP_H];
-#pragma unroll
-	for (int i = 0; i < MLP_H; i++) dh1[i] = 0.f;
-	for (int j = 0; j < MLP_H; j++) {
-		float z = B2[j];
-#pragma unroll
-		for (int i = 0; i < MLP_H; i++) z = fmaf(W2[MLP_H * j + i], a1[i], z);
-		const float a2 = tanhf(z);
-		const float dh2 = W3[j] * dy[0] + W3[MLP_H + j] * dy[1] + W3[2 * MLP_H + j] * dy[2];
-		const float dz2 = dh2 * (1.f - a2 * a2);
-		put(slot, MLP_W3 + j, dy[0] * a2);
-		put(slot, MLP_W3 + MLP_H + j, dy[1] * a2);
-		put(slot, MLP_W3 + 2 * MLP_H + j, dy[2] * a2);
-		put(slot, MLP_B2 + j, dz2);
-#pragma unroll
-		for (int i = 0; i < MLP_H; i++) {
-			put(slot, MLP_W2 + MLP_H * j + i, dz2 * a1[i]);
-			dh1[i] = fmaf(W2[MLP_H * j + i], dz2, dh1[i]);
+			for (int k = 0; k < 4; k++)
+				a[k] = tanhf(T.b1[j + k] + T.w1[3 * (j + k)] * v[0] + T.w1[3 * (j + k) + 1] * v[1]
+				             + T.w1[3 * (j + k) + 2] * v[2]);
+			*(float4 *) &T.a1[s * MT_LD + j] = make_float4(a[0], a[1], a[2], a[3]);
 		}
-	}
+		__syncthreads();
+		float a1[MLP_H];
 #pragma unroll
-	for (int j = 0; j < MLP_H; j++) {
-		const float dz1 = dh1[j] * (1.f - a1[j] * a1[j]);
-		put(slot, MLP_B1 + j, dz1);
-		put(slot, MLP_W1 + 3 * j, dz1 * v[0]);
-		put(slot, MLP_W1 + 3 * j + 1, dz1 * v[1]);
-		put(slot, MLP_W1 + 3 * j + 2, dz1 * v[2]);
+		for (int i = 0; i < MLP_H; i += 4) {
+			const float4 f = *(const float4 *) &T.a1[s * MT_LD + i];
+			a1[i] = f.x; a1[i + 1] = f.y; a1[i + 2] = f.z; a1[i + 3] = f.w;
+		}
+		float o[3] = { 0.f, 0.f, 0.f };
+		for (int j = j0; j < j0 + MLP_H / 2; j += 4) {
+			float z[4];
+#pragma unroll
+			for (int k = 0; k < 4; k++) z[k] = T.b2[j + k];
+#pragma unroll
+			for (int i = 0; i < MLP_H; i += 4)
+#pragma unroll
+				for (int k = 0; k < 4; k++) {
+					const float4 w = *(const float4 *) &T.w2[MLP_H * (j + k) + i];
+					z[k] = fmaf(w.x, a1[i], z[k]);
+					z[k] = fmaf(w.y, a1[i + 1], z[k]);
+					z[k] = fmaf(w.z, a1[i + 2], z[k]);
+					z[k] = fmaf(w.w, a1[i + 3], z[k]);
+				}
+#pragma unroll
+			for (int k = 0; k < 4; k++) {
+				z[k] = tanhf(z[k]);
+				o[0] = fmaf(T.w3[j + k], z[k], o[0]);
+				o[1] = fmaf(T.w3[MLP_H + j + k], z[k], o[1]);
+				o[2] = fmaf(T.w3[2 * MLP_H + j + k], z[k], o[2]);
+			}
+			*(float4 *) &T.a2[s * MT_LD + j] = make_float4(z[0], z[1], z[2], z[3]);
+		}
+#pragma unroll
+		for (int d = 0; d < 3; d++) T.out[half][s][d] = o[d];
+		__syncthreads();
+		float dy[3];
+#pragma unroll
+		for (int d = 0; d < 3; d++) {
+			const float r = have ? T.b3[d] + T.out[0][s][d] + T.out[1][s][d] - t[d] : 0.f;
+			if (half == 0) loss = fmaf(r, r, loss);
+			dy[d] = 2.f * r * inv_norm;
+			if (half == 0) T.dy[s][d] = dy[d];
+		}
+		for (int j = j0; j < j0 + MLP_H / 2; j += 4) {
+			const float4 f = *(const float4 *) &T.a2[s * MT_LD + j];
+			const float a2[4] = { f.x, f.y, f.z, f.w };
+			float dz[4];
+#pragma unroll
+			for (int k = 0; k < 4; k++)
+				dz[k] = (T.w3[j + k] * dy[0] + T.w3[MLP_H + j + k] * dy[1] + T.w3[2 * MLP_H + j + k] * dy[2])
+				      * (1.f - a2[k] * a2[k]);
+			*(float4 *) &T.dz2[s * MT_LD + j] = make_float4(dz[0], dz[1], dz[2], dz[3]);
+		}
+		__syncthreads();
+		// dz1 of this half's neurons: W2^T dz2
+		float dh[MLP_H / 2];
+#pragma unroll
+		for (int i = 0; i < MLP_H / 2; i++) dh[i] = 0.f;
+#pragma unroll 2
+		for (int j = 0; j < MLP_H; j++) {
+			const float d = T.dz2[s * MT_LD + j];
+#pragma unroll
+			for (int i = 0; i < MLP_H / 2; i += 4) {
+				const float4 w = *(const float4 *) &T.w2[MLP_H * j + j0 + i];
+				dh[i] = fmaf(w.x, d, dh[i]);
+				dh[i + 1] = fmaf(w.y, d, dh[i + 1]);
+				dh[i + 2] = fmaf(w.z, d, dh[i + 2]);
+				dh[i + 3] = fmaf(w.w, d, dh[i + 3]);
+			}
+		}
+#pragma unroll
+		for (int i = 0; i < MLP_H / 2; i += 4) {
+			const float4 f = *(const float4 *) &T.a1[s * MT_LD + j0 + i];
+			*(float4 *) &T.dz1[s * MT_LD + j0 + i] =
+			    make_float4(dh[i] * (1.f - f.x * f.x), dh[i + 1] * (1.f - f.y * f.y),
+			                dh[i + 2] * (1.f - f.z * f.z), dh[i + 3] * (1.f - f.w * f.w));
+		}
+		__syncthreads();
+		// the tile's gradients
+#pragma unroll 2
+		for (int k = 0; k < MT; k++) {
+			const float4 d0 = *(const float4 *) &T.dz2[k * MT_LD + tj], d1 = *(const float4 *) &T.dz2[k * MT_LD + tj + 4],
+			             a = *(const float4 *) &T.a1[k * MT_LD + ti];
+			const float d[8] = { d0.x, d0.y, d0.z, d0.w, d1.x, d1.y, d1.z, d1.w };
+#pragma unroll
+			for (int e = 0; e < 8; e++) {
+				g2[e][0] = fmaf(d[e], a.x, g2[e][0]);
+				g2[e][1] = fmaf(d[e], a.y, g2[e][1]);
+				g2[e][2] = fmaf(d[e], a.z, g2[e][2]);
+				g2[e][3] = fmaf(d[e], a.w, g2[e][3]);
+			}
+		}
+		if (half == 0) {
+			for (int k = 0; k < MT; k++) {
+				const float a = T.a2[k * MT_LD + s];
+				gs[0] += T.dz2[k * MT_LD + s];
+#pragma unroll
+				for (int d = 0; d < 3; d++) gs[1 + d] = fmaf(T.dy[k][d], a, gs[1 + d]);
+			}
+		} else {
+			for (int k = 0; k < MT; k++) {
+				const float a = T.dz1[k * MT_LD + s];
+				gs[0] += a;
+#pragma unroll
+				for (int d = 0; d < 3; d++) gs[1 + d] = fmaf(a, T.v[k][d], gs[1 + d]);
+			}
+		}
+		if (tid < 3)
+			for (int k = 0; k < MT; k++) g3 += T.dy[k][tid];
 	}
+	float *slot = slots + (int64_t) blockIdx.x * MLP_NNET;
+#pragma unroll
+	for (int e = 0; e < 8; e++)
+#pragma unroll
+		for (int k = 0; k < 4; k++) slot[MLP_W2 + MLP_H * (tj + e) + ti + k] = g2[e][k];
+	if (half == 0) {
+		slot[MLP_B2 + s] = gs[0];
+#pragma unroll
+		for (int d = 0; d < 3; d++) slot[MLP_W3 + d * MLP_H + s] = gs[1 + d];
+	} else {
+		slot[MLP_B1 + s] = gs[0];
+#pragma unroll
+		for (int d = 0; d < 3; d++) slot[MLP_W1 + 3 * s + d] = gs[1 + d];
+	}
+	if (tid < 3) slot[MLP_B3 + tid] = g3;
+	// half 0 is warps 0 and 1
+	loss = warp_sum(loss);
+	if (tid == 0 || tid == 32) T.out[0][tid / 32][0] = loss;
+	__syncthreads();
+	if (tid == 0) loss_slots[blockIdx.x] = T.out[0][0][0] + T.out[0][1][0];
 }
 
-// sum of the warp slots in slot order (deterministic)
-__global__ void k_mlp_sum(int nslots, const float *__restrict__ slots, const float *__restrict__ lslots,
-                          float *grad, float *loss)
+// sums of the blocks' slots in FP64, each parameter over four interleaved
+// parts that are added in order (deterministic)
+__global__ void __launch_bounds__(256)
+k_mlp_sum(int nslots, const float *__restrict__ slots, const float *__restrict__ lslots,
+          float *grad, float *loss)
 {
-	const int e = blockIdx.x * blockDim.x + threadIdx.x;
+	__shared__ double part[4][64];
+	const int c = threadIdx.x & 63, w = threadIdx.x >> 6, e = blockIdx.x * 64 + c;
+	double g = 0;
 	if (e < MLP_NNET) {
-		float g = 0.f;
-		for (int w = 0; w < nslots; w++) g += slots[(int64_t) w * MLP_NNET + e];
-		grad[e] = g;
+#pragma unroll 4
+		for (int k = w; k < nslots; k += 4) g += (double) slots[(int64_t) k * MLP_NNET + e];
+	} else if (e == MLP_NNET) {
+		for (int k = w; k < nslots; k += 4) g += (double) lslots[k];
 	}
-	if (e == MLP_NNET) {
-		double l = 0;
-		for (int w = 0; w < nslots; w++) l += lslots[w];
-		*loss = (float) l;
-	}
+	part[w][c] = g;
+	__syncthreads();
+	if (w > 0 || e > MLP_NNET) return;
+	g = ((part[0][c] + part[1][c]) + part[2][c]) + part[3][c];
+	if (e < MLP_NNET) grad[e] = (float) g;
+	else *loss = (float) g;
 }
 
 // Adam (Kingma & Ba 2015)
@@ -305,9 +425,11 @@ k_mlp_eval(int64_t n, const double *__restrict__ x, const __nv_bfloat16 *__restr
 
 // ------------------------------------------------------------ host
 
-// one gradient / loss slot per launched warp (blocks of 128 threads): the
-// warps past n write zeros into their own slots
-static inline int64_t mlp_slots(int64_t n) { return ((n + 127) / 128) * 4; }
+// blocks of the gradient kernel, and its slots: two tiles on an SM at a time
+static inline int grad_blocks(int64_t n) { return (int) std::min<int64_t>((n + MT - 1) / MT, 2 * 148); }
+
+// a loss slot per warp of the forward kernel (blocks of 128 threads)
+static inline int64_t loss_slots(int64_t n) { return ((n + 127) / 128) * 4; }
 
 static int dmalloc(tvg_context *ctx, void **p, size_t b)
 {
@@ -409,12 +531,13 @@ static int refresh_bf16(tvg_context *ctx)
 static int grad_batch(tvg_context *ctx, int64_t n, const float *x, const float *y, float *grad,
                       float *loss, float *slots, float *lslots)
 {
-	const int nslots = (int) mlp_slots(n);
-	k_mlp_grad<<<TVG_CNT(ctx, tvg_blocks(n, 128)), 128, 0, ctx->stream>>>(
+	const int nb = grad_blocks(n);
+	TVG_CUDA(ctx, cudaFuncSetAttribute(k_mlp_grad, cudaFuncAttributeMaxDynamicSharedMemorySize,
+	                                   (int) sizeof(MlpTile)));
+	k_mlp_grad<<<TVG_CNT(ctx, nb), MT_THREADS, sizeof(MlpTile), ctx->stream>>>(
 	    n, x, y, ctx->mlp_prm, 1.f / (3.f * (float) n), slots, lslots);
 	TVG_CUDA(ctx, cudaGetLastError());
-	k_mlp_sum<<<TVG_CNT(ctx, (MLP_NNET + 1 + 255) / 256), 256, 0, ctx->stream>>>(nslots, slots, lslots,
-	                                                                             grad, loss);
+	k_mlp_sum<<<TVG_CNT(ctx, (MLP_NNET + 1 + 63) / 64), 256, 0, ctx->stream>>>(nb, slots, lslots, grad, loss);
 	TVG_CUDA(ctx, cudaGetLastError());
 	return TVG_OK;
 }
@@ -442,7 +565,7 @@ extern "C" int tvg_ewald_mlp_train(tvg_context *ctx, const tvg_mlp_train_config 
 		return TVG_OK;
 	};
 	int rc = TVG_OK;
-	const int nslots = (int) mlp_slots(nb);
+	const int nslots = grad_blocks(nb);
 	if ((rc = alloc(&x, 12 * (size_t) ns)) || (rc = alloc(&y, 12 * (size_t) ns))
 	    || (rc = alloc(&slots, 4 * (size_t) nslots * MLP_NPARAM)) || (rc = alloc(&lslots, 4 * (size_t) nslots))
 	    || (rc = alloc(&grad, 4 * MLP_NPARAM)) || (rc = alloc(&m, 4 * MLP_NPARAM))
@@ -492,10 +615,10 @@ extern "C" int tvg_ewald_mlp_train(tvg_context *ctx, const tvg_mlp_train_config 
 	}
 	// mean-square residual of the trained FP32 weights over all samples
 	float *lall = nullptr;
-	if ((rc = alloc(&lall, 4 * (size_t) mlp_slots(ns)))) return done(rc);
+	if ((rc = alloc(&lall, 4 * (size_t) loss_slots(ns)))) return done(rc);
 	k_mlp_loss<<<TVG_CNT(ctx, tvg_blocks(ns, 128)), 128, 0, s>>>(ns, x, y, ctx->mlp_prm, lall);
 	if (cudaGetLastError() != cudaSuccess) return done(tvg_fail(ctx, TVG_E_CUDA, "mlp loss launch"));
-	std::vector<float> lw((size_t) mlp_slots(ns));
+	std::vector<float> lw((size_t) loss_slots(ns));
 	float sc = 1.f;
 	if (cudaMemcpyAsync(lw.data(), lall, 4 * lw.size(), cudaMemcpyDeviceToHost, s) != cudaSuccess
 	    || cudaMemcpyAsync(&sc, ctx->mlp_prm + MLP_SCALE, 4, cudaMemcpyDeviceToHost, s) != cudaSuccess)
@@ -525,6 +648,9 @@ extern "C" int tvg_ewald_mlp_weights(tvg_context *ctx, float *params, int32_t se
 	return TVG_OK;
 }
 
+// device memory kept between gradient calls (released with the context)
+#define MLP_KEEP ((size_t) 64 << 20)
+
 extern "C" int tvg_ewald_mlp_grad(tvg_context *ctx, int64_t n, const float *x, const float *y,
                                   float *grad, float *loss)
 {
@@ -532,14 +658,27 @@ extern "C" int tvg_ewald_mlp_grad(tvg_context *ctx, int64_t n, const float *x, c
 	if (!ctx->have_mlp) return tvg_fail(ctx, TVG_E_STATE, "mlp: no weights");
 	TVG_CUDA(ctx, cudaSetDevice(ctx->device));
 	cudaStream_t s = ctx->stream;
-	const int nslots = (int) mlp_slots(n);
-	float *dx, *dy, *sl, *ll, *g, *l;
-	TVG_CUDA(ctx, cudaMalloc((void **) &dx, 12 * (size_t) n));
-	TVG_CUDA(ctx, cudaMalloc((void **) &dy, 12 * (size_t) n));
-	TVG_CUDA(ctx, cudaMalloc((void **) &sl, 4 * (size_t) nslots * MLP_NPARAM));
-	TVG_CUDA(ctx, cudaMalloc((void **) &ll, 4 * (size_t) nslots));
-	TVG_CUDA(ctx, cudaMalloc((void **) &g, 4 * MLP_NPARAM + 4));
-	l = g + MLP_NPARAM;
+	// samples, slots, gradient and loss in one block of device memory, kept in
+	// the context up to MLP_KEEP bytes (the five allocations and their frees took
+	// 1.1 ms of a call with 16,384 samples)
+	const int nslots = grad_blocks(n);
+	const size_t b_xy = ((size_t) 12 * n + 255) & ~(size_t) 255, b_sl = 4 * (size_t) nslots * MLP_NNET,
+	             bytes = 2 * b_xy + b_sl + 4 * (size_t) nslots + 4 * MLP_NPARAM + 4;
+	char *ws = (char *) ctx->mlp_ws;
+	if (bytes > ctx->mlp_ws_bytes) {
+		if (bytes <= MLP_KEEP && ctx->mlp_ws) {
+			cudaFree(ctx->mlp_ws);
+			ctx->mlp_ws = nullptr;
+			ctx->mlp_ws_bytes = 0;
+		}
+		TVG_CUDA(ctx, cudaMalloc((void **) &ws, bytes));
+		if (bytes <= MLP_KEEP) {
+			ctx->mlp_ws = ws;
+			ctx->mlp_ws_bytes = bytes;
+		}
+	}
+	float *dx = (float *) ws, *dy = (float *) (ws + b_xy), *g = (float *) (ws + 2 * b_xy),
+	      *l = g + MLP_NPARAM, *ll = l + 1, *sl = ll + nslots;
 	cudaMemsetAsync(g, 0, 4 * MLP_NPARAM + 4, s);      // the fitted entries have no gradient
 	cudaMemcpyAsync(dx, x, 12 * (size_t) n, cudaMemcpyHostToDevice, s);
 	cudaMemcpyAsync(dy, y, 12 * (size_t) n, cudaMemcpyHostToDevice, s);
@@ -549,7 +688,7 @@ extern "C" int tvg_ewald_mlp_grad(tvg_context *ctx, int64_t n, const float *x, c
 		if (loss) cudaMemcpyAsync(loss, l, 4, cudaMemcpyDeviceToHost, s);
 		if (cudaStreamSynchronize(s) != cudaSuccess) rc = tvg_fail(ctx, TVG_E_CUDA, "mlp grad copy");
 	}
-	cudaFree(dx); cudaFree(dy); cudaFree(sl); cudaFree(ll); cudaFree(g);
+	if (ws != ctx->mlp_ws) cudaFree(ws);
 	return rc;
 }
 

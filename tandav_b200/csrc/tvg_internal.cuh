@@ -215,6 +215,8 @@ struct tvg_context {
 	// learned Ewald correction (tvg_ewald_mlp.cu)
 	float *mlp_prm = nullptr;          // FP32 parameters (4611)
 	void *mlp_bf16 = nullptr;          // BF16 copy used for inference
+	void *mlp_ws = nullptr;            // tvg_ewald_mlp_grad's device memory (at most 64 MB kept)
+	size_t mlp_ws_bytes = 0;
 	bool have_mlp = false, mlp_ok = false;
 	double mlp_max_err = 0;
 

@@ -103,3 +103,23 @@ def test_walk_with_learned_correction(trained):
     # walk's own error dominates both)
     assert res["learned"] < res["none"] / 1000
     assert res["learned"] <= 1.1 * res["table"]
+
+
+@pytest.mark.parametrize("n", [1, 63, 64, 65, 4097, 19009])
+def test_mlp_gradient_tiles(n):
+    """Tiles of 64 samples over at most 296 blocks: one sample, the edges of a
+    tile, and more tiles than blocks. FP32 sums against FP64, the existing
+    gradient test's bound."""
+    rng = np.random.default_rng(n)
+    p = (rng.standard_normal(O.NPARAM) * 0.3).astype(np.float32)
+    x = (rng.random((n, 3)) * 0.5).astype(np.float32)
+    y = (rng.standard_normal((n, 3)) * 0.5).astype(np.float32)
+    with G.GravityContext(1024, periodic=True, boxsize=1.0) as ctx:
+        ctx.mlp_weights(p)
+        g, loss = ctx.mlp_grad(x, y)
+        again, loss2 = ctx.mlp_grad(x, y)
+    np.testing.assert_array_equal(g, again)
+    assert loss == loss2
+    go, lo = O.grad(p.astype(np.float64), x.astype(np.float64), y.astype(np.float64))
+    assert loss == pytest.approx(lo, rel=1e-4)
+    assert np.abs(g - go).max() < 2e-4 * np.abs(go).max()
