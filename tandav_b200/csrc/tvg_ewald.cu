@@ -56,36 +56,6 @@ int tvg_impl_ewald_init(tvg_context *ctx)
 	return TVG_OK;
 }
 
-// The group form's correction table: T(x) (box units, unit G m: the force of
-// the periodic lattice minus the image at the origin, the quantity of the
-// table above) at x = 0.5 i / 64 for i = -1..66 per axis, in FP64 then stored
-// FP32 as (Tx, Ty, Tz, 0). The layer at i = -1 and the layers beyond L/2 let
-// a 4-point stencil stay centred everywhere on the octant; beyond L/2 the
-// values are the analytic continuation of that correction, which a Taylor
-// expansion about a point near the half-box plane needs.
-#define N_EXT 68
-
-__global__ void k_ewald_ext(float4 *ext)
-{
-	const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-	if (idx >= N_EXT * N_EXT * N_EXT) return;
-	const int i = idx / (N_EXT * N_EXT) - 1, j = (idx / N_EXT) % N_EXT - 1, k = idx % N_EXT - 1;
-	const double x[3] = { (0.5 * i) / N_EWALD, (0.5 * j) / N_EWALD, (0.5 * k) / N_EWALD };
-	double f[3], pot;
-	ewald_point(x, f, &pot);
-	ext[idx] = make_float4((float) f[0], (float) f[1], (float) f[2], 0.f);
-}
-
-int tvg_impl_ewald_ext(tvg_context *ctx)
-{
-	const size_t npt = (size_t) N_EXT * N_EXT * N_EXT;
-	if (!ctx->ewald_ext) TVG_CUDA(ctx, cudaMalloc((void **) &ctx->ewald_ext, 16 * npt));
-	k_ewald_ext<<<TVG_CNT(ctx, tvg_blocks((int64_t) npt, 128)), 128, 0, ctx->stream>>>(
-	    (float4 *) ctx->ewald_ext);
-	TVG_CUDA(ctx, cudaGetLastError());
-	return TVG_OK;
-}
-
 // Taylor table of the group form: at each node x = i / (2 (N - 1)) (box
 // units, i = 0..N-1 per axis, N = TVG_TAYLOR_NODES) of the octant, T and its
 // first three derivatives, the k-th derivative taken with respect to the node
@@ -191,6 +161,108 @@ int tvg_impl_ewald_taylor(tvg_context *ctx)
 	if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
 	cudaFree(fine);
 	if (e != cudaSuccess) return tvg_fail(ctx, TVG_E_CUDA, "ewald taylor table: %s", cudaGetErrorString(e));
+	return TVG_OK;
+}
+
+// Table of the lattice force for single points (the group form's wide groups,
+// k_ewald_wide): at each node x = i / (2 (N - 1)), N = TVG_WIDE_NODES, of the
+// octant, T and its first three derivatives in node units. T is a gradient and
+// its divergence is 4 pi, so the derivative tensors are symmetric and
+// traceless (but for that constant) and 24 numbers hold them all: 96 bytes,
+// three 32-byte loads, where a tricubic lookup of a 68^3 value table took 64
+// loads. Record:
+//   Tx Ty Tz, d2 phi xx yy xy xz yz -> dT;
+//   d2T as xxx xxy xxz xyy xyz yyy yyz, d3T as xxxx;
+//   xxxy xxxz yyyy xyyy yyyz xxyy xxyz xyyz.
+// With 41 nodes the third-order expansion about the nearest node is within
+// 5e-8 rms of direct lattice sums over the octant (tricubic: 8e-8, and 1.2e-7
+// with its FP32 sums). The lattice sums on the grid of half the spacing are
+// evaluated for sorted coordinates only; the others are their permutations.
+#define N_WIDE TVG_WIDE_NODES
+#define N_WFINE (2 * (N_WIDE - 1) + 1 + 4)
+
+__global__ void k_wide_fine(double *fine)
+{
+	const int idx = blockIdx.x * blockDim.x + threadIdx.x;
+	if (idx >= N_WFINE * N_WFINE * N_WFINE) return;
+	const int i[3] = { idx / (N_WFINE * N_WFINE), (idx / N_WFINE) % N_WFINE, idx % N_WFINE };
+	if (i[0] > i[1] || i[1] > i[2]) return;
+	const double d = 1.0 / (4.0 * (N_WIDE - 1));
+	const double x[3] = { (i[0] - 2) * d, (i[1] - 2) * d, (i[2] - 2) * d };
+	double f[3], pot;
+	ewald_point(x, f, &pot);
+	const int perm[6][3] = { { 0, 1, 2 }, { 0, 2, 1 }, { 1, 0, 2 }, { 1, 2, 0 }, { 2, 0, 1 }, { 2, 1, 0 } };
+	for (int q = 0; q < 6; q++) {
+		const int *o = perm[q];
+		double *w = fine + 3 * (((int64_t) i[o[0]] * N_WFINE + i[o[1]]) * N_WFINE + i[o[2]]);
+		for (int a = 0; a < 3; a++) w[a] = f[o[a]];
+	}
+}
+
+__global__ void k_wide_table(const double *__restrict__ fine, float *tab)
+{
+	const int idx = blockIdx.x * blockDim.x + threadIdx.x;
+	if (idx >= N_WIDE * N_WIDE * N_WIDE) return;
+	const int ci = 2 * (idx / (N_WIDE * N_WIDE)) + 2, cj = 2 * ((idx / N_WIDE) % N_WIDE) + 2,
+	          ck = 2 * (idx % N_WIDE) + 2;
+	const double h = 0.5, h2 = h * h, h3 = h2 * h;       // fine spacing, node units
+	auto f = [&](int a, int di, int dj, int dk) {
+		return fine[3 * (((int64_t) (ci + di) * N_WFINE + (cj + dj)) * N_WFINE + (ck + dk)) + a];
+	};
+	auto g = [&](int a, int b, int s) {
+		return b == 0 ? f(a, s, 0, 0) : b == 1 ? f(a, 0, s, 0) : f(a, 0, 0, s);
+	};
+	auto g2 = [&](int a, int b, int sb, int e, int se) {
+		int d[3] = { 0, 0, 0 };
+		d[b] += sb;
+		d[e] += se;
+		return f(a, d[0], d[1], d[2]);
+	};
+	auto d1 = [&](int a, int b) { return (-g(a, b, 2) + 8 * g(a, b, 1) - 8 * g(a, b, -1) + g(a, b, -2)) / (12 * h); };
+	auto d2 = [&](int a, int b) {
+		return (-g(a, b, 2) + 16 * g(a, b, 1) - 30 * f(a, 0, 0, 0) + 16 * g(a, b, -1) - g(a, b, -2)) / (12 * h2);
+	};
+	auto d2m = [&](int a, int b, int e) {
+		return (g2(a, b, 1, e, 1) - g2(a, b, 1, e, -1) - g2(a, b, -1, e, 1) + g2(a, b, -1, e, -1)) / (4 * h2);
+	};
+	auto d3 = [&](int a, int b) { return (g(a, b, 2) - 2 * g(a, b, 1) + 2 * g(a, b, -1) - g(a, b, -2)) / (2 * h3); };
+	// d3 T_a / db db de
+	auto d3m = [&](int a, int b, int e) {
+		const double up = g2(a, b, 1, e, 1) - 2 * g2(a, b, 0, e, 1) + g2(a, b, -1, e, 1);
+		const double dn = g2(a, b, 1, e, -1) - 2 * g2(a, b, 0, e, -1) + g2(a, b, -1, e, -1);
+		return (up - dn) / (2 * h3);
+	};
+	float *r = tab + 24 * (int64_t) idx;
+	const double v[24] = {
+		f(0, 0, 0, 0), f(1, 0, 0, 0), f(2, 0, 0, 0), d1(0, 0), d1(1, 1), d1(0, 1), d1(0, 2), d1(1, 2),
+		d2(0, 0), d2(1, 0), d2(2, 0), d2(0, 1), (d2m(0, 1, 2) + d2m(1, 0, 2) + d2m(2, 0, 1)) / 3, d2(1, 1), d2(2, 1),
+		d3(0, 0),
+		d3(1, 0), d3(2, 0), d3(1, 1), d3(0, 1), d3(2, 1), 0.5 * (d3m(1, 0, 1) + d3m(0, 1, 0)), d3m(2, 0, 1),
+		d3m(2, 1, 0)
+	};
+	for (int q = 0; q < 24; q++) r[q] = (float) v[q];
+}
+
+int tvg_impl_ewald_wide(tvg_context *ctx)
+{
+	const size_t n = (size_t) N_WIDE * N_WIDE * N_WIDE, nfine = (size_t) N_WFINE * N_WFINE * N_WFINE;
+	double *fine = nullptr;
+	TVG_CUDA(ctx, cudaMalloc((void **) &fine, 24 * nfine));
+	float *tab = nullptr;
+	cudaError_t e = cudaMalloc((void **) &tab, 96 * n);
+	if (e == cudaSuccess) {
+		k_wide_fine<<<TVG_CNT(ctx, tvg_blocks((int64_t) nfine, 128)), 128, 0, ctx->stream>>>(fine);
+		k_wide_table<<<TVG_CNT(ctx, tvg_blocks((int64_t) n, 128)), 128, 0, ctx->stream>>>(fine, tab);
+		e = cudaGetLastError();
+		const cudaError_t es = cudaStreamSynchronize(ctx->stream);
+		if (e == cudaSuccess) e = es;
+	}
+	cudaFree(fine);
+	if (e != cudaSuccess) {
+		cudaFree(tab);
+		return tvg_fail(ctx, TVG_E_CUDA, "ewald table of the wide groups: %s", cudaGetErrorString(e));
+	}
+	ctx->ewald_wide = tab;
 	return TVG_OK;
 }
 

@@ -441,11 +441,11 @@ struct GroupParams {
 	float gravity;
 	float eps2, inv_eps2, c16;     // softening (h^2, 1/h^2, 1/(16 h^3))
 	float near2;        // h^2 with a rounding margin: closer sources use the softened kernel
-	float grid;         // Ewald table cells per length (2 * 64 / L)
 	float inv_box;
 	float ew_rel;       // Ewald opening: alpha_E / TREE_OPEN_PARAM_REL (relative mode)
 	float ew_bh;        // Ewald opening: s^2 h2 limit in units of L^2 (Barnes-Hut mode)
 	float taylor_h;     // groups with a larger half extent take per-target images (with Ewald)
+	float wide_grid;    // node spacings per length of the table for single points
 	float tay_grid;     // Taylor-table node spacings per length (2 (TVG_TAYLOR_NODES - 1) / L)
 	double uniform_g;   // G / L^2: times the total mass, the scale of the uniform-background remainder
 };
@@ -1100,30 +1100,9 @@ k_walk_group(GroupParams p, const int32_t *__restrict__ active, const int32_t *_
 
 // ------------------------------------------------------ the Ewald walk
 
-// 4-point Lagrange basis on the nodes -1, 0, 1, 2 at t in [0, 1]: weights,
-// first and second derivatives
-__device__ __forceinline__ void lagrange4(float t, float w[4], float d[4], float dd[4])
-{
-	const float t2 = t * t, t3 = t2 * t;
-	w[0] = (-t3 + 3.f * t2 - 2.f * t) * (1.f / 6.f);
-	w[1] = (t3 - 2.f * t2 - t + 2.f) * 0.5f;
-	w[2] = (-t3 + t2 + 2.f * t) * 0.5f;
-	w[3] = (t3 - t) * (1.f / 6.f);
-	d[0] = (-3.f * t2 + 6.f * t - 2.f) * (1.f / 6.f);
-	d[1] = (3.f * t2 - 4.f * t - 1.f) * 0.5f;
-	d[2] = (-3.f * t2 + 2.f * t + 2.f) * 0.5f;
-	d[3] = (3.f * t2 - 1.f) * (1.f / 6.f);
-	dd[0] = 1.f - t;
-	dd[1] = 3.f * t - 2.f;
-	dd[2] = 1.f - 3.f * t;
-	dd[3] = t;
-}
-
 // The lattice-minus-image force T(x) (box units, unit G m, target at x from
-// the source) is tabulated on x = 0.5 i / 64, i = -1..66 per axis (one ghost
-// layer below 0 and the analytic continuation beyond 1/2), interleaved
-// (Tx, Ty, Tz, 0). The correction for a source at d from the target is
-// K(d) = -G m T(d / L) / L^2 (the reference's sign rule, periodic.c:100-112),
+// the source) on the octant; the correction for a source at d from the target
+// is K(d) = -G m T(d / L) / L^2 (the reference's sign rule, periodic.c:100-112),
 // looked up at |d| with the symmetries T_a(.., -x_b, ..) = -T_a if a = b,
 // +T_a otherwise.
 
@@ -1228,39 +1207,54 @@ __device__ __forceinline__ void ewald_kjh_taylor(const GroupParams &p, const flo
 	}
 }
 
-// K(d) alone (tricubic value of the extended table), for per-target
-// evaluation, added to a
-__device__ __forceinline__ void ewald_k(const GroupParams &p, const float4 *__restrict__ tab, float ex,
-                                        float ey, float ez, float gm, float &ax, float &ay, float &az)
+// K(d) alone, for per-target evaluation, m0 = -G m / L^2, added to a: the
+// third-order expansion about the nearest node of the table of
+// tvg_impl_ewald_wide (tvg_ewald.cu). The lanes of a warp read as many records,
+// one L1 wavefront each a load, which is what bounds the wide groups.
+__device__ __forceinline__ void ewald_k(const GroupParams &p, const float *__restrict__ tab, float ex,
+                                        float ey, float ez, float m0, float &ax, float &ay, float &az)
 {
-	const float sx = ex < 0.f ? -1.f : 1.f, sy = ey < 0.f ? -1.f : 1.f, sz = ez < 0.f ? -1.f : 1.f;
-	const float u = fabsf(ex) * p.grid, v = fabsf(ey) * p.grid, w = fabsf(ez) * p.grid;
-	const int i = min((int) u, 64), j = min((int) v, 64), l = min((int) w, 64);
-	float wx[4], wy[4], wz[4], d_[4], dd_[4];
-	lagrange4(u - (float) i, wx, d_, dd_);
-	lagrange4(v - (float) j, wy, d_, dd_);
-	lagrange4(w - (float) l, wz, d_, dd_);
-	float vx = 0.f, vy = 0.f, vz = 0.f;
-	const int base = (i * 68 + j) * 68 + l;
-#pragma unroll 1
-	for (int a = 0; a < 4; a++) {
-		float yx = 0.f, yy = 0.f, yz = 0.f;
-#pragma unroll
-		for (int b = 0; b < 4; b++) {
-			const float4 *row = tab + base + (a * 68 + b) * 68;
-			const float4 t0 = __ldg(row), t1 = __ldg(row + 1), t2 = __ldg(row + 2), t3 = __ldg(row + 3);
-			yx = fmaf(wy[b], wz[0] * t0.x + wz[1] * t1.x + wz[2] * t2.x + wz[3] * t3.x, yx);
-			yy = fmaf(wy[b], wz[0] * t0.y + wz[1] * t1.y + wz[2] * t2.y + wz[3] * t3.y, yy);
-			yz = fmaf(wy[b], wz[0] * t0.z + wz[1] * t1.z + wz[2] * t2.z + wz[3] * t3.z, yz);
-		}
-		vx = fmaf(wx[a], yx, vx);
-		vy = fmaf(wx[a], yy, vy);
-		vz = fmaf(wx[a], yz, vz);
-	}
-	const float m0 = -gm * p.inv_box * p.inv_box;
-	ax = fmaf(m0 * sx, vx, ax);
-	ay = fmaf(m0 * sy, vy, ay);
-	az = fmaf(m0 * sz, vz, az);
+	const float u = fabsf(ex) * p.wide_grid, v = fabsf(ey) * p.wide_grid, w = fabsf(ez) * p.wide_grid;
+	const int i = min(__float2int_rn(u), TVG_WIDE_NODES - 1);
+	const int j = min(__float2int_rn(v), TVG_WIDE_NODES - 1);
+	const int l = min(__float2int_rn(w), TVG_WIDE_NODES - 1);
+	const float x = u - (float) i, y = v - (float) j, z = w - (float) l;
+	const float *rec = tab + 24 * ((i * TVG_WIDE_NODES + j) * TVG_WIDE_NODES + l);
+	float t[3], B[5], C[7], D[9];
+	asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+	    : "=f"(t[0]), "=f"(t[1]), "=f"(t[2]), "=f"(B[0]), "=f"(B[1]), "=f"(B[2]), "=f"(B[3]), "=f"(B[4])
+	    : "l"(rec));
+	asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+	    : "=f"(C[0]), "=f"(C[1]), "=f"(C[2]), "=f"(C[3]), "=f"(C[4]), "=f"(C[5]), "=f"(C[6]), "=f"(D[0])
+	    : "l"(rec + 8));
+	asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+	    : "=f"(D[1]), "=f"(D[2]), "=f"(D[3]), "=f"(D[4]), "=f"(D[5]), "=f"(D[6]), "=f"(D[7]), "=f"(D[8])
+	    : "l"(rec + 16));
+	// D: xxxx xxxy xxxz yyyy xyyy yyyz xxyy xxyz xyyz; the entries with two z
+	// follow from the zero trace, here and in C + D u / 3 (xxx xxy xxz xyy xyz yyy
+	// yyz) and, its trace the constant 4 pi, in B + M u / 2 (xx yy xy xz yz)
+	const float th = 1.f / 3.f, x3 = th * x, y3 = th * y, z3 = th * z;
+	const float xxzz = -D[0] - D[6], xyzz = -D[1] - D[4], yyzz = -D[6] - D[3];
+	const float mxxx = fmaf(D[0], x3, fmaf(D[1], y3, fmaf(D[2], z3, C[0])));
+	const float mxxy = fmaf(D[1], x3, fmaf(D[6], y3, fmaf(D[7], z3, C[1])));
+	const float mxxz = fmaf(D[2], x3, fmaf(D[7], y3, fmaf(xxzz, z3, C[2])));
+	const float mxyy = fmaf(D[6], x3, fmaf(D[4], y3, fmaf(D[8], z3, C[3])));
+	const float mxyz = fmaf(D[7], x3, fmaf(D[8], y3, fmaf(xyzz, z3, C[4])));
+	const float myyy = fmaf(D[4], x3, fmaf(D[3], y3, fmaf(D[5], z3, C[5])));
+	const float myyz = fmaf(D[8], x3, fmaf(D[5], y3, fmaf(yyzz, z3, C[6])));
+	const float x2 = 0.5f * x, y2 = 0.5f * y, z2 = 0.5f * z;
+	const float nxx = fmaf(mxxx, x2, fmaf(mxxy, y2, fmaf(mxxz, z2, B[0])));
+	const float nyy = fmaf(mxyy, x2, fmaf(myyy, y2, fmaf(myyz, z2, B[1])));
+	const float nxy = fmaf(mxxy, x2, fmaf(mxyy, y2, fmaf(mxyz, z2, B[2])));
+	const float nxz = fmaf(mxxz, x2, fmaf(mxyz, y2, fmaf(-mxxx - mxyy, z2, B[3])));
+	const float nyz = fmaf(mxyz, x2, fmaf(myyz, y2, fmaf(-mxxy - myyy, z2, B[4])));
+	const float tr = 12.566370614f / (2 * (TVG_WIDE_NODES - 1));
+	const float vx = t[0] + fmaf(nxx, x, fmaf(nxy, y, nxz * z));
+	const float vy = t[1] + fmaf(nxy, x, fmaf(nyy, y, nyz * z));
+	const float vz = t[2] + fmaf(nxz, x, fmaf(nyz, y, (tr - nxx - nyy) * z));
+	ax = fmaf(ex < 0.f ? -m0 : m0, vx, ax);
+	ay = fmaf(ey < 0.f ? -m0 : m0, vy, ay);
+	az = fmaf(ez < 0.f ? -m0 : m0, vz, az);
 }
 
 // bound of |d2 T| (box units) within distance r (box units) of the source:
@@ -1333,8 +1327,7 @@ __device__ __noinline__ void mlp_forward_warp_call(const float *mlp, const uint3
 // wq (TVG_CFG_QUADRUPOLE, groups without per-target images): the walk
 // nodes' stored quadrupoles, lnode the list entries' nodes
 template <int TPL, bool MLP>
-__device__ __forceinline__ void ewald_batch(const GroupParams &p, const float4 *tab, const float4 *tay,
-                                            const float *mlp, const uint32_t *w2b, const float4 *list,
+__device__ __forceinline__ void ewald_batch(const GroupParams &p, const float4 *tay, const float *mlp, const uint32_t *w2b, const float4 *list,
                                             int from, int cnt, bool per_target, CorrSum &c,
                                             Target (&t)[TPL], float &nev,
                                             const int32_t *lnode = nullptr,
@@ -1363,7 +1356,7 @@ __device__ __forceinline__ void ewald_batch(const GroupParams &p, const float4 *
 			else ewald_kjh_taylor<false>(p, tay, list[from + lane], c, nullptr);
 			nev += 1.f;
 		}
-	} else {
+	} else if constexpr (MLP) {
 		float ax[TPL], ay[TPL], az[TPL];
 #pragma unroll
 		for (int k = 0; k < TPL; k++) ax[k] = ay[k] = az[k] = 0.f;
@@ -1374,17 +1367,13 @@ __device__ __forceinline__ void ewald_batch(const GroupParams &p, const float4 *
 				const float dx = wrap_half(s.x - t[k].tx, p.box, p.half_box);
 				const float dy = wrap_half(s.y - t[k].ty, p.box, p.half_box);
 				const float dz = wrap_half(s.z - t[k].tz, p.box, p.half_box);
-				if (MLP) {
-					const float xs[3] = { fabsf(dx) * p.inv_box, fabsf(dy) * p.inv_box, fabsf(dz) * p.inv_box };
-					float tv[3];
-					mlp_forward_warp_call(mlp, w2b, xs, tv);
-					const float m0 = -s.w * p.inv_box * p.inv_box;
-					ax[k] = fmaf(dx < 0.f ? -m0 : m0, tv[0], ax[k]);
-					ay[k] = fmaf(dy < 0.f ? -m0 : m0, tv[1], ay[k]);
-					az[k] = fmaf(dz < 0.f ? -m0 : m0, tv[2], az[k]);
-				} else {
-					ewald_k(p, tab, dx, dy, dz, s.w, ax[k], ay[k], az[k]);
-				}
+				const float xs[3] = { fabsf(dx) * p.inv_box, fabsf(dy) * p.inv_box, fabsf(dz) * p.inv_box };
+				float tv[3];
+				mlp_forward_warp_call(mlp, w2b, xs, tv);
+				const float m0 = -s.w * p.inv_box * p.inv_box;
+				ax[k] = fmaf(dx < 0.f ? -m0 : m0, tv[0], ax[k]);
+				ay[k] = fmaf(dy < 0.f ? -m0 : m0, tv[1], ay[k]);
+				az[k] = fmaf(dz < 0.f ? -m0 : m0, tv[2], az[k]);
 				if (t[k].valid) nev += 1.f;
 			}
 		}
@@ -1463,11 +1452,11 @@ template <int TPL, bool MLP>
 __device__ void ewald_group(const GroupParams &p, EwaldSmem &S, const tvg_wnode *__restrict__ wt,
                             const uint32_t *__restrict__ ix, const uint32_t *__restrict__ iy,
                             const uint32_t *__restrict__ iz, const float *__restrict__ mass_f,
-                            const float *__restrict__ last_acc, const float4 *__restrict__ tab,
-                            const float4 *__restrict__ tay, const float *mlp, const uint32_t *w2b,
+                            const float *__restrict__ last_acc, const float4 *__restrict__ tay,
+                            const float *mlp, const uint32_t *w2b,
                             int64_t first, int cnt, const int32_t *__restrict__ active,
                             Target (&t)[TPL], float &nev, EwaldStage *st, StageState &ss, int *status,
-                            const float4 *__restrict__ wq_all)
+                            const float4 *__restrict__ wq_all, int64_t group, int32_t *wide)
 {
 	const int lane = threadIdx.x & 31;
 	const unsigned lt = (1u << lane) - 1u;
@@ -1476,6 +1465,11 @@ __device__ void ewald_group(const GroupParams &p, EwaldSmem &S, const tvg_wnode 
 	const float hmax = fmaxf(g.hx, fmaxf(g.hy, g.hz));
 	// the gravity walk makes the same choice (walk_group)
 	const bool per_target = hmax >= p.taylor_h;
+	// with the table such groups are left to k_ewald_wide (wide[0] counts them)
+	if (!MLP && per_target) {
+		if (lane == 0) wide[1 + atomicAdd(&wide[0], 1)] = (int32_t) group;
+		return;
+	}
 	// node quadrupoles (TVG_CFG_QUADRUPOLE) in the expansion about the group
 	// centre; per-target images evaluate K alone and keep monopoles
 	const float4 *wq = per_target ? nullptr : wq_all;
@@ -1587,7 +1581,7 @@ __device__ void ewald_group(const GroupParams &p, EwaldSmem &S, const tvg_wnode 
 			if (full || (final && nl > 0)) {
 				const int cnt = full ? 32 : nl;
 				if (full && st && ss.ok && !per_target) stage_batch(p, tay, st, S.list, nl - 32, ss, c, nev, status);
-				else ewald_batch<TPL, MLP>(p, tab, tay, mlp, w2b, S.list, nl - cnt, cnt, per_target, c, t, nev,
+				else ewald_batch<TPL, MLP>(p, tay, mlp, w2b, S.list, nl - cnt, cnt, per_target, c, t, nev,
 				                           S.lnode, wq);
 				nl -= cnt;
 				continue;
@@ -1666,11 +1660,10 @@ k_ewald_group(GroupParams p, const int32_t *__restrict__ active, const int32_t *
               const tvg_wnode *__restrict__ wt,
               const uint32_t *__restrict__ ix, const uint32_t *__restrict__ iy,
               const uint32_t *__restrict__ iz, const float *__restrict__ mass_f,
-              const float *__restrict__ last_acc, const float4 *__restrict__ tab,
-              const float4 *__restrict__ tay, const __nv_bfloat16 *__restrict__ mlp_w,
-              const float *__restrict__ mlp_f32, F *acc0, F *acc1,
+              const float *__restrict__ last_acc, const float4 *__restrict__ tay,
+              const __nv_bfloat16 *__restrict__ mlp_w, const float *__restrict__ mlp_f32, F *acc0, F *acc1,
               F *acc2, F *gacc0, F *gacc1, F *gacc2, int32_t *work, double *counter, int *status,
-              const float4 *__restrict__ wq)
+              const float4 *__restrict__ wq, int32_t *wide)
 {
 	extern __shared__ __align__(16) unsigned char smem_raw[];
 	EwaldSmem &S = ((EwaldSmem *) smem_raw)[threadIdx.x >> 5];
@@ -1715,8 +1708,8 @@ k_ewald_group(GroupParams p, const int32_t *__restrict__ active, const int32_t *
 		}
 		Target t[TPL];
 		float nev = 0.f;
-		ewald_group<TPL, MLP>(p, S, wt, ix, iy, iz, mass_f, last_acc, tab, tay, mlp, w2b, first, cnt, active, t, nev,
-		                 st, ss, status, wq);
+		ewald_group<TPL, MLP>(p, S, wt, ix, iy, iz, mass_f, last_acc, tay, mlp, w2b, first, cnt, active, t, nev,
+		                      st, ss, status, wq, g, wide);
 		ev_acc += nev;
 #pragma unroll
 		for (int k = 0; k < TPL; k++) {
@@ -1734,6 +1727,232 @@ k_ewald_group(GroupParams p, const int32_t *__restrict__ active, const int32_t *
 #pragma unroll
 	for (int o = 16; o; o >>= 1) ev_acc += __shfl_xor_sync(0xFFFFFFFFu, ev_acc, o);
 	if (lane == 0 && ev_acc != 0) atomicAdd(counter, ev_acc);
+}
+
+// The groups that take per-target images (wide[1 ..], wide[0] of them): every
+// source at every target's nearest image. Such groups open almost every node, and
+// one of them can cost as much as a thousand others, so they are split: the
+// roots are dealt to `parts` items per group (root r to item r mod parts), so
+// that there are two items for each of the 16 warps an SM holds, each with its
+// own partial sums, which k_ewald_wide_sum adds in order. Box of 100^3 with a
+// few wide groups: 38 ms of Ewald walk with a warp for each, 1.7 ms so; of 48^3,
+// all wide, monopoles: 1990 and 113 ms (there the smaller records count).
+#define WIDE_ITEMS 4736
+__device__ __forceinline__ int wide_parts(int nwide, int ntop)
+{
+	return max(1, min(ntop, WIDE_ITEMS / max(nwide, 1)));
+}
+
+template <int TPL>
+__device__ void ewald_wide_item(const GroupParams &p, EwaldSmem &S, const tvg_wnode *__restrict__ wt,
+                                const uint32_t *__restrict__ ix, const uint32_t *__restrict__ iy,
+                                const uint32_t *__restrict__ iz, const float *__restrict__ mass_f,
+                                const GroupBox &g, const float *__restrict__ tab, int part, int parts,
+                                Target (&t)[TPL], double &nev, int nvalid, int *status)
+{
+	const int lane = threadIdx.x & 31;
+	const unsigned lt = (1u << lane) - 1u;
+	const float margin = 8.f * p.scale, hmax = fmaxf(g.hx, fmaxf(g.hy, g.hz));
+	const float l2 = p.inv_box * p.inv_box;
+	int sp = 0, nl = 0, root = part, guard = 0;
+	const int ntop = p.dc->ntop;
+	auto evaluate = [&](int from, int cnt) {
+		float ax[TPL], ay[TPL], az[TPL];
+#pragma unroll
+		for (int k = 0; k < TPL; k++) ax[k] = ay[k] = az[k] = 0.f;
+#pragma unroll 1
+		for (int e = 0; e < cnt; e++) {
+			const float4 s = S.list[from + e];
+			const float m0 = -s.w * p.inv_box * p.inv_box;
+#pragma unroll
+			for (int k = 0; k < TPL; k++)
+				ewald_k(p, tab, wrap_half(s.x - t[k].tx, p.box, p.half_box),
+				        wrap_half(s.y - t[k].ty, p.box, p.half_box), wrap_half(s.z - t[k].tz, p.box, p.half_box),
+				        m0, ax[k], ay[k], az[k]);
+		}
+#pragma unroll
+		for (int k = 0; k < TPL; k++) {
+			t[k].ax += (double) ax[k];
+			t[k].ay += (double) ay[k];
+			t[k].az += (double) az[k];
+		}
+		nev += (double) cnt * nvalid;
+		__syncwarp();
+	};
+	for (;;) {
+		if (sp == 0) {
+			if (root >= ntop) break;
+			int nr = 0;
+			for (; root < ntop && nr < GW_ROOTS; root += parts, nr++)
+				if (lane == 0) S.stack[nr] = root;
+			sp = nr;
+			__syncwarp();
+		}
+		if (++guard > p.max_iter) {
+			atomicOr(status, TVG_ST_TIMEOUT);
+			break;
+		}
+		bool stop;
+		const int node = pop_nodes(S.stack, sp, status, stop);
+		if (stop) break;
+		bool accept = false, open_int = false, open_bundle = false;
+		float4 entry = make_float4(0.f, 0.f, 0.f, 0.f);
+		int nchild = 0, child = 0;
+		if (node >= 0) {
+			const tvg_wnode nd = wt[node];
+			const float dx = ioff(nd.cx, g.cx, p.scale), dy = ioff(nd.cy, g.cy, p.scale),
+			            dz = ioff(nd.cz, g.cz, p.scale);
+			const float gx = ioff(nd.gx, g.cx, p.scale), gy = ioff(nd.gy, g.cy, p.scale),
+			            gz = ioff(nd.gz, g.cz, p.scale);
+			const float hs = 0.5f * nd.size + margin;
+			const bool straddle = fabsf(gx) + hs + g.hx > p.half_box || fabsf(gy) + hs + g.hy > p.half_box
+			                   || fabsf(gz) + hs + g.hz > p.half_box;
+			bool open;
+			if (straddle) {
+				float r2;
+				open = gravity_opens(p, g, nd, node, dx, dy, dz, gx, gy, gz, r2, false);
+			} else {
+				// monopole error of K: G M h2 s^2 / (8 L^4), as in ewald_group
+				const float rfar = (sqrtf(gx * gx + gy * gy + gz * gz) + nd.size + hmax) * p.inv_box;
+				const float hs2 = ewald_h2(rfar) * nd.size2 * l2;
+				open = p.use_bh ? hs2 > p.ew_bh : nd.mass * hs2 * 0.125f * l2 > p.ew_rel * g.fac;
+			}
+			if (!open) {
+				accept = true;
+				entry = make_float4(dx, dy, dz, p.gravity * nd.mass);
+			} else if (nd.nchild > 0) {
+				open_int = true;
+				nchild = nd.nchild;
+				child = nd.child;
+			} else {
+				open_bundle = true;
+				nchild = -nd.nchild;
+				child = nd.child;
+			}
+		}
+		const unsigned bm = __ballot_sync(0xFFFFFFFFu, accept);
+		if (accept) S.list[nl + __popc(bm & lt)] = entry;
+		nl += __popc(bm);               // below 64: fewer than 32 were left
+		push_children(S.stack, sp, open_int, nchild, child);
+		const unsigned bb = __ballot_sync(0xFFFFFFFFu, open_bundle);
+		if (open_bundle) S.bq[__popc(bb & lt)] = make_int2(child, nchild);
+		__syncwarp();
+		if (nl >= 32) {
+			nl -= 32;
+			evaluate(nl, 32);
+		}
+		for (int b = 0; b < __popc(bb); b++) {
+			const int2 q = S.bq[b];
+			for (int o = 0; o < q.y; o += 32) {
+				const int m = min(32, q.y - o);
+				if (lane < m) {
+					const int64_t jp = (int64_t) q.x + o + lane;
+					S.list[nl + lane] = make_float4(ioff(ix[jp], g.cx, p.scale), ioff(iy[jp], g.cy, p.scale),
+					                                ioff(iz[jp], g.cz, p.scale), p.gravity * mass_f[jp]);
+				}
+				nl += m;
+				__syncwarp();
+				if (nl >= 32) {
+					nl -= 32;
+					evaluate(nl, 32);
+				}
+			}
+		}
+		__syncwarp();
+	}
+	if (nl > 0) evaluate(0, nl);
+}
+
+template <int TPL, typename F>
+__global__ void __launch_bounds__(GE_THREADS, 4)
+k_ewald_wide(GroupParams p, const int32_t *__restrict__ active, const int32_t *__restrict__ gfirst,
+             const tvg_wnode *__restrict__ wt, const uint32_t *__restrict__ ix, const uint32_t *__restrict__ iy,
+             const uint32_t *__restrict__ iz, const float *__restrict__ mass_f,
+             const float *__restrict__ last_acc, const float *__restrict__ tab, F *acc0, F *acc1, F *acc2,
+             F *gacc0, F *gacc1, F *gacc2, const int32_t *__restrict__ wide, double *part, int32_t *work,
+             double *counter, int *status)
+{
+	extern __shared__ __align__(16) unsigned char smem_raw[];
+	EwaldSmem &S = ((EwaldSmem *) smem_raw)[threadIdx.x >> 5];
+	const int lane = threadIdx.x & 31, nwide = wide[0];
+	if (nwide == 0) return;
+	const int parts = wide_parts(nwide, p.dc->ntop);
+	double nev = 0;
+	for (;;) {
+		int item = 0;
+		if (lane == 0) item = atomicAdd(work, 1);
+		item = __shfl_sync(0xFFFFFFFFu, item, 0);
+		if (item >= nwide * parts) break;
+		const int w = item / parts;
+		const int64_t gi = wide[1 + w];
+		int64_t first;
+		int cnt;
+		if (gfirst) {
+			first = gfirst[gi];
+			cnt = (int) (gfirst[gi + 1] - first);
+		} else {
+			first = gi * p.gsize;
+			cnt = (int) min((int64_t) p.gsize, p.n - first);
+		}
+		Target t[TPL];
+		GroupBox g;
+		group_setup<TPL>(p, ix, iy, iz, last_acc, active, first, cnt, t, g);
+		ewald_wide_item<TPL>(p, S, wt, ix, iy, iz, mass_f, g, tab, item % parts, parts, t, nev, cnt, status);
+#pragma unroll
+		for (int k = 0; k < TPL; k++) {
+			const int slot = lane + 32 * k;
+			if (parts > 1) {
+				double *o = part + 3 * ((int64_t) item * p.gsize + slot);
+				o[0] = t[k].ax;
+				o[1] = t[k].ay;
+				o[2] = t[k].az;
+			} else if (t[k].valid) {
+				const int64_t i = active ? (int64_t) active[first + slot] : first + slot;
+				acc0[i] += (F) t[k].ax;
+				acc1[i] += (F) t[k].ay;
+				acc2[i] += (F) t[k].az;
+				gacc0[i] += (F) t[k].ax;
+				gacc1[i] += (F) t[k].ay;
+				gacc2[i] += (F) t[k].az;
+			}
+		}
+		__syncwarp();
+	}
+	if (lane == 0 && nev != 0) atomicAdd(counter, nev);
+}
+
+// the items' sums of each target, in item order
+template <typename F>
+__global__ void k_ewald_wide_sum(GroupParams p, const int32_t *__restrict__ active,
+                                 const int32_t *__restrict__ gfirst, const int32_t *__restrict__ wide,
+                                 const double *__restrict__ part, F *acc0, F *acc1, F *acc2, F *gacc0,
+                                 F *gacc1, F *gacc2)
+{
+	const int nwide = wide[0], parts = nwide ? wide_parts(nwide, p.dc->ntop) : 1;
+	if (parts <= 1) return;
+	for (int64_t e = blockIdx.x * (int64_t) blockDim.x + threadIdx.x; e < (int64_t) nwide * p.gsize;
+	     e += (int64_t) gridDim.x * blockDim.x) {
+		const int64_t w = e / p.gsize;
+		const int slot = (int) (e % p.gsize);
+		const int64_t gi = wide[1 + w];
+		const int64_t first = gfirst ? (int64_t) gfirst[gi] : gi * p.gsize;
+		const int64_t last = gfirst ? (int64_t) gfirst[gi + 1] : min(first + p.gsize, p.n);
+		if (first + slot >= last) continue;
+		double s[3] = { 0, 0, 0 };
+		for (int q = 0; q < parts; q++) {
+			const double *o = part + 3 * ((w * parts + q) * p.gsize + slot);
+			s[0] += o[0];
+			s[1] += o[1];
+			s[2] += o[2];
+		}
+		const int64_t i = active ? (int64_t) active[first + slot] : first + slot;
+		acc0[i] += (F) s[0];
+		acc1[i] += (F) s[1];
+		acc2[i] += (F) s[2];
+		gacc0[i] += (F) s[0];
+		gacc1[i] += (F) s[1];
+		gacc2[i] += (F) s[2];
+	}
 }
 
 template <typename F>
@@ -1925,13 +2144,28 @@ static int launch_ewald(tvg_context *ctx, GroupParams p, const float *mass_f, co
 	k_ewald_group<TPL, MLP, F><<<TVG_CNT(ctx, nblk), GE_THREADS, smem, ctx->stream>>>(
 	    p, ctx->use_active ? ctx->active : nullptr, ctx->use_active ? ctx->group_first : nullptr,
 	    ctx->wtree, ctx->ipos[0], ctx->ipos[1],
-	    ctx->ipos[2], mass_f, last_f, (const float4 *) ctx->ewald_ext,
-	    (const float4 *) ctx->ewald_taylor, (const __nv_bfloat16 *) ctx->mlp_bf16, ctx->mlp_prm,
+	    ctx->ipos[2], mass_f, last_f, (const float4 *) ctx->ewald_taylor, (const __nv_bfloat16 *) ctx->mlp_bf16, ctx->mlp_prm,
 	    (F *) ctx->f[FS_ACC0],
 	    (F *) ctx->f[FS_ACC1], (F *) ctx->f[FS_ACC2], (F *) ctx->f[FS_GACC0], (F *) ctx->f[FS_GACC1],
 	    (F *) ctx->f[FS_GACC2], ctx->work_counter + 1, counter, ctx->status,
-	    p.quad ? (const float4 *) ctx->wquad : nullptr);
+	    p.quad ? (const float4 *) ctx->wquad : nullptr, ctx->wide_list);
 	TVG_CUDA(ctx, cudaGetLastError());
+	if constexpr (!MLP) {
+		static int nwide_dev[TVG_MAX_DEVICES] = { 0 };
+		int &nb = nwide_dev[ctx->device];
+		const size_t sm = sizeof(EwaldSmem) * GE_WARPS;
+		TVG_CHECK(blocks_for(ctx, k_ewald_wide<TPL, F>, sm, &nb, GE_THREADS));
+		const int32_t *act = ctx->use_active ? ctx->active : nullptr, *gf = ctx->use_active ? ctx->group_first : nullptr;
+		F *a[6] = { (F *) ctx->f[FS_ACC0], (F *) ctx->f[FS_ACC1], (F *) ctx->f[FS_ACC2],
+		            (F *) ctx->f[FS_GACC0], (F *) ctx->f[FS_GACC1], (F *) ctx->f[FS_GACC2] };
+		k_ewald_wide<TPL, F><<<TVG_CNT(ctx, nb), GE_THREADS, sm, ctx->stream>>>(
+		    p, act, gf, ctx->wtree, ctx->ipos[0], ctx->ipos[1], ctx->ipos[2], mass_f, last_f, ctx->ewald_wide,
+		    a[0], a[1], a[2], a[3], a[4], a[5], ctx->wide_list, ctx->wide_part, ctx->work_counter + 2, counter,
+		    ctx->status);
+		k_ewald_wide_sum<F><<<TVG_CNT(ctx, 148), 256, 0, ctx->stream>>>(
+		    p, act, gf, ctx->wide_list, ctx->wide_part, a[0], a[1], a[2], a[3], a[4], a[5]);
+		TVG_CUDA(ctx, cudaGetLastError());
+	}
 	return TVG_OK;
 }
 
@@ -1981,7 +2215,15 @@ static int walk_group_typed(tvg_context *ctx, int use_bh, uint32_t parts, int ew
 		                "the table (tvg_ewald_mlp_validate)");
 	cudaStream_t s = ctx->stream;
 	if (!ctx->have_walktree) TVG_CHECK(prepare_typed<F>(ctx));
-	if (ewald && !ctx->ewald_ext) TVG_CHECK(tvg_impl_ewald_ext(ctx));
+	if (ewald && !mlp) {
+		if (!ctx->ewald_wide) TVG_CHECK(tvg_impl_ewald_wide(ctx));
+		// the list holds every group (at most one per 32 particles), the partial
+		// sums WIDE_ITEMS items of the largest groups
+		if (!ctx->wide_list)
+			TVG_CUDA(ctx, cudaMalloc((void **) &ctx->wide_list, 4 * (size_t) (ctx->cap / 32 + 1024)));
+		if (!ctx->wide_part) TVG_CUDA(ctx, cudaMalloc((void **) &ctx->wide_part, 24 * (size_t) WIDE_ITEMS * 128));
+		TVG_CUDA(ctx, cudaMemsetAsync(ctx->wide_list, 0, 4, s));
+	}
 	if (ewald && !ctx->ewald_taylor) TVG_CHECK(tvg_impl_ewald_taylor(ctx));
 	// FP32 copies of mass / last |a| (views when Float is float)
 	const float *mass_f = (const float *) ctx->f[FS_MASS];
@@ -2021,8 +2263,8 @@ static int walk_group_typed(tvg_context *ctx, int use_bh, uint32_t parts, int ew
 	p.inv_eps2 = (float) (1.0 / (h * h));
 	p.c16 = (float) (1.0 / (16.0 * h * h * h));
 	p.near2 = (float) (h * h * 1.001);
-	p.grid = (float) (cf.periodic ? 2.0 * 64.0 / cf.boxsize : 0.0);
 	p.inv_box = (float) (cf.periodic ? 1.0 / cf.boxsize : 0.0);
+	p.wide_grid = (float) (cf.periodic ? 2.0 * (TVG_WIDE_NODES - 1) / cf.boxsize : 0.0);
 	p.tay_grid = (float) (cf.periodic ? 2.0 * (TVG_TAYLOR_NODES - 1) / cf.boxsize : 0.0);
 	p.ew_rel = (float) (ctx->ewald_open_rel / cf.open_rel);   // times g.fac: alpha_E |a_old| / G
 	p.ew_bh = (float) (ctx->ewald_open_bh * cf.open_bh);
@@ -2040,7 +2282,7 @@ static int walk_group_typed(tvg_context *ctx, int use_bh, uint32_t parts, int ew
 		TVG_CUDA(ctx, cudaGetLastError());
 	}
 	TVG_CUDA(ctx, cudaMemsetAsync(ctx->counters, 0, 24, s));
-	TVG_CUDA(ctx, cudaMemsetAsync(ctx->work_counter, 0, 8, s));
+	TVG_CUDA(ctx, cudaMemsetAsync(ctx->work_counter, 0, 12, s));
 	TVG_CUDA(ctx, tvg_record(ctx, ctx->ev[0]));
 	double *cnt = ctx->counters;
 	if (tpl == 1) TVG_CHECK((launch_pair<1, F>(ctx, p, ewald, mlp, mass_f, last_f, cnt)));

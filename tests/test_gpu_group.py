@@ -297,3 +297,39 @@ def test_quadrupole_with_many_top_nodes():
     (t1, e1, _), (t8, e8, q8) = out
     assert t8 > 256 and t8 > 4 * t1 and q8 > 0
     assert e8 < 1.3 * e1 and e8 < 2e-3
+
+
+@pytest.mark.parametrize("fsize,flags", [(4, 0), (4, G.CFG_QUADRUPOLE), (8, 0)])
+@pytest.mark.parametrize("use_bh", [False, True])
+def test_wide_groups_split(fsize, flags, use_bh):
+    """In a box of 20^3 every group is wider than L/20 and takes per-target
+    images (k_ewald_wide). How many items a group is split into follows from
+    the number of such groups: a walk over a few windows of the order (64 items
+    each) must give the force that the walk over all of them (37 each) gives.
+    The order of the sums differs: FP32 sums of at most 32 entries carried in
+    FP64, whose partial sums are up to a few hundred times the net force at
+    z = 50, so 1e-4 of the largest component. The force itself against the
+    FP64 direct sum (relative criterion)."""
+    p = ics.zeldovich_box(n_side=20, seed=8)
+    n = p.n
+    parts = G.WALK_GRAVITY | G.WALK_EWALD
+    with G.GravityContext(n, float_bytes=fsize, periodic=True, boxsize=p.box, softening=p.softening,
+                          flags=flags, open_rel=5e-3) as ctx:
+        ctx.upload(p.pos, p.mass, last_acc=np.full(n, 0.02))
+        ctx.set_domain((0.0, 0.0, 0.0), p.box)
+        ctx.force_step(form=G.FORM_GROUP, use_bh=use_bh, parts=parts)
+        full = ctx.download(G.F_GRAV_ACC)["grav_acc"].astype(np.float64)
+        _, _, err = ctx.forcetest(np.arange(0, n, 8))
+        _, ew_all = ctx.walk_counters()
+        tot = 0.0
+        for lo, hi in ((0, 64), (64, 77), (3000, 3200), (n - 70, n)):
+            active = np.arange(lo, hi)
+            ctx.set_active(active)
+            ctx.walk(G.FORM_GROUP, use_bh=use_bh, parts=parts)
+            got = ctx.download(G.F_GRAV_ACC)["grav_acc"].astype(np.float64)
+            if lo % 64 == 0 and hi % 64 == 0:      # whole windows: the same groups
+                assert np.abs(got[:, active] - full[:, active]).max() < 1e-4 * np.abs(full).max()
+            tot += ctx.walk_counters()[1]
+        assert 0 < tot < ew_all
+    if not use_bh:
+        assert err["rms"] < 1e-2
