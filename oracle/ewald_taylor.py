@@ -1,6 +1,8 @@
-"""CPU restatement of the group form's Taylor table of the Ewald correction
-(tandav_b200/csrc/tvg_ewald.cu: k_ewald_fine, k_ewald_taylor; the lookup in
-tandav_b200/csrc/tvg_walk_group.cu: ewald_kjh_taylor).
+"""CPU restatement of the group form's Taylor tables of the Ewald correction
+(tandav_b200/csrc/tvg_ewald.cu: k_ewald_fine, k_ewald_taylor,
+k_ewald_wide_table; the lookups in tandav_b200/csrc/tvg_walk_group.cu:
+ewald_kjh, ewald_k). `record` takes the derivatives component by component;
+the tables hold its symmetric part (`tensors`, `compact`).
 
 TEST INFRASTRUCTURE ONLY: it checks the scheme (finite differences on a
 grid of half the node spacing, third-order expansion about the nearest node)
@@ -13,6 +15,8 @@ Record layout, 20 values per component a (node units u = 2 (N - 1) x):
 [10 + t] d3T_a for t in xxx yyy zzz xxy xxz yyx yyz zzx zzy xyz.
 """
 from __future__ import annotations
+
+import itertools
 
 import numpy as np
 
@@ -90,3 +94,47 @@ def evaluate(rec, du):
         grad[a] = r[1:4] + (H + D / 2) @ du
         val[a] = r[0] + du @ (r[1:4] + 0.5 * ((H + D / 3) @ du))
     return val, grad, hess
+
+
+def tensors(rec):
+    """dT, d2T and d3T of a record, each averaged over its index permutations
+    (T is a gradient): what a 32-float record of the table holds."""
+    B, C, D = np.zeros((3, 3)), np.zeros((3, 3, 3)), np.zeros((3, 3, 3, 3))
+    t3 = ("xxx", "yyy", "zzz", "xxy", "xxz", "xyy", "yyz", "xzz", "yzz", "xyz")
+    for a in range(3):
+        r = rec[20 * a:20 * a + 20]
+        B[a] = r[1:4]
+        for b in range(3):
+            C[a, b, b] = r[4 + b]
+        for q, (b, e) in enumerate(PAIRS):
+            C[a, b, e] = C[a, e, b] = r[7 + q]
+        for idx in np.ndindex(3, 3, 3):
+            D[(a,) + idx] = r[10 + t3.index("".join(sorted("xyz"[k] for k in idx)))]
+
+    def mean(t):
+        perms = list(itertools.permutations(range(t.ndim)))
+        return sum(np.transpose(t, p) for p in perms) / len(perms)
+
+    return rec[0::20][:3], mean(B), mean(C), mean(D)
+
+
+def compact(rec, nodes):
+    """The 24 numbers of the wide groups' table: the components with two z
+    more follow from the trace (4 pi for dT, in node units)."""
+    T, B, C, D = rec[0::20][:3], *tensors(rec)[1:]
+    B, C, D = B.copy(), C.copy(), D.copy()
+    B[2, 2] = 4 * np.pi / (2 * (nodes - 1)) - B[0, 0] - B[1, 1]
+    for a in range(3):
+        for idx in set(itertools.permutations((a, 2, 2))):
+            C[idx] = -C[a, 0, 0] - C[a, 1, 1]
+    for a, b in ((0, 0), (0, 1), (1, 1), (0, 2), (1, 2), (2, 2)):
+        for idx in set(itertools.permutations((a, b, 2, 2))):
+            D[idx] = -D[a, b, 0, 0] - D[a, b, 1, 1]
+    return T, B, C, D
+
+
+def evaluate_tensors(t, du):
+    """T, dT/du and d2T/du du at node + du from (T, dT, d2T, d3T)."""
+    T, B, C, D = t
+    d = D @ du
+    return T + (B + 0.5 * ((C + d / 3) @ du)) @ du, B + (C + d / 2) @ du, C + d

@@ -56,112 +56,128 @@ int tvg_impl_ewald_init(tvg_context *ctx)
 	return TVG_OK;
 }
 
-// Taylor table of the group form: at each node x = i / (2 (N - 1)) (box
-// units, i = 0..N-1 per axis, N = TVG_TAYLOR_NODES) of the octant, T and its
-// first three derivatives, the k-th derivative taken with respect to the node
-// coordinate u = 2 (N - 1) x (so scaled by the node spacing^k). Record of 64
-// floats, 20 per component a (then 4 pad):
-//   [20a] T_a; [20a + 1 + b] dT_a/du_b; [20a + 4 + s] d2T_a, s over
-//   xx yy zz xy xz yz; [20a + 10 + t] d3T_a, t over xxx yyy zzz xxy xxz yyx
-//   yyz zzx zzy xyz.
-// A lookup expands T about the nearest node (|du| <= 1/2 per axis): T to
-// third order, dT to second, d2T to first. With 33 nodes (spacing 1/64, a
-// 9.2 MB table that stays in L2) the value is within 4e-7 of |T| and the
-// gradient within 3e-5 of its largest component, against direct lattice sums
-// at off-node points across the octant (the origin, face, edge and corner
-// nodes included); with 65 nodes, 6e-8 and 7e-6. The derivatives are
-// finite differences of FP64 lattice sums on a grid of half the node spacing
-// (two ghost points beyond each end): fourth-order central differences for the
-// first and pure second derivatives, second-order ones for the mixed and third
-// derivatives (small correction terms); FP64 round-off enters as
-// ~1e-16 / delta^3, below 1e-8.
-#define N_TAY TVG_TAYLOR_NODES
-#define N_FINE (2 * (N_TAY - 1) + 1 + 4)
+// Lattice force T (the periodic lattice minus the image at the origin, box
+// units, unit G m) on the grid of half the node spacing of a table of `nodes`
+// nodes per axis, with two ghost points beyond each end (the analytic
+// continuation beyond L/2 and below 0). Evaluated for sorted coordinates only; the
+// others are their permutations.
+__host__ __device__ __forceinline__ int fine_points(int nodes) { return 2 * (nodes - 1) + 1 + 4; }
 
-__global__ void k_ewald_fine(double *fine)
+__global__ void k_ewald_fine(int nodes, double *fine)
 {
+	const int nf = fine_points(nodes);
 	const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-	if (idx >= N_FINE * N_FINE * N_FINE) return;
-	const int i = idx / (N_FINE * N_FINE), j = (idx / N_FINE) % N_FINE, k = idx % N_FINE;
-	const double d = 1.0 / (4.0 * (N_TAY - 1));
-	const double x[3] = { (i - 2) * d, (j - 2) * d, (k - 2) * d };
+	if (idx >= nf * nf * nf) return;
+	const int i[3] = { idx / (nf * nf), (idx / nf) % nf, idx % nf };
+	if (i[0] > i[1] || i[1] > i[2]) return;
+	const double d = 1.0 / (4.0 * (nodes - 1));
+	const double x[3] = { (i[0] - 2) * d, (i[1] - 2) * d, (i[2] - 2) * d };
 	double f[3], pot;
 	ewald_point(x, f, &pot);
-	fine[3 * (int64_t) idx + 0] = f[0];
-	fine[3 * (int64_t) idx + 1] = f[1];
-	fine[3 * (int64_t) idx + 2] = f[2];
+	const int perm[6][3] = { { 0, 1, 2 }, { 0, 2, 1 }, { 1, 0, 2 }, { 1, 2, 0 }, { 2, 0, 1 }, { 2, 1, 0 } };
+	for (int q = 0; q < 6; q++) {
+		const int *o = perm[q];
+		double *w = fine + 3 * (((int64_t) i[o[0]] * nf + i[o[1]]) * nf + i[o[2]]);
+		for (int a = 0; a < 3; a++) w[a] = f[o[a]];
+	}
 }
 
-__global__ void k_ewald_taylor(const double *__restrict__ fine, float *tay)
-{
-	const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-	if (idx >= N_TAY * N_TAY * N_TAY) return;
-	const int ni = idx / (N_TAY * N_TAY), nj = (idx / N_TAY) % N_TAY, nk = idx % N_TAY;
-	const int ci = 2 * ni + 2, cj = 2 * nj + 2, ck = 2 * nk + 2;
-	// fine spacing in node units: 1/2
-	const double h = 0.5, h2 = h * h, h3 = h2 * h;
-	float *r = tay + 64 * (int64_t) idx;
-	for (int a = 0; a < 3; a++) {
-		float *ra = r + 20 * a;
-		// component a at fine offsets from the node
-		auto f = [&](int di, int dj, int dk) {
-			return fine[3 * (((int64_t) (ci + di) * N_FINE + (cj + dj)) * N_FINE + (ck + dk)) + a];
-		};
-		auto g = [&](int b, int s) { return b == 0 ? f(s, 0, 0) : b == 1 ? f(0, s, 0) : f(0, 0, s); };
-		auto g2 = [&](int b, int sb, int e, int se) {
-			int d[3] = { 0, 0, 0 };
-			d[b] += sb;
-			d[e] += se;
-			return f(d[0], d[1], d[2]);
-		};
-		const double c = f(0, 0, 0);
-		ra[0] = (float) c;
-		for (int b = 0; b < 3; b++)
-			ra[1 + b] = (float) ((-g(b, 2) + 8 * g(b, 1) - 8 * g(b, -1) + g(b, -2)) / (12 * h));
-		for (int b = 0; b < 3; b++)
-			ra[4 + b] = (float) ((-g(b, 2) + 16 * g(b, 1) - 30 * c + 16 * g(b, -1) - g(b, -2)) / (12 * h2));
-		const int pr[3][2] = { { 0, 1 }, { 0, 2 }, { 1, 2 } };
-		for (int q = 0; q < 3; q++) {
-			const int b = pr[q][0], e = pr[q][1];
-			ra[7 + q] = (float) ((g2(b, 1, e, 1) - g2(b, 1, e, -1) - g2(b, -1, e, 1) + g2(b, -1, e, -1))
-			                     / (4 * h2));
-		}
-		for (int b = 0; b < 3; b++)
-			ra[10 + b] = (float) ((g(b, 2) - 2 * g(b, 1) + 2 * g(b, -1) - g(b, -2)) / (2 * h3));
-		// d3 T / db db de: the difference along e of the second differences along b
-		const int bbe[6][2] = { { 0, 1 }, { 0, 2 }, { 1, 0 }, { 1, 2 }, { 2, 0 }, { 2, 1 } };
-		for (int q = 0; q < 6; q++) {
-			const int b = bbe[q][0], e = bbe[q][1];
-			const double up = g2(b, 1, e, 1) - 2 * g2(b, 0, e, 1) + g2(b, -1, e, 1);
-			const double dn = g2(b, 1, e, -1) - 2 * g2(b, 0, e, -1) + g2(b, -1, e, -1);
-			ra[13 + q] = (float) ((up - dn) / (2 * h3));
-		}
+// Finite differences of T_a at fine point (ci, cj, ck), in node units (fine
+// spacing 1/2): fourth-order central differences for the first and pure second
+// derivatives, second-order ones for the mixed and third derivatives (small
+// correction terms); FP64 round-off enters as ~1e-16 / delta^3, below 1e-8.
+struct FineDiff {
+	const double *fine;
+	int nf, c[3];
+	__device__ double f(int a, int di, int dj, int dk) const
+	{
+		return fine[3 * (((int64_t) (c[0] + di) * nf + (c[1] + dj)) * nf + (c[2] + dk)) + a];
+	}
+	__device__ double g(int a, int b, int s) const
+	{
+		return b == 0 ? f(a, s, 0, 0) : b == 1 ? f(a, 0, s, 0) : f(a, 0, 0, s);
+	}
+	__device__ double g2(int a, int b, int sb, int e, int se) const
+	{
+		int d[3] = { 0, 0, 0 };
+		d[b] += sb;
+		d[e] += se;
+		return f(a, d[0], d[1], d[2]);
+	}
+	__device__ double d1(int a, int b) const
+	{
+		return (-g(a, b, 2) + 8 * g(a, b, 1) - 8 * g(a, b, -1) + g(a, b, -2)) / 6;
+	}
+	__device__ double d2(int a, int b) const
+	{
+		return (-g(a, b, 2) + 16 * g(a, b, 1) - 30 * f(a, 0, 0, 0) + 16 * g(a, b, -1) - g(a, b, -2)) / 3;
+	}
+	__device__ double d2m(int a, int b, int e) const
+	{
+		return g2(a, b, 1, e, 1) - g2(a, b, 1, e, -1) - g2(a, b, -1, e, 1) + g2(a, b, -1, e, -1);
+	}
+	__device__ double d3(int a, int b) const
+	{
+		return (g(a, b, 2) - 2 * g(a, b, 1) + 2 * g(a, b, -1) - g(a, b, -2)) * 4;
+	}
+	// d3 T_a / db db de: the difference along e of the second differences along b
+	__device__ double d3m(int a, int b, int e) const
+	{
+		const double up = g2(a, b, 1, e, 1) - 2 * g2(a, b, 0, e, 1) + g2(a, b, -1, e, 1);
+		const double dn = g2(a, b, 1, e, -1) - 2 * g2(a, b, 0, e, -1) + g2(a, b, -1, e, -1);
+		return (up - dn) * 4;
+	}
+	__device__ double d3xyz(int a) const
+	{
 		double s3 = 0;
 		for (int sx = -1; sx <= 1; sx += 2)
 			for (int sy = -1; sy <= 1; sy += 2)
-				for (int sz = -1; sz <= 1; sz += 2) s3 += sx * sy * sz * f(sx, sy, sz);
-		ra[19] = (float) (s3 / (8 * h3));
+				for (int sz = -1; sz <= 1; sz += 2) s3 += sx * sy * sz * f(a, sx, sy, sz);
+		return s3;
 	}
-	for (int q = 60; q < 64; q++) r[q] = 0.f;
+};
+
+__device__ __forceinline__ FineDiff fine_diff(const double *fine, int nodes, int idx)
+{
+	return { fine, fine_points(nodes),
+	         { 2 * (idx / (nodes * nodes)) + 2, 2 * ((idx / nodes) % nodes) + 2, 2 * (idx % nodes) + 2 } };
 }
 
-int tvg_impl_ewald_taylor(tvg_context *ctx)
+// Taylor table of the group form: at each node x = i / (2 (N - 1)) (box units, i
+// = 0..N-1 per axis, N = TVG_TAYLOR_NODES) of the octant, T and its first three
+// derivatives, the k-th with respect to the node coordinate u = 2 (N - 1) x. T is a
+// gradient, so the derivative tensors are symmetric: each entry is the mean of
+// the finite differences that approximate it. Record of 32 floats:
+//   Tx Ty Tz, dT xx yy zz xy xz yz, d2T xxx xxy xxz xyy xyz xzz yyy yyz yzz zzz,
+//   d3T xxxx yyyy zzzz xxyy xxzz yyzz xxxy xxxz xyyy yyyz xxyz xyyz (xyzz, xzzz and yzzz
+//   from the zero trace), 0.
+// A lookup expands T about the nearest node (|du| <= 1/2 per axis): T to third
+// order, dT to second, d2T to first. With 33 nodes (spacing 1/64) the value is
+// within 4e-7 of |T| and the gradient within 4e-5 rms of direct lattice sums at
+// off-node points across the octant.
+__global__ void k_ewald_taylor(const double *__restrict__ fine, float *tay)
 {
-	const size_t ntay = (size_t) N_TAY * N_TAY * N_TAY, nfine = (size_t) N_FINE * N_FINE * N_FINE;
-	if (!ctx->ewald_taylor) TVG_CUDA(ctx, cudaMalloc((void **) &ctx->ewald_taylor, 256 * ntay));
-	double *fine = nullptr;
-	TVG_CUDA(ctx, cudaMalloc((void **) &fine, 24 * nfine));
-	k_ewald_fine<<<TVG_CNT(ctx, tvg_blocks((int64_t) nfine, 128)), 128, 0, ctx->stream>>>(fine);
-	cudaError_t e = cudaGetLastError();
-	if (e == cudaSuccess) {
-		k_ewald_taylor<<<TVG_CNT(ctx, tvg_blocks((int64_t) ntay, 128)), 128, 0, ctx->stream>>>(
-		    fine, ctx->ewald_taylor);
-		e = cudaGetLastError();
-	}
-	if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
-	cudaFree(fine);
-	if (e != cudaSuccess) return tvg_fail(ctx, TVG_E_CUDA, "ewald taylor table: %s", cudaGetErrorString(e));
-	return TVG_OK;
+	const int idx = blockIdx.x * blockDim.x + threadIdx.x;
+	if (idx >= TVG_TAYLOR_NODES * TVG_TAYLOR_NODES * TVG_TAYLOR_NODES) return;
+	const FineDiff F = fine_diff(fine, TVG_TAYLOR_NODES, idx);
+	// the components that approximate d2T_bbe (b != e) and d3T_bbbe, d3T_bbee
+	auto c2 = [&](int b, int e) { return (F.d2(e, b) + 2 * F.d2m(b, b, e)) / 3; };
+	auto d31 = [&](int b, int e) { return (F.d3(e, b) + 3 * F.d3m(b, b, e)) / 4; };
+	auto d22 = [&](int b, int e) { return 0.5 * (F.d3m(b, e, b) + F.d3m(e, b, e)); };
+	auto d211 = [&](int b, int e, int f) {
+		return (F.d3m(f, b, e) + F.d3m(e, b, f) + 2 * F.d3xyz(b)) / 4;
+	};
+	const double v[32] = {
+		F.f(0, 0, 0, 0), F.f(1, 0, 0, 0), F.f(2, 0, 0, 0),
+		F.d1(0, 0), F.d1(1, 1), F.d1(2, 2), 0.5 * (F.d1(0, 1) + F.d1(1, 0)), 0.5 * (F.d1(0, 2) + F.d1(2, 0)),
+		0.5 * (F.d1(1, 2) + F.d1(2, 1)),
+		F.d2(0, 0), c2(0, 1), c2(0, 2), c2(1, 0), (F.d2m(0, 1, 2) + F.d2m(1, 0, 2) + F.d2m(2, 0, 1)) / 3,
+		c2(2, 0), F.d2(1, 1), c2(1, 2), c2(2, 1), F.d2(2, 2),
+		F.d3(0, 0), F.d3(1, 1), F.d3(2, 2), d22(0, 1), d22(0, 2), d22(1, 2), d31(0, 1), d31(0, 2), d31(1, 0),
+		d31(1, 2), d211(0, 1, 2), d211(1, 0, 2), 0
+	};
+	float *r = tay + 32 * (int64_t) idx;
+	for (int q = 0; q < 32; q++) r[q] = (float) v[q];
 }
 
 // Table of the lattice force for single points (the group form's wide groups,
@@ -176,83 +192,36 @@ int tvg_impl_ewald_taylor(tvg_context *ctx)
 //   xxxy xxxz yyyy xyyy yyyz xxyy xxyz xyyz.
 // With 41 nodes the third-order expansion about the nearest node is within
 // 5e-8 rms of direct lattice sums over the octant (tricubic: 8e-8, and 1.2e-7
-// with its FP32 sums). The lattice sums on the grid of half the spacing are
-// evaluated for sorted coordinates only; the others are their permutations.
-#define N_WIDE TVG_WIDE_NODES
-#define N_WFINE (2 * (N_WIDE - 1) + 1 + 4)
-
-__global__ void k_wide_fine(double *fine)
+// with its FP32 sums).
+__global__ void k_ewald_wide_table(const double *__restrict__ fine, float *tab)
 {
 	const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-	if (idx >= N_WFINE * N_WFINE * N_WFINE) return;
-	const int i[3] = { idx / (N_WFINE * N_WFINE), (idx / N_WFINE) % N_WFINE, idx % N_WFINE };
-	if (i[0] > i[1] || i[1] > i[2]) return;
-	const double d = 1.0 / (4.0 * (N_WIDE - 1));
-	const double x[3] = { (i[0] - 2) * d, (i[1] - 2) * d, (i[2] - 2) * d };
-	double f[3], pot;
-	ewald_point(x, f, &pot);
-	const int perm[6][3] = { { 0, 1, 2 }, { 0, 2, 1 }, { 1, 0, 2 }, { 1, 2, 0 }, { 2, 0, 1 }, { 2, 1, 0 } };
-	for (int q = 0; q < 6; q++) {
-		const int *o = perm[q];
-		double *w = fine + 3 * (((int64_t) i[o[0]] * N_WFINE + i[o[1]]) * N_WFINE + i[o[2]]);
-		for (int a = 0; a < 3; a++) w[a] = f[o[a]];
-	}
-}
-
-__global__ void k_wide_table(const double *__restrict__ fine, float *tab)
-{
-	const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-	if (idx >= N_WIDE * N_WIDE * N_WIDE) return;
-	const int ci = 2 * (idx / (N_WIDE * N_WIDE)) + 2, cj = 2 * ((idx / N_WIDE) % N_WIDE) + 2,
-	          ck = 2 * (idx % N_WIDE) + 2;
-	const double h = 0.5, h2 = h * h, h3 = h2 * h;       // fine spacing, node units
-	auto f = [&](int a, int di, int dj, int dk) {
-		return fine[3 * (((int64_t) (ci + di) * N_WFINE + (cj + dj)) * N_WFINE + (ck + dk)) + a];
-	};
-	auto g = [&](int a, int b, int s) {
-		return b == 0 ? f(a, s, 0, 0) : b == 1 ? f(a, 0, s, 0) : f(a, 0, 0, s);
-	};
-	auto g2 = [&](int a, int b, int sb, int e, int se) {
-		int d[3] = { 0, 0, 0 };
-		d[b] += sb;
-		d[e] += se;
-		return f(a, d[0], d[1], d[2]);
-	};
-	auto d1 = [&](int a, int b) { return (-g(a, b, 2) + 8 * g(a, b, 1) - 8 * g(a, b, -1) + g(a, b, -2)) / (12 * h); };
-	auto d2 = [&](int a, int b) {
-		return (-g(a, b, 2) + 16 * g(a, b, 1) - 30 * f(a, 0, 0, 0) + 16 * g(a, b, -1) - g(a, b, -2)) / (12 * h2);
-	};
-	auto d2m = [&](int a, int b, int e) {
-		return (g2(a, b, 1, e, 1) - g2(a, b, 1, e, -1) - g2(a, b, -1, e, 1) + g2(a, b, -1, e, -1)) / (4 * h2);
-	};
-	auto d3 = [&](int a, int b) { return (g(a, b, 2) - 2 * g(a, b, 1) + 2 * g(a, b, -1) - g(a, b, -2)) / (2 * h3); };
-	// d3 T_a / db db de
-	auto d3m = [&](int a, int b, int e) {
-		const double up = g2(a, b, 1, e, 1) - 2 * g2(a, b, 0, e, 1) + g2(a, b, -1, e, 1);
-		const double dn = g2(a, b, 1, e, -1) - 2 * g2(a, b, 0, e, -1) + g2(a, b, -1, e, -1);
-		return (up - dn) / (2 * h3);
+	if (idx >= TVG_WIDE_NODES * TVG_WIDE_NODES * TVG_WIDE_NODES) return;
+	const FineDiff F = fine_diff(fine, TVG_WIDE_NODES, idx);
+	const double v[24] = {
+		F.f(0, 0, 0, 0), F.f(1, 0, 0, 0), F.f(2, 0, 0, 0), F.d1(0, 0), F.d1(1, 1), F.d1(0, 1), F.d1(0, 2),
+		F.d1(1, 2),
+		F.d2(0, 0), F.d2(1, 0), F.d2(2, 0), F.d2(0, 1), (F.d2m(0, 1, 2) + F.d2m(1, 0, 2) + F.d2m(2, 0, 1)) / 3,
+		F.d2(1, 1), F.d2(2, 1), F.d3(0, 0),
+		F.d3(1, 0), F.d3(2, 0), F.d3(1, 1), F.d3(0, 1), F.d3(2, 1), 0.5 * (F.d3m(1, 0, 1) + F.d3m(0, 1, 0)),
+		F.d3m(2, 0, 1), F.d3m(2, 1, 0)
 	};
 	float *r = tab + 24 * (int64_t) idx;
-	const double v[24] = {
-		f(0, 0, 0, 0), f(1, 0, 0, 0), f(2, 0, 0, 0), d1(0, 0), d1(1, 1), d1(0, 1), d1(0, 2), d1(1, 2),
-		d2(0, 0), d2(1, 0), d2(2, 0), d2(0, 1), (d2m(0, 1, 2) + d2m(1, 0, 2) + d2m(2, 0, 1)) / 3, d2(1, 1), d2(2, 1),
-		d3(0, 0),
-		d3(1, 0), d3(2, 0), d3(1, 1), d3(0, 1), d3(2, 1), 0.5 * (d3m(1, 0, 1) + d3m(0, 1, 0)), d3m(2, 0, 1),
-		d3m(2, 1, 0)
-	};
 	for (int q = 0; q < 24; q++) r[q] = (float) v[q];
 }
 
-int tvg_impl_ewald_wide(tvg_context *ctx)
+// one of the two tables: the fine grid, then the records
+static int make_table(tvg_context *ctx, int nodes, size_t record, void (*kernel)(const double *, float *), float **out)
 {
-	const size_t n = (size_t) N_WIDE * N_WIDE * N_WIDE, nfine = (size_t) N_WFINE * N_WFINE * N_WFINE;
+	const int nf = fine_points(nodes);
+	const int64_t n = (int64_t) nodes * nodes * nodes, nfine = (int64_t) nf * nf * nf;
 	double *fine = nullptr;
-	TVG_CUDA(ctx, cudaMalloc((void **) &fine, 24 * nfine));
+	TVG_CUDA(ctx, cudaMalloc((void **) &fine, 24 * (size_t) nfine));
 	float *tab = nullptr;
-	cudaError_t e = cudaMalloc((void **) &tab, 96 * n);
+	cudaError_t e = cudaMalloc((void **) &tab, record * (size_t) n);
 	if (e == cudaSuccess) {
-		k_wide_fine<<<TVG_CNT(ctx, tvg_blocks((int64_t) nfine, 128)), 128, 0, ctx->stream>>>(fine);
-		k_wide_table<<<TVG_CNT(ctx, tvg_blocks((int64_t) n, 128)), 128, 0, ctx->stream>>>(fine, tab);
+		k_ewald_fine<<<TVG_CNT(ctx, tvg_blocks(nfine, 128)), 128, 0, ctx->stream>>>(nodes, fine);
+		kernel<<<TVG_CNT(ctx, tvg_blocks(n, 128)), 128, 0, ctx->stream>>>(fine, tab);
 		e = cudaGetLastError();
 		const cudaError_t es = cudaStreamSynchronize(ctx->stream);
 		if (e == cudaSuccess) e = es;
@@ -260,10 +229,20 @@ int tvg_impl_ewald_wide(tvg_context *ctx)
 	cudaFree(fine);
 	if (e != cudaSuccess) {
 		cudaFree(tab);
-		return tvg_fail(ctx, TVG_E_CUDA, "ewald table of the wide groups: %s", cudaGetErrorString(e));
+		return tvg_fail(ctx, TVG_E_CUDA, "ewald taylor table: %s", cudaGetErrorString(e));
 	}
-	ctx->ewald_wide = tab;
+	*out = tab;
 	return TVG_OK;
+}
+
+int tvg_impl_ewald_taylor(tvg_context *ctx)
+{
+	return make_table(ctx, TVG_TAYLOR_NODES, 128, k_ewald_taylor, &ctx->ewald_taylor);
+}
+
+int tvg_impl_ewald_wide(tvg_context *ctx)
+{
+	return make_table(ctx, TVG_WIDE_NODES, 96, k_ewald_wide_table, &ctx->ewald_wide);
 }
 
 // raw Float tables (box units) -> device tables, as after

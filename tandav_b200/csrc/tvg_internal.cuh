@@ -188,7 +188,7 @@ struct tvg_context {
 	// sums of WIDE_ITEMS items
 	int32_t *wide_list = nullptr;
 	double *wide_part = nullptr;
-	float *ewald_taylor = nullptr;     // T and 3 derivatives at TVG_TAYLOR_NODES^3 nodes, 64 floats each
+	float *ewald_taylor = nullptr;     // T and 3 derivatives at TVG_TAYLOR_NODES^3 nodes, 32 floats each
 	// Ewald-walk opening of the group form: the monopole error of the
 	// correction may reach ewald_open_rel |a_old| (relative mode); the limit of
 	// h2 s^2 / L^2 in units of TREE_OPEN_PARAM_BH (Barnes-Hut mode)

@@ -30,9 +30,9 @@
 // for the same image: Newton + K is the lattice force, which is smooth across
 // the half-box plane, so no target needs its own image. K is evaluated by a
 // second, per-group traversal (k_ewald_group): at the centre of mass of each
-// accepted node it evaluates K, its Jacobian J and Hessian H (tricubic
-// interpolation of the lattice sum tabulated on the octant, with the
-// analytic continuation one cell beyond L/2), sums them over the group's
+// accepted node it evaluates K, its Jacobian J and Hessian H (a third-order
+// expansion of the lattice sum about the nearest node of a table on the octant,
+// with the analytic continuation beyond L/2), sums them over the group's
 // nodes, and each target adds the second-order Taylor expansion
 // K - J t + H:tt/2 about the group centre. Nodes are opened for K by their
 // own error estimate (the monopole error of K, G M h2 s^2 / (8 L^4) with h2 a
@@ -77,14 +77,10 @@
 #define GW_ROOTS 256        // top nodes pushed at a time
 #define GW_ELIST 64
 #define GW_DEFAULT_TPL 2
-// resident blocks per SM the table-evaluating Ewald walk is compiled for:
-// 4 (128 registers, 8 B of spill: 15.2 against 15.8 ms per step at 256^3
-// with 3 blocks of 168 registers, and 18.4 ms with 2 blocks of 206, since
-// the uniform remainder is a polynomial). Before that,
-// capping the registers had made it slower, with the tricubic lookup (1340,
-// 1442 ms against 1252 ms per step) and with the Taylor table and the closed
-// form (140.4 against 136.9 ms at 128^3). The learned correction's walk keeps
-// 1 (its network needs the registers).
+// resident blocks per SM the table-evaluating Ewald walk is compiled for: 4 / 5 /
+// 6 take 10.1 / 9.5 / 10.8 ms of a 256^3 step with quadrupoles and 19.5 / 20.3 /
+// 20.2 ms of a 64^3 step with monopoles. The learned correction's walk keeps 1 (its
+// network needs the registers).
 #ifndef GW_EWALD_MINB
 #define GW_EWALD_MINB 4
 #endif
@@ -480,69 +476,13 @@ struct EwaldSmem {
 	int2 bq[GW_BQ];
 };
 
-// Per-warp stage of the Ewald walk's Taylor records (table evaluation),
-// compiled in with GW_EWALD_STAGE=1: a full batch of 32 accepted sources has
-// its 32 records (256 B each) copied from the table in global memory into
-// shared memory by the bulk-copy (TMA) engine, cp.async.bulk completing on an
-// mbarrier, while the warp goes on walking; the batch is evaluated from
-// shared memory when the next one is issued. Two buffers: a new batch is
-// issued before the pending one is evaluated. Sources are this GPU's own
-// memory; no multicast. The results are those of the direct loads bit for
-// bit, but the walk is slower (768 against 462 ms per 256^3 step): the
-// records of neighbouring groups are reused through L1, which bulk copies
-// bypass and the 92 KB stage per block shrinks. Off by default.
-#ifndef GW_EWALD_STAGE
-#define GW_EWALD_STAGE 0
-#endif
-struct EwaldStage {
-	float4 rec[2][32][16];     // the batches' records
-	float4 pend[2][32];        // the batches' sources
-	uint64_t bar[2];           // completion barriers (arrival count 1 + transaction bytes)
-};
-
-__device__ __forceinline__ uint32_t smem_addr(const void *p)
-{
-	return (uint32_t) __cvta_generic_to_shared(p);
-}
-
-__device__ __forceinline__ void mbar_init(uint64_t *bar, uint32_t count)
-{
-	asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(bar)), "r"(count) : "memory");
-}
-
-__device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t *bar, uint32_t bytes)
-{
-	asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)), "r"(bytes)
-	             : "memory");
-}
-
-__device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, uint32_t parity)
-{
-	uint32_t done;
-	asm volatile("{\n\t.reg .pred p;\n\t"
-	             "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-	             "selp.u32 %0, 1, 0, p;\n\t}"
-	             : "=r"(done)
-	             : "r"(smem_addr(bar)), "r"(parity)
-	             : "memory");
-	return done != 0;
-}
-
-// 1-D bulk copy global -> shared (16-byte aligned addresses, size a multiple
-// of 16), completing `bytes` transactions on the mbarrier
-__device__ __forceinline__ void bulk_g2s(void *dst, const void *src, uint32_t bytes, uint64_t *bar)
-{
-	asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-	             ::"r"(smem_addr(dst)), "l"(src), "r"(bytes), "r"(smem_addr(bar))
-	             : "memory");
-}
-
 // per-lane sums over accepted sources of m K, m J and m H (about the group
-// centre), FP32 (a few hundred terms per lane)
+// centre), FP32 (a few hundred terms per lane). K is a gradient, so J and H are
+// symmetric.
 struct CorrSum {
 	float k[3];
-	float j[9];     // J[a][b] = dK_a / dd_b
-	float h[18];    // H[a][xx, yy, zz, xy, xz, yz]
+	float j[6];     // J: xx yy zz xy xz yz
+	float h[10];    // H: xxx xxy xxz xyy xyz xzz yyy yyz yzz zzz
 };
 
 struct Target {
@@ -1106,104 +1046,150 @@ k_walk_group(GroupParams p, const int32_t *__restrict__ active, const int32_t *_
 // looked up at |d| with the symmetries T_a(.., -x_b, ..) = -T_a if a = b,
 // +T_a otherwise.
 
-// K(d), its Jacobian J and Hessian H, summed into c, from the Taylor table
-// (tvg_ewald.cu, k_ewald_taylor): the record of the node nearest to |d| holds
-// T and its first three derivatives in node units; with D = d3T . du, the
-// value is T + du . (dT + 1/2 (d2T + D/3) du), the gradient dT + (d2T + D/2)
-// du and the second derivatives d2T + D (exact for a cubic). With OVR the
-// value is ovr (T at |d| from the learned correction) instead.
-// K_a = -s_a T_a, J_ab = -s_a s_b g dT_a/du_b, H_abc = -s_a s_b s_c g^2
-// d2T_a/du_b du_c, all times G m / L^2 (s the signs of d, g node spacings per
-// length).
-// index of the Taylor-table record nearest to |d| (node units)
-__device__ __forceinline__ int taylor_record(const GroupParams &p, float4 e)
-{
-	const int i = min(__float2int_rn(fabsf(e.x) * p.tay_grid), TVG_TAYLOR_NODES - 1);
-	const int j = min(__float2int_rn(fabsf(e.y) * p.tay_grid), TVG_TAYLOR_NODES - 1);
-	const int l = min(__float2int_rn(fabsf(e.z) * p.tay_grid), TVG_TAYLOR_NODES - 1);
-	return (i * TVG_TAYLOR_NODES + j) * TVG_TAYLOR_NODES + l;
-}
+// The record of the Taylor table (tvg_impl_ewald_taylor, tvg_ewald.cu) at the
+// node nearest to |d|, and |d|'s offset from the node in node units: T, dT (xx yy
+// zz xy xz yz), d2T (xxx xxy xxz xyy xyz xzz yyy yyz yzz zzz) and d3T (xxxx yyyy
+// zzzz xxyy xxzz yyzz xxxy xxxz xyyy yyyz xxyz xyyz; xyzz, xzzz and yzzz follow from the
+// zero trace). The lanes of a warp read as many records, one L1 wavefront for
+// each of their 32-byte loads, which bounds the evaluation: 4 loads, where the
+// tensors component by component took 60 numbers in fifteen 16-byte loads (64^3
+// box, monopoles: 44.8 -> 19.5 ms; 256^3, quadrupoles: 16.6 -> 10.1 ms).
+struct EwRec {
+	float t[3], B[6], C[10], D[12];
+	float x, y, z;
+};
 
-// STAGED: the record is `staged` (shared memory) instead of the table entry.
-// SQ (TVG_CFG_QUADRUPOLE): srcq is the source node's stored -G Q (two float4,
-// null for a particle), and the value also takes the node's quadrupole term,
-// the second-order term of the expansion about its centre of mass:
-// sum_j m_j y_b y_c / 2 d2K_a/dd_b dd_c = Q_bc / 6 d2K_a/dd_b dd_c (d2K_a is
-// traceless: the lattice sum's divergence is constant away from the source).
-template <bool OVR, bool STAGED = false, bool SQ = false>
-__device__ __forceinline__ void ewald_kjh_taylor(const GroupParams &p, const float4 *__restrict__ tay,
-                                                 float4 e, CorrSum &c, const float *ovr,
-                                                 const float4 *staged = nullptr,
-                                                 const float4 *__restrict__ srcq = nullptr)
+__device__ __forceinline__ EwRec ewald_record(const GroupParams &p, const float *__restrict__ tab, float4 e)
 {
-	const float sg[3] = { e.x < 0.f ? -1.f : 1.f, e.y < 0.f ? -1.f : 1.f, e.z < 0.f ? -1.f : 1.f };
+	EwRec r;
 	const float u = fabsf(e.x) * p.tay_grid, v = fabsf(e.y) * p.tay_grid, w = fabsf(e.z) * p.tay_grid;
 	const int i = min(__float2int_rn(u), TVG_TAYLOR_NODES - 1);
 	const int j = min(__float2int_rn(v), TVG_TAYLOR_NODES - 1);
 	const int l = min(__float2int_rn(w), TVG_TAYLOR_NODES - 1);
-	const float du = u - (float) i, dv = v - (float) j, dw = w - (float) l;
-	const float4 *rec = STAGED ? staged : tay + 16 * ((i * TVG_TAYLOR_NODES + j) * TVG_TAYLOR_NODES + l);
-	const float m0 = -e.w * p.inv_box * p.inv_box, m1 = m0 * p.tay_grid, m2 = m1 * p.tay_grid;
-	float4 q0 = make_float4(0.f, 0.f, 0.f, 0.f), q1 = q0;
-	if (SQ && srcq) {
-		q0 = __ldg(srcq);
-		q1 = __ldg(srcq + 1);
-		q0.w *= 2.f * sg[0] * sg[1];      // both off-diagonal terms, with their signs
-		q1.x *= 2.f * sg[0] * sg[2];
-		q1.y *= 2.f * sg[1] * sg[2];
-	}
-	const float mq = p.tay_grid * p.tay_grid * p.inv_box * p.inv_box * (1.f / 6.f);
+	r.x = u - (float) i;
+	r.y = v - (float) j;
+	r.z = w - (float) l;
+	const float *rec = tab + 32 * ((i * TVG_TAYLOR_NODES + j) * TVG_TAYLOR_NODES + l);
+	float pad;
+	asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+	    : "=f"(r.t[0]), "=f"(r.t[1]), "=f"(r.t[2]), "=f"(r.B[0]), "=f"(r.B[1]), "=f"(r.B[2]), "=f"(r.B[3]),
+	      "=f"(r.B[4])
+	    : "l"(rec));
+	asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+	    : "=f"(r.B[5]), "=f"(r.C[0]), "=f"(r.C[1]), "=f"(r.C[2]), "=f"(r.C[3]), "=f"(r.C[4]), "=f"(r.C[5]),
+	      "=f"(r.C[6])
+	    : "l"(rec + 8));
+	asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+	    : "=f"(r.C[7]), "=f"(r.C[8]), "=f"(r.C[9]), "=f"(r.D[0]), "=f"(r.D[1]), "=f"(r.D[2]), "=f"(r.D[3]),
+	      "=f"(r.D[4])
+	    : "l"(rec + 16));
+	asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+	    : "=f"(r.D[5]), "=f"(r.D[6]), "=f"(r.D[7]), "=f"(r.D[8]), "=f"(r.D[9]), "=f"(r.D[10]), "=f"(r.D[11]),
+	      "=f"(pad)
+	    : "l"(rec + 24));
+	(void) pad;
+	return r;
+}
+
+// d = D u: xxx xxy xxz xyy xyz xzz yyy yyz yzz zzz
+__device__ __forceinline__ void ewald_third(const EwRec &r, float d[10])
+{
+	const float *D = r.D;
+	const float xyzz = -D[6] - D[8], xzzz = -D[7] - D[11], yzzz = -D[10] - D[9];
+	d[0] = fmaf(D[0], r.x, fmaf(D[6], r.y, D[7] * r.z));
+	d[1] = fmaf(D[6], r.x, fmaf(D[3], r.y, D[10] * r.z));
+	d[2] = fmaf(D[7], r.x, fmaf(D[10], r.y, D[4] * r.z));
+	d[3] = fmaf(D[3], r.x, fmaf(D[8], r.y, D[11] * r.z));
+	d[4] = fmaf(D[10], r.x, fmaf(D[11], r.y, xyzz * r.z));
+	d[5] = fmaf(D[4], r.x, fmaf(xyzz, r.y, xzzz * r.z));
+	d[6] = fmaf(D[8], r.x, fmaf(D[1], r.y, D[9] * r.z));
+	d[7] = fmaf(D[11], r.x, fmaf(D[9], r.y, D[5] * r.z));
+	d[8] = fmaf(xyzz, r.x, fmaf(D[5], r.y, yzzz * r.z));
+	d[9] = fmaf(xzzz, r.x, fmaf(yzzz, r.y, D[2] * r.z));
+}
+
+// n = B + f (C + g d) u: xx yy zz xy xz yz
+__device__ __forceinline__ void ewald_first(const EwRec &r, const float d[10], float f, float g, float n[6])
+{
+	float m[10];
 #pragma unroll
-	for (int q = 0; q < 3; q++) {
-		float4 r0, r1, r2, r3, r4;
-		if (STAGED) {
-			r0 = rec[5 * q]; r1 = rec[5 * q + 1]; r2 = rec[5 * q + 2]; r3 = rec[5 * q + 3]; r4 = rec[5 * q + 4];
-		} else {
-			r0 = __ldg(rec + 5 * q); r1 = __ldg(rec + 5 * q + 1); r2 = __ldg(rec + 5 * q + 2);
-			r3 = __ldg(rec + 5 * q + 3); r4 = __ldg(rec + 5 * q + 4);
-		}
-		// D_bc = sum_d d3T_bcd du_d
-		const float dxx = fmaf(r2.z, du, fmaf(r3.y, dv, r3.z * dw));
-		const float dyy = fmaf(r3.w, du, fmaf(r2.w, dv, r4.x * dw));
-		const float dzz = fmaf(r4.y, du, fmaf(r4.z, dv, r3.x * dw));
-		const float dxy = fmaf(r3.y, du, fmaf(r3.w, dv, r4.w * dw));
-		const float dxz = fmaf(r3.z, du, fmaf(r4.w, dv, r4.y * dw));
-		const float dyz = fmaf(r4.w, du, fmaf(r4.x, dv, r4.z * dw));
-		const float hxx = r1.x + dxx, hyy = r1.y + dyy, hzz = r1.z + dzz;
-		const float hxy = r1.w + dxy, hxz = r2.x + dxz, hyz = r2.y + dyz;
-		// gradient: dT + (d2T + D/2) du
-		const float gx = r0.y + fmaf(fmaf(0.5f, dxx, r1.x), du, fmaf(fmaf(0.5f, dxy, r1.w), dv,
-		                              fmaf(0.5f, dxz, r2.x) * dw));
-		const float gy = r0.z + fmaf(fmaf(0.5f, dxy, r1.w), du, fmaf(fmaf(0.5f, dyy, r1.y), dv,
-		                              fmaf(0.5f, dyz, r2.y) * dw));
-		const float gz = r0.w + fmaf(fmaf(0.5f, dxz, r2.x), du, fmaf(fmaf(0.5f, dyz, r2.y), dv,
-		                              fmaf(0.5f, dzz, r1.z) * dw));
-		// value: T + du . (dT + 1/2 (d2T + D/3) du)
-		const float t3 = 1.f / 3.f;
-		const float bx = fmaf(fmaf(t3, dxx, r1.x), du, fmaf(fmaf(t3, dxy, r1.w), dv, fmaf(t3, dxz, r2.x) * dw));
-		const float by = fmaf(fmaf(t3, dxy, r1.w), du, fmaf(fmaf(t3, dyy, r1.y), dv, fmaf(t3, dyz, r2.y) * dw));
-		const float bz = fmaf(fmaf(t3, dxz, r2.x), du, fmaf(fmaf(t3, dyz, r2.y), dv, fmaf(t3, dzz, r1.z) * dw));
-		const float val = OVR ? ovr[q]
-		                      : r0.x + fmaf(fmaf(0.5f, bx, r0.y), du, fmaf(fmaf(0.5f, by, r0.z), dv,
-		                                                                    fmaf(0.5f, bz, r0.w) * dw));
-		const float sq = sg[q];
-		c.k[q] = fmaf(m0 * sq, val, c.k[q]);
-		if (SQ) {
-			// per unit G m, d2K_a/dd_b dd_c = -s_a s_b s_c h_bc tay_grid^2 / L^2;
-			// with G Q = -(stored), the term is mq s_a sum_bc stored_bc s_b s_c h_bc
-			const float hq = fmaf(q0.x, hxx, fmaf(q0.y, hyy, fmaf(q0.z, hzz,
-			                 fmaf(q0.w, hxy, fmaf(q1.x, hxz, q1.y * hyz)))));
-			c.k[q] = fmaf(mq * sq, hq, c.k[q]);
-		}
-		c.j[3 * q + 0] = fmaf(m1 * sq * sg[0], gx, c.j[3 * q + 0]);
-		c.j[3 * q + 1] = fmaf(m1 * sq * sg[1], gy, c.j[3 * q + 1]);
-		c.j[3 * q + 2] = fmaf(m1 * sq * sg[2], gz, c.j[3 * q + 2]);
-		c.h[6 * q + 0] = fmaf(m2 * sq, hxx, c.h[6 * q + 0]);
-		c.h[6 * q + 1] = fmaf(m2 * sq, hyy, c.h[6 * q + 1]);
-		c.h[6 * q + 2] = fmaf(m2 * sq, hzz, c.h[6 * q + 2]);
-		c.h[6 * q + 3] = fmaf(m2 * sq * sg[0] * sg[1], hxy, c.h[6 * q + 3]);
-		c.h[6 * q + 4] = fmaf(m2 * sq * sg[0] * sg[2], hxz, c.h[6 * q + 4]);
-		c.h[6 * q + 5] = fmaf(m2 * sq * sg[1] * sg[2], hyz, c.h[6 * q + 5]);
+	for (int q = 0; q < 10; q++) m[q] = fmaf(g, d[q], r.C[q]);
+	const float x = f * r.x, y = f * r.y, z = f * r.z;
+	n[0] = fmaf(m[0], x, fmaf(m[1], y, fmaf(m[2], z, r.B[0])));
+	n[1] = fmaf(m[3], x, fmaf(m[6], y, fmaf(m[7], z, r.B[1])));
+	n[2] = fmaf(m[5], x, fmaf(m[8], y, fmaf(m[9], z, r.B[2])));
+	n[3] = fmaf(m[1], x, fmaf(m[3], y, fmaf(m[4], z, r.B[3])));
+	n[4] = fmaf(m[2], x, fmaf(m[4], y, fmaf(m[5], z, r.B[4])));
+	n[5] = fmaf(m[4], x, fmaf(m[7], y, fmaf(m[8], z, r.B[5])));
+}
+
+// K(d), its Jacobian J and Hessian H, summed into c: value, gradient and
+// second derivatives of the record's expansion (third, second and first
+// order). With OVR the value is ovr (T at |d| from the learned correction).
+// K_a = -s_a T_a, J_ab = -s_a s_b g dT_a/du_b, H_abc = -s_a s_b s_c g^2
+// d2T_a/du_b du_c, all times G m / L^2 (s the signs of d, g node spacings per
+// length). SQ (TVG_CFG_QUADRUPOLE): srcq is the source node's stored -G Q (two
+// float4, null for a particle), and the value also takes the node's quadrupole
+// term, the second-order term of the expansion about its centre of mass:
+// sum_j m_j y_b y_c / 2 d2K_a/dd_b dd_c = Q_bc / 6 d2K_a/dd_b dd_c (d2K_a is
+// traceless: the lattice sum's divergence is constant away from the source).
+template <bool OVR, bool SQ = false>
+__device__ __forceinline__ void ewald_kjh(const GroupParams &p, const float *__restrict__ tab, float4 e,
+                                          CorrSum &c, const float *ovr,
+                                          const float4 *__restrict__ srcq = nullptr)
+{
+	const EwRec r = ewald_record(p, tab, e);
+	const float sx = e.x < 0.f ? -1.f : 1.f, sy = e.y < 0.f ? -1.f : 1.f, sz = e.z < 0.f ? -1.f : 1.f;
+	const float m0 = -e.w * p.inv_box * p.inv_box, m1 = m0 * p.tay_grid, m2 = m1 * p.tay_grid;
+	float d[10], n[6], v[3];
+	ewald_third(r, d);
+	if (OVR) {
+		v[0] = ovr[0];
+		v[1] = ovr[1];
+		v[2] = ovr[2];
+	} else {
+		// T + u . (dT + 1/2 (d2T + D u / 3) u)
+		ewald_first(r, d, 0.5f, 1.f / 3.f, n);
+		v[0] = r.t[0] + fmaf(n[0], r.x, fmaf(n[3], r.y, n[4] * r.z));
+		v[1] = r.t[1] + fmaf(n[3], r.x, fmaf(n[1], r.y, n[5] * r.z));
+		v[2] = r.t[2] + fmaf(n[4], r.x, fmaf(n[5], r.y, n[2] * r.z));
+	}
+	c.k[0] = fmaf(m0 * sx, v[0], c.k[0]);
+	c.k[1] = fmaf(m0 * sy, v[1], c.k[1]);
+	c.k[2] = fmaf(m0 * sz, v[2], c.k[2]);
+	ewald_first(r, d, 1.f, 0.5f, n);
+	const float sxy = sx * sy, sxz = sx * sz, syz = sy * sz;
+	c.j[0] = fmaf(m1, n[0], c.j[0]);
+	c.j[1] = fmaf(m1, n[1], c.j[1]);
+	c.j[2] = fmaf(m1, n[2], c.j[2]);
+	c.j[3] = fmaf(m1 * sxy, n[3], c.j[3]);
+	c.j[4] = fmaf(m1 * sxz, n[4], c.j[4]);
+	c.j[5] = fmaf(m1 * syz, n[5], c.j[5]);
+#pragma unroll
+	for (int q = 0; q < 10; q++) d[q] += r.C[q];
+	const float hx = m2 * sx, hy = m2 * sy, hz = m2 * sz;
+	c.h[0] = fmaf(hx, d[0], c.h[0]);
+	c.h[1] = fmaf(hy, d[1], c.h[1]);
+	c.h[2] = fmaf(hz, d[2], c.h[2]);
+	c.h[3] = fmaf(hx, d[3], c.h[3]);
+	c.h[4] = fmaf(hx * syz, d[4], c.h[4]);
+	c.h[5] = fmaf(hx, d[5], c.h[5]);
+	c.h[6] = fmaf(hy, d[6], c.h[6]);
+	c.h[7] = fmaf(hz, d[7], c.h[7]);
+	c.h[8] = fmaf(hy, d[8], c.h[8]);
+	c.h[9] = fmaf(hz, d[9], c.h[9]);
+	if (SQ && srcq) {
+		// per unit G m, d2K_a/dd_b dd_c = -s_a s_b s_c d_abc tay_grid^2 / L^2; with
+		// G Q = -(stored), the term is mq s_a sum_bc stored_bc s_b s_c d_abc
+		const float4 q0 = __ldg(srcq), q1 = __ldg(srcq + 1);
+		const float mq = p.tay_grid * p.tay_grid * p.inv_box * p.inv_box * (1.f / 6.f);
+		const float qxy = 2.f * sxy * q0.w, qxz = 2.f * sxz * q1.x, qyz = 2.f * syz * q1.y;
+		c.k[0] = fmaf(mq * sx, fmaf(q0.x, d[0], fmaf(q0.y, d[3], fmaf(q0.z, d[5],
+		              fmaf(qxy, d[1], fmaf(qxz, d[2], qyz * d[4]))))), c.k[0]);
+		c.k[1] = fmaf(mq * sy, fmaf(q0.x, d[1], fmaf(q0.y, d[6], fmaf(q0.z, d[8],
+		              fmaf(qxy, d[3], fmaf(qxz, d[4], qyz * d[7]))))), c.k[1]);
+		c.k[2] = fmaf(mq * sz, fmaf(q0.x, d[2], fmaf(q0.y, d[7], fmaf(q0.z, d[9],
+		              fmaf(qxy, d[4], fmaf(qxz, d[5], qyz * d[8]))))), c.k[2]);
 	}
 }
 
@@ -1327,7 +1313,7 @@ __device__ __noinline__ void mlp_forward_warp_call(const float *mlp, const uint3
 // wq (TVG_CFG_QUADRUPOLE, groups without per-target images): the walk
 // nodes' stored quadrupoles, lnode the list entries' nodes
 template <int TPL, bool MLP>
-__device__ __forceinline__ void ewald_batch(const GroupParams &p, const float4 *tay, const float *mlp, const uint32_t *w2b, const float4 *list,
+__device__ __forceinline__ void ewald_batch(const GroupParams &p, const float *tay, const float *mlp, const uint32_t *w2b, const float4 *list,
                                             int from, int cnt, bool per_target, CorrSum &c,
                                             Target (&t)[TPL], float &nev,
                                             const int32_t *lnode = nullptr,
@@ -1347,13 +1333,13 @@ __device__ __forceinline__ void ewald_batch(const GroupParams &p, const float4 *
 			float tv[3];
 			mlp_forward_warp(mlp, w2b, xs, tv);
 			if (lane < cnt) {
-				if (wq) ewald_kjh_taylor<true, false, true>(p, tay, e, c, tv, nullptr, srcq);
-				else ewald_kjh_taylor<true>(p, tay, e, c, tv);
+				if (wq) ewald_kjh<true, true>(p, tay, e, c, tv, srcq);
+				else ewald_kjh<true>(p, tay, e, c, tv);
 				nev += 1.f;
 			}
 		} else if (lane < cnt) {
-			if (wq) ewald_kjh_taylor<false, false, true>(p, tay, list[from + lane], c, nullptr, nullptr, srcq);
-			else ewald_kjh_taylor<false>(p, tay, list[from + lane], c, nullptr);
+			if (wq) ewald_kjh<false, true>(p, tay, list[from + lane], c, nullptr, srcq);
+			else ewald_kjh<false>(p, tay, list[from + lane], c, nullptr);
 			nev += 1.f;
 		}
 	} else if constexpr (MLP) {
@@ -1386,77 +1372,15 @@ __device__ __forceinline__ void ewald_batch(const GroupParams &p, const float4 *
 	}
 }
 
-// pipeline state of a warp's record stage (uniform across its lanes)
-struct StageState {
-	uint32_t phase;    // bit b: parity of buffer b's next completion
-	int cur;           // the buffer the next batch goes to
-	bool pending;      // the other buffer holds an issued batch
-	bool ok;           // false after a wait gave up: no more staging
-};
-
-// bounded wait for buffer b's copies (TVG_ST_TIMEOUT when they never land)
-__device__ __forceinline__ bool stage_wait(EwaldStage *st, int b, StageState &ss, int *status)
-{
-	const uint32_t par = (ss.phase >> b) & 1u;
-	for (int it = 0; !mbar_try_wait(&st->bar[b], par);) {
-		if (++it > (1 << 20)) {
-			atomicOr(status, TVG_ST_TIMEOUT);
-			ss.ok = false;
-			return false;
-		}
-	}
-	ss.phase ^= 1u << b;
-	return true;
-}
-
-__device__ __forceinline__ void stage_eval(const GroupParams &p, EwaldStage *st, int b, CorrSum &c, float &nev)
-{
-	const int lane = threadIdx.x & 31;
-	ewald_kjh_taylor<false, true>(p, nullptr, st->pend[b][lane], c, nullptr, &st->rec[b][lane][0]);
-	nev += 1.f;
-}
-
-// a full batch of 32 sources (list[from + lane]) goes to the free buffer;
-// then the batch issued before it is evaluated. Every lane copies its own
-// record; lane 0 posts the batch's 8 KB on the buffer's barrier first.
-__device__ __forceinline__ void stage_batch(const GroupParams &p, const float4 *__restrict__ tay,
-                                            EwaldStage *st, const float4 *list, int from, StageState &ss,
-                                            CorrSum &c, float &nev, int *status)
-{
-	const int lane = threadIdx.x & 31;
-	const float4 e = list[from + lane];
-	const int b = ss.cur;
-	if (lane == 0) mbar_arrive_expect_tx(&st->bar[b], 32 * 16 * sizeof(float4));
-	__syncwarp();
-	st->pend[b][lane] = e;
-	// this lane read the slot as generic memory when the buffer was last
-	// evaluated: order that before the bulk copy writes it
-	asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-	bulk_g2s(&st->rec[b][lane][0], tay + 16 * taylor_record(p, e), 16 * sizeof(float4), &st->bar[b]);
-	if (ss.pending && stage_wait(st, b ^ 1, ss, status)) stage_eval(p, st, b ^ 1, c, nev);
-	ss.pending = true;
-	ss.cur = b ^ 1;
-	__syncwarp();
-}
-
-// evaluates the batch still in flight (end of a group)
-__device__ __forceinline__ void stage_drain(const GroupParams &p, EwaldStage *st, StageState &ss, CorrSum &c,
-                                            float &nev, int *status)
-{
-	if (ss.pending && stage_wait(st, ss.cur ^ 1, ss, status)) stage_eval(p, st, ss.cur ^ 1, c, nev);
-	ss.pending = false;
-	__syncwarp();
-}
-
 template <int TPL, bool MLP>
 __device__ void ewald_group(const GroupParams &p, EwaldSmem &S, const tvg_wnode *__restrict__ wt,
                             const uint32_t *__restrict__ ix, const uint32_t *__restrict__ iy,
                             const uint32_t *__restrict__ iz, const float *__restrict__ mass_f,
-                            const float *__restrict__ last_acc, const float4 *__restrict__ tay,
+                            const float *__restrict__ last_acc, const float *__restrict__ tay,
                             const float *mlp, const uint32_t *w2b,
                             int64_t first, int cnt, const int32_t *__restrict__ active,
-                            Target (&t)[TPL], float &nev, EwaldStage *st, StageState &ss, int *status,
-                            const float4 *__restrict__ wq_all, int64_t group, int32_t *wide)
+                            Target (&t)[TPL], float &nev, int *status, const float4 *__restrict__ wq_all,
+                            int64_t group, int32_t *wide)
 {
 	const int lane = threadIdx.x & 31;
 	const unsigned lt = (1u << lane) - 1u;
@@ -1473,7 +1397,6 @@ __device__ void ewald_group(const GroupParams &p, EwaldSmem &S, const tvg_wnode 
 	// node quadrupoles (TVG_CFG_QUADRUPOLE) in the expansion about the group
 	// centre; per-target images evaluate K alone and keep monopoles
 	const float4 *wq = per_target ? nullptr : wq_all;
-	if (wq) st = nullptr;
 	// straddling: the node (and, with per-target images, the group box) reaches
 	// the half-box plane; then the gravity walk's decision is repeated
 	const float margin = 8.f * p.scale;
@@ -1483,9 +1406,9 @@ __device__ void ewald_group(const GroupParams &p, EwaldSmem &S, const tvg_wnode 
 #pragma unroll
 	for (int a = 0; a < 3; a++) c.k[a] = 0.f;
 #pragma unroll
-	for (int a = 0; a < 9; a++) c.j[a] = 0.f;
+	for (int a = 0; a < 6; a++) c.j[a] = 0.f;
 #pragma unroll
-	for (int a = 0; a < 18; a++) c.h[a] = 0.f;
+	for (int a = 0; a < 10; a++) c.h[a] = 0.f;
 
 	int sp = 0, nl = 0, r0 = 0;
 	const int ntop = p.dc->ntop;
@@ -1580,8 +1503,7 @@ __device__ void ewald_group(const GroupParams &p, EwaldSmem &S, const tvg_wnode 
 			const bool full = nl >= 32;
 			if (full || (final && nl > 0)) {
 				const int cnt = full ? 32 : nl;
-				if (full && st && ss.ok && !per_target) stage_batch(p, tay, st, S.list, nl - 32, ss, c, nev, status);
-				else ewald_batch<TPL, MLP>(p, tay, mlp, w2b, S.list, nl - cnt, cnt, per_target, c, t, nev,
+				ewald_batch<TPL, MLP>(p, tay, mlp, w2b, S.list, nl - cnt, cnt, per_target, c, t, nev,
 				                           S.lnode, wq);
 				nl -= cnt;
 				continue;
@@ -1613,36 +1535,35 @@ __device__ void ewald_group(const GroupParams &p, EwaldSmem &S, const tvg_wnode 
 		__syncwarp();
 		if (final) break;
 	}
-	if (st && ss.ok) stage_drain(p, st, ss, c, nev, status);
 	if (per_target) return;
 	// sum over lanes (FP64), then K(d_c - t) ~ K - J t + H:tt / 2 per target
-	double K[3], J[9], H[18];
+	double K[3], J[6], H[10];
 #pragma unroll
 	for (int a = 0; a < 3; a++) K[a] = c.k[a];
 #pragma unroll
-	for (int a = 0; a < 9; a++) J[a] = c.j[a];
+	for (int a = 0; a < 6; a++) J[a] = c.j[a];
 #pragma unroll
-	for (int a = 0; a < 18; a++) H[a] = c.h[a];
+	for (int a = 0; a < 10; a++) H[a] = c.h[a];
 #pragma unroll
 	for (int o = 16; o; o >>= 1) {
 #pragma unroll
 		for (int a = 0; a < 3; a++) K[a] += __shfl_xor_sync(0xFFFFFFFFu, K[a], o);
 #pragma unroll
-		for (int a = 0; a < 9; a++) J[a] += __shfl_xor_sync(0xFFFFFFFFu, J[a], o);
+		for (int a = 0; a < 6; a++) J[a] += __shfl_xor_sync(0xFFFFFFFFu, J[a], o);
 #pragma unroll
-		for (int a = 0; a < 18; a++) H[a] += __shfl_xor_sync(0xFFFFFFFFu, H[a], o);
+		for (int a = 0; a < 10; a++) H[a] += __shfl_xor_sync(0xFFFFFFFFu, H[a], o);
 	}
 #pragma unroll
 	for (int k = 0; k < TPL; k++) {
 		const double x = t[k].tx, y = t[k].ty, z = t[k].tz;
+		const double xx = 0.5 * x * x, yy = 0.5 * y * y, zz = 0.5 * z * z, xy = x * y, xz = x * z, yz = y * z;
 		double out[3];
-#pragma unroll
-		for (int a = 0; a < 3; a++) {
-			const double *h = H + 6 * a;
-			out[a] = K[a] - (J[3 * a] * x + J[3 * a + 1] * y + J[3 * a + 2] * z)
-			       + 0.5 * (h[0] * x * x + h[1] * y * y + h[2] * z * z)
-			       + h[3] * x * y + h[4] * x * z + h[5] * y * z;
-		}
+		out[0] = K[0] - (J[0] * x + J[3] * y + J[4] * z)
+		       + (H[0] * xx + H[3] * yy + H[5] * zz + H[1] * xy + H[2] * xz + H[4] * yz);
+		out[1] = K[1] - (J[3] * x + J[1] * y + J[5] * z)
+		       + (H[1] * xx + H[6] * yy + H[8] * zz + H[3] * xy + H[4] * xz + H[7] * yz);
+		out[2] = K[2] - (J[4] * x + J[5] * y + J[2] * z)
+		       + (H[2] * xx + H[7] * yy + H[9] * zz + H[4] * xy + H[5] * xz + H[8] * yz);
 		double rem[3];
 		uniform_remainder(p, x, y, z, rem);
 		out[0] += rem[0];
@@ -1660,7 +1581,7 @@ k_ewald_group(GroupParams p, const int32_t *__restrict__ active, const int32_t *
               const tvg_wnode *__restrict__ wt,
               const uint32_t *__restrict__ ix, const uint32_t *__restrict__ iy,
               const uint32_t *__restrict__ iz, const float *__restrict__ mass_f,
-              const float *__restrict__ last_acc, const float4 *__restrict__ tay,
+              const float *__restrict__ last_acc, const float *__restrict__ tay,
               const __nv_bfloat16 *__restrict__ mlp_w, const float *__restrict__ mlp_f32, F *acc0, F *acc1,
               F *acc2, F *gacc0, F *gacc1, F *gacc2, int32_t *work, double *counter, int *status,
               const float4 *__restrict__ wq, int32_t *wide)
@@ -1676,20 +1597,6 @@ k_ewald_group(GroupParams p, const int32_t *__restrict__ active, const int32_t *
 		__syncthreads();
 	}
 	const int lane = threadIdx.x & 31;
-	// with GW_EWALD_STAGE the table path stages its records (EwaldStage after
-	// the warps' areas)
-	EwaldStage *st = (MLP || !GW_EWALD_STAGE)
-	                     ? nullptr
-	                     : ((EwaldStage *) (smem_raw + sizeof(EwaldSmem) * GE_WARPS)) + (threadIdx.x >> 5);
-	StageState ss = { 0u, 0, false, true };
-	if (st) {
-		if (lane == 0) {
-			mbar_init(&st->bar[0], 1);
-			mbar_init(&st->bar[1], 1);
-			asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-		}
-		__syncwarp();
-	}
 	double ev_acc = 0;
 	const int64_t ngroups = p.dc->ngroups;
 	for (;;) {
@@ -1709,7 +1616,7 @@ k_ewald_group(GroupParams p, const int32_t *__restrict__ active, const int32_t *
 		Target t[TPL];
 		float nev = 0.f;
 		ewald_group<TPL, MLP>(p, S, wt, ix, iy, iz, mass_f, last_acc, tay, mlp, w2b, first, cnt, active, t, nev,
-		                      st, ss, status, wq, g, wide);
+		                      status, wq, g, wide);
 		ev_acc += nev;
 #pragma unroll
 		for (int k = 0; k < TPL; k++) {
@@ -2139,12 +2046,12 @@ static int launch_ewald(tvg_context *ctx, GroupParams p, const float *mass_f, co
 	TVG_CHECK(device_slot(ctx));
 	int &nblk = nblk_dev[ctx->device];
 	const size_t smem = sizeof(EwaldSmem) * GE_WARPS
-	                  + (MLP ? 4 * MLP_NPARAM + 2 * MLP_H * MLP_H : (GW_EWALD_STAGE ? sizeof(EwaldStage) * GE_WARPS : 0));
+	                  + (MLP ? 4 * MLP_NPARAM + 2 * MLP_H * MLP_H : 0);
 	TVG_CHECK(blocks_for(ctx, k_ewald_group<TPL, MLP, F>, smem, &nblk, GE_THREADS));
 	k_ewald_group<TPL, MLP, F><<<TVG_CNT(ctx, nblk), GE_THREADS, smem, ctx->stream>>>(
 	    p, ctx->use_active ? ctx->active : nullptr, ctx->use_active ? ctx->group_first : nullptr,
 	    ctx->wtree, ctx->ipos[0], ctx->ipos[1],
-	    ctx->ipos[2], mass_f, last_f, (const float4 *) ctx->ewald_taylor, (const __nv_bfloat16 *) ctx->mlp_bf16, ctx->mlp_prm,
+	    ctx->ipos[2], mass_f, last_f, ctx->ewald_taylor, (const __nv_bfloat16 *) ctx->mlp_bf16, ctx->mlp_prm,
 	    (F *) ctx->f[FS_ACC0],
 	    (F *) ctx->f[FS_ACC1], (F *) ctx->f[FS_ACC2], (F *) ctx->f[FS_GACC0], (F *) ctx->f[FS_GACC1],
 	    (F *) ctx->f[FS_GACC2], ctx->work_counter + 1, counter, ctx->status,
