@@ -134,7 +134,7 @@ extern "C" int tvg_init(int device, const tvg_config *cfg, tvg_context **out)
 	TVG_CHECK(dalloc(ctx, (void **) &ctx->pref, 8 * 4 * (cap + 1)));
 	for (int k = 0; k < 3; k++) TVG_CHECK(dalloc(ctx, (void **) &ctx->ipos[k], 4 * cap));
 	TVG_CHECK(dalloc(ctx, (void **) &ctx->wtree, sizeof(tvg_wnode) * ctx->tcap));
-	TVG_CHECK(dalloc(ctx, (void **) &ctx->big_list, 4 * (ctx->tcap + 1)));
+	TVG_CHECK(dalloc(ctx, (void **) &ctx->big_list, 4 * (ctx->tcap + 2)));
 	TVG_CHECK(dalloc(ctx, (void **) &ctx->group_first, 4 * (cap / 8 + 1024)));
 	TVG_CHECK(dalloc(ctx, (void **) &ctx->work_counter, 64));
 	TVG_CHECK(dalloc(ctx, (void **) &ctx->counters, 8 * 8));
