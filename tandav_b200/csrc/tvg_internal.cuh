@@ -84,6 +84,7 @@ struct tvg_devcount {
 	int32_t ntop;            // top nodes
 	int32_t max_active_bin;  // bins <= this are active
 	int32_t sort_skip[8];    // radix digit d is the same for all keys
+	uint32_t sort_tiles[8];  // tiles taken by digit d's pass
 	int64_t nwchild;         // walk nodes below the top nodes (TVG_CFG_QUADRUPOLE)
 };
 
@@ -139,9 +140,9 @@ struct tvg_context {
 	// key split for the sort
 	uint64_t *key_hi = nullptr, *key_lo = nullptr, *key_tmp = nullptr;
 	uint32_t *perm = nullptr, *perm_tmp = nullptr;
-	uint32_t *sort_hist = nullptr;     // per-tile digit histograms
-	uint32_t *sort_off = nullptr;      // scanned
-	uint32_t *digit_count = nullptr;   // 8 x 256 global digit histogram
+	uint32_t *sort_hist = nullptr;     // tile states of the even radix passes (256 a tile)
+	uint32_t *sort_off = nullptr;      // and of the odd ones
+	uint32_t *digit_count = nullptr;   // 8 x 256 global digit histogram, then offsets
 	void *scan_tmp = nullptr;
 	size_t scan_tmp_bytes = 0;
 	int *status = nullptr;             // device status word

@@ -3,14 +3,16 @@
 // Replaces Qsort_Index on the 128-bit keys (sort.c:90-341, cmp_peanoKeys at
 // peano.c:6-12) and reorder_collisionless_particles (peano.c:50-82).
 //  1. LSD radix sort of (key_hi, index) on the 64-bit high key word: 8-bit
-//     digits; a digit that is equal for every key (decided on the device) is
-//     not ranked: its pass copies the keys through, so the number of passes,
-//     and with it the buffer a step ends in, never depends on the data. Each
-//     pass is
-//     reduce-then-scan: per-tile (4096 keys) digit histograms, one device
-//     scan of the digit-major histogram, then a scatter in which every tile
-//     ranks its keys stably with warp __match_any_sync and writes them through
-//     a shared-memory staging sort (coalesced runs per digit).
+//     digits, one kernel per digit (k_radix_pass). All eight digit histograms are
+//     counted in one pass over the keys beforehand; a pass takes tiles of 4096 keys
+//     in the order of a device counter, ranks a tile's keys stably with warp
+//     matches, finds the tile's place among the equal digits of earlier tiles by
+//     looking back over their published counts, and writes through a
+//     shared-memory staging sort (coalesced runs per digit). A digit that is
+//     equal for every key (decided on the device) is not ranked: its pass copies
+//     the keys through, so the number of passes, and with it the buffer a step
+//     ends in, never depends on the data. Up to one tile of keys is sorted by one
+//     block in shared memory (k_sort_tile).
 //  2. Runs of equal high words are ordered by the low word (insertion sort
 //     per run, one thread per run; runs are rare and short unless positions
 //     coincide).
@@ -20,8 +22,11 @@
 // The resulting order is the ascending 128-bit key order, equal keys in
 // input order (the reference's quicksort leaves equal keys in an
 // unspecified order).
-// Roofline: HBM bound; per pass 8 B read (histogram) + 12 B read + 12 B write
-// per key.
+// Roofline: HBM bound; per pass 12 B read + 12 B write per key. Histogram, scan
+// and scatter kernels per digit (three to five launches, 20 B read) took, with
+// the gather of the fields, 4.65 ms for 16.7M particles, 0.47 ms for 400,000 and
+// 0.28 ms for 3001; this 2.80, 0.22 and 0.06 ms (a pass over 16.7M keys 243 us, 1.7
+// TB/s, bound by the warp matches of the ranking).
 #include <mutex>
 
 #include "tvg_internal.cuh"
@@ -30,12 +35,6 @@
 #define RS_IPT 16
 #define RS_TILE (RS_THREADS * RS_IPT)
 #define RS_WARPS (RS_THREADS / 32)
-
-__global__ void k_iota(int64_t n, uint32_t *p)
-{
-	int64_t i = blockIdx.x * (int64_t) blockDim.x + threadIdx.x;
-	if (i < n) p[i] = (uint32_t) i;
-}
 
 // global histogram of all 8 digits of key_hi (to skip constant digits)
 __global__ void k_digit_counts(int64_t n, const uint64_t *__restrict__ key, uint32_t *count)
@@ -54,154 +53,237 @@ __global__ void k_digit_counts(int64_t n, const uint64_t *__restrict__ key, uint
 		if (h[i]) atomicAdd(&count[i], h[i]);
 }
 
-// skip[d] = 1 when digit d has the same value in all n keys
-__global__ void k_digit_skip(int64_t n, const uint32_t *__restrict__ count, int32_t *skip)
+// A block per digit: its counts to exclusive offsets, skip[d] = 1 when the digit
+// has the same value in all n keys, and the pass's tile counter to zero.
+__global__ void __launch_bounds__(256) k_digit_offsets(int64_t n, uint32_t *count, int32_t *skip, uint32_t *tiles)
 {
-	const int d = threadIdx.x;
-	if (d >= 8) return;
-	int sk = 0;
-	for (int b = 0; b < 256; b++)
-		if (count[d * 256 + b] == (uint32_t) n) sk = 1;
-	skip[d] = sk;
+	__shared__ uint32_t s_warp[8];
+	const int d = blockIdx.x, t = threadIdx.x, lane = t & 31, w = t >> 5;
+	const uint32_t c = count[d * 256 + t];
+	const int all = __syncthreads_or(c == (uint32_t) n);
+	uint32_t inc = c;
+#pragma unroll
+	for (int o = 1; o < 32; o <<= 1) {
+		const uint32_t u = __shfl_up_sync(0xFFFFFFFFu, inc, o);
+		if (lane >= o) inc += u;
+	}
+	if (lane == 31) s_warp[w] = inc;
+	__syncthreads();
+	for (int k = 0; k < w; k++) inc += s_warp[k];
+	count[d * 256 + t] = inc - c;
+	if (t == 0) {
+		skip[d] = all;
+		tiles[d] = 0;
+	}
 }
 
-// per-tile digit histogram, stored digit-major: hist[d * ntiles + tile]
-// (zeros for a digit that skip marks)
-__global__ void k_tile_hist(int64_t n, int shift, const uint64_t *__restrict__ key,
-                            uint32_t *__restrict__ hist, int64_t ntiles,
-                            const int32_t *__restrict__ skip = nullptr)
+// exclusive prefix sum of one value per thread of a 256-thread block
+__device__ __forceinline__ uint32_t scan256(uint32_t v, uint32_t *s_warp)
 {
-	if (skip && skip[shift >> 3]) {
-		hist[(int64_t) threadIdx.x * ntiles + blockIdx.x] = 0;
-		return;
+	const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+	uint32_t inc = v;
+#pragma unroll
+	for (int o = 1; o < 32; o <<= 1) {
+		const uint32_t u = __shfl_up_sync(0xFFFFFFFFu, inc, o);
+		if (lane >= o) inc += u;
 	}
-	__shared__ uint32_t h[256];
-	h[threadIdx.x] = 0;
+	if (lane == 31) s_warp[w] = inc;
 	__syncthreads();
-	const int64_t base = (int64_t) blockIdx.x * RS_TILE;
-#pragma unroll 4
-	for (int k = 0; k < RS_IPT; k++) {
-		int64_t i = base + (int64_t) k * RS_THREADS + threadIdx.x;
-		if (i < n) {
-			uint32_t d = (uint32_t) (key[i] >> shift) & 0xFF;
-			unsigned peers = __match_any_sync(__activemask(), d);
-			int leader = __ffs(peers) - 1;
-			if ((int) (threadIdx.x & 31) == leader) atomicAdd(&h[d], (uint32_t) __popc(peers));
+	uint32_t base = 0;
+#pragma unroll
+	for (int k = 0; k < RS_WARPS; k++) base += k < w ? s_warp[k] : 0u;
+	return base + inc - v;
+}
+
+// Ranks a tile's digits: a warp holds RS_IPT x 32 consecutive keys, key r of
+// lane l at r * 32 + l; whist[w][d] counts digit d of warp w as it goes, so that
+// rank[r] is the key's place among the equal digits of its warp. Returns with
+// whist holding, per digit, the offset of each warp among the tile's equal
+// digits, and in thread t the tile's count of digit t.
+__device__ __forceinline__ uint32_t rank_tile(const uint32_t (&d)[RS_IPT], uint32_t (&rank)[RS_IPT],
+                                              uint32_t (*whist)[256])
+{
+	const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+	const unsigned lt = (1u << lane) - 1u;
+#pragma unroll
+	for (int k = 0; k < RS_WARPS; k++) whist[k][t] = 0;
+	__syncthreads();
+#pragma unroll
+	for (int r = 0; r < RS_IPT; r++) {
+		const unsigned peers = __match_any_sync(0xFFFFFFFFu, d[r]);
+		const int leader = __ffs(peers) - 1;
+		uint32_t old = 0;
+		if (lane == leader && d[r] < 256) {
+			old = whist[w][d[r]];
+			whist[w][d[r]] = old + (uint32_t) __popc(peers);
 		}
+		old = __shfl_sync(0xFFFFFFFFu, old, leader);
+		rank[r] = old + (uint32_t) __popc(peers & lt);
+		__syncwarp();
 	}
 	__syncthreads();
-	hist[(int64_t) threadIdx.x * ntiles + blockIdx.x] = h[threadIdx.x];
+	uint32_t run = 0;
+#pragma unroll
+	for (int k = 0; k < RS_WARPS; k++) {
+		const uint32_t c = whist[k][t];
+		whist[k][t] = run;
+		run += c;
+	}
+	return run;
 }
 
-__global__ void __launch_bounds__(RS_THREADS)
-k_radix_scatter(int64_t n, int shift, const uint64_t *__restrict__ kin,
-                const uint32_t *__restrict__ vin, uint64_t *__restrict__ kout,
-                uint32_t *__restrict__ vout, const uint32_t *__restrict__ off, int64_t ntiles,
-                const int32_t *__restrict__ skip = nullptr)
+// published state of (tile, digit): the tile's count, or the count of all tiles
+// up to it; 0: not published yet
+#define RS_COUNT 0x40000000u
+#define RS_TOTAL 0x80000000u
+#define RS_VALUE 0x3FFFFFFFu
+// polls of one predecessor's state before the pass gives up (about a second);
+// tiles are taken in order, so the predecessors run or have run
+#define RS_SPIN (1 << 21)
+
+// One digit's pass. state: ntiles x 256 words of this pass, zero at its start;
+// next: those of the next pass, zeroed here. vin null: the values are the
+// indices.
+__global__ void __launch_bounds__(RS_THREADS, 3)
+k_radix_pass(int64_t n, int shift, const uint64_t *__restrict__ kin, const uint32_t *__restrict__ vin,
+             uint64_t *__restrict__ kout, uint32_t *__restrict__ vout, const uint32_t *__restrict__ offsets,
+             volatile uint32_t *state, uint32_t *__restrict__ next, uint32_t *tiles,
+             const int32_t *__restrict__ skip, int *status)
 {
-	if (skip && skip[shift >> 3]) {     // constant digit: the order stays
+	__shared__ __align__(16) uint64_t skey[RS_TILE];     // keys, then values
+	__shared__ uint32_t whist[RS_WARPS][256];
+	__shared__ uint32_t dstart[256], gstart[256], s_warp[RS_WARPS], s_tile;
+	const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+	next[(int64_t) blockIdx.x * 256 + t] = 0;
+	if (skip[shift >> 3]) {                              // constant digit: the order stays
 		const int64_t b0 = (int64_t) blockIdx.x * RS_TILE;
 		const int c0 = (int) min((int64_t) RS_TILE, n - b0);
-		for (int p = threadIdx.x; p < c0; p += RS_THREADS) {
+		for (int p = t; p < c0; p += RS_THREADS) {
 			kout[b0 + p] = kin[b0 + p];
-			vout[b0 + p] = vin[b0 + p];
+			vout[b0 + p] = vin ? vin[b0 + p] : (uint32_t) (b0 + p);
 		}
 		return;
 	}
-	extern __shared__ __align__(16) unsigned char smem[];
-	uint64_t *skey = (uint64_t *) smem;                          // RS_TILE
-	uint32_t *sval = (uint32_t *) (skey + RS_TILE);              // RS_TILE
-	uint32_t *whist = sval + RS_TILE;                            // RS_WARPS * 256
-	uint32_t *dstart = whist + RS_WARPS * 256;                   // 256
-	uint32_t *gstart = dstart + 256;                             // 256
-	uint32_t *running = gstart + 256;                            // 256
-	int32_t *s_warp = (int32_t *) (running + 256);               // 33
-
-	const int t = threadIdx.x, lane = t & 31, w = t >> 5;
-	const int64_t base = (int64_t) blockIdx.x * RS_TILE;
+	if (t == 0) s_tile = atomicAdd(&tiles[shift >> 3], 1u);
+	__syncthreads();
+	const int64_t tile = s_tile, base = tile * RS_TILE;
 	const int cnt = (int) min((int64_t) RS_TILE, n - base);
-	for (int i = t; i < RS_WARPS * 256; i += RS_THREADS) whist[i] = 0;
-	running[t] = 0;
-	gstart[t] = off[(int64_t) t * ntiles + blockIdx.x];
-	__syncthreads();
-	// tile digit counts -> tile-local exclusive offsets
+	uint64_t k[RS_IPT];
+	uint32_t d[RS_IPT], rank[RS_IPT];
+	const int first = w * (32 * RS_IPT) + lane;
+#pragma unroll
 	for (int r = 0; r < RS_IPT; r++) {
-		int idx = r * RS_THREADS + t;
-		if (idx < cnt) {
-			uint32_t d = (uint32_t) (kin[base + idx] >> shift) & 0xFF;
-			unsigned peers = __match_any_sync(__activemask(), d);
-			if (lane == __ffs(peers) - 1) atomicAdd(&running[d], (uint32_t) __popc(peers));
-		}
+		const int idx = first + 32 * r;
+		k[r] = idx < cnt ? kin[base + idx] : 0;
+		d[r] = idx < cnt ? (uint32_t) (k[r] >> shift) & 0xFF : 256u;
 	}
-	__syncthreads();
-	{
-		int32_t c = (int32_t) running[t], ex;
-		// 256 threads: reuse the generic block scan pattern
-		int32_t inc = c;
-#pragma unroll
-		for (int o = 1; o < 32; o <<= 1) {
-			int32_t u = __shfl_up_sync(0xFFFFFFFFu, inc, o);
-			if (lane >= o) inc += u;
-		}
-		if (lane == 31) s_warp[w] = inc;
-		__syncthreads();
-		if (w == 0) {
-			int32_t v = lane < RS_WARPS ? s_warp[lane] : 0;
-			int32_t vi = v;
-#pragma unroll
-			for (int o = 1; o < 32; o <<= 1) {
-				int32_t u = __shfl_up_sync(0xFFFFFFFFu, vi, o);
-				if (lane >= o) vi += u;
+	const uint32_t count = rank_tile(d, rank, whist);
+	state[tile * 256 + t] = (tile == 0 ? RS_TOTAL : RS_COUNT) | count;
+	dstart[t] = scan256(count, s_warp);
+	// look back: thread t sums digit t's counts of the earlier tiles
+	uint32_t before = 0;
+	for (int64_t q = tile - 1; q >= 0; q--) {
+		uint32_t v = state[q * 256 + t];
+		for (int spin = 0; v == 0; spin++) {
+			if (spin > RS_SPIN) {
+				atomicOr(status, TVG_ST_TIMEOUT);
+				v = RS_TOTAL;
+				break;
 			}
-			if (lane < RS_WARPS) s_warp[lane] = vi - v;
+			v = state[q * 256 + t];
 		}
-		__syncthreads();
-		ex = inc - c + s_warp[w];
-		dstart[t] = (uint32_t) ex;
-		running[t] = 0;
+		before += v & RS_VALUE;
+		if (v & RS_TOTAL) break;
 	}
+	if (tile > 0) state[tile * 256 + t] = RS_TOTAL | ((before + count) & RS_VALUE);
+	gstart[t] = offsets[t] + before - dstart[t];
 	__syncthreads();
-	const unsigned lt_mask = (1u << lane) - 1u;
+#pragma unroll
 	for (int r = 0; r < RS_IPT; r++) {
-		const int idx = r * RS_THREADS + t;
-		const bool valid = idx < cnt;
-		uint64_t k = 0;
-		uint32_t v = 0, d = 256 + lane;      // invalid lanes match nobody
-		if (valid) {
-			k = kin[base + idx];
-			v = vin[base + idx];
-			d = (uint32_t) (k >> shift) & 0xFF;
+		if (d[r] < 256) {
+			rank[r] += dstart[d[r]] + whist[w][d[r]];
+			skey[rank[r]] = k[r];
 		}
-		unsigned peers = __match_any_sync(0xFFFFFFFFu, d);
-		int rank_w = __popc(peers & lt_mask);
-		if (valid && rank_w == 0) whist[w * 256 + d] = (uint32_t) __popc(peers);
-		__syncthreads();
-		{   // per digit: exclusive prefix over warps, continuing the running count
-			uint32_t run = running[t];
+	}
+	__syncthreads();
+	uint32_t dest[RS_IPT];
 #pragma unroll
-			for (int ww = 0; ww < RS_WARPS; ww++) {
-				uint32_t c = whist[ww * 256 + t];
-				whist[ww * 256 + t] = run;
-				run += c;
+	for (int r = 0; r < RS_IPT; r++) {
+		const int p = t + RS_THREADS * r;
+		dest[r] = 0xFFFFFFFFu;
+		if (p < cnt) {
+			const uint64_t key = skey[p];
+			dest[r] = gstart[(uint32_t) (key >> shift) & 0xFF] + (uint32_t) p;
+			if (dest[r] < n) kout[dest[r]] = key;
+		}
+	}
+	__syncthreads();
+	uint32_t *sval = (uint32_t *) skey;
+#pragma unroll
+	for (int r = 0; r < RS_IPT; r++) {
+		const int idx = first + 32 * r;
+		if (idx < cnt) sval[rank[r]] = vin ? vin[base + idx] : (uint32_t) (base + idx);
+	}
+	__syncthreads();
+#pragma unroll
+	for (int r = 0; r < RS_IPT; r++) {
+		const int p = t + RS_THREADS * r;
+		if (dest[r] < n) vout[dest[r]] = sval[p];
+	}
+}
+
+// up to RS_TILE keys in one block: all eight digits in shared memory; key is
+// sorted in place, perm receives the input indices
+__global__ void __launch_bounds__(RS_THREADS)
+k_sort_tile(int n, uint64_t *__restrict__ key, uint32_t *__restrict__ perm)
+{
+	__shared__ __align__(16) uint64_t skey[RS_TILE];
+	__shared__ uint32_t whist[RS_WARPS][256];
+	__shared__ uint32_t dstart[256], s_warp[RS_WARPS];
+	uint32_t *sval = (uint32_t *) skey;
+	const int t = threadIdx.x, lane = t & 31, w = t >> 5, first = w * (32 * RS_IPT) + lane;
+	uint64_t k[RS_IPT];
+	uint32_t v[RS_IPT], d[RS_IPT], rank[RS_IPT];
+#pragma unroll
+	for (int r = 0; r < RS_IPT; r++) {
+		const int idx = first + 32 * r;
+		k[r] = idx < n ? key[idx] : 0;
+		v[r] = (uint32_t) idx;
+	}
+	for (int shift = 0; shift < 64; shift += 8) {
+#pragma unroll
+		for (int r = 0; r < RS_IPT; r++) d[r] = first + 32 * r < n ? (uint32_t) (k[r] >> shift) & 0xFF : 256u;
+		const uint32_t count = rank_tile(d, rank, whist);
+		if (__syncthreads_or(count == (uint32_t) n)) continue;
+		dstart[t] = scan256(count, s_warp);
+		__syncthreads();
+#pragma unroll
+		for (int r = 0; r < RS_IPT; r++)
+			if (d[r] < 256) {
+				rank[r] += dstart[d[r]] + whist[w][d[r]];
+				skey[rank[r]] = k[r];
 			}
-			running[t] = run;
-		}
 		__syncthreads();
-		if (valid) {
-			uint32_t pos = dstart[d] + whist[w * 256 + d] + (uint32_t) rank_w;
-			skey[pos] = k;
-			sval[pos] = v;
-		}
+#pragma unroll
+		for (int r = 0; r < RS_IPT; r++)
+			if (d[r] < 256) k[r] = skey[first + 32 * r];
 		__syncthreads();
-		for (int ww = 0; ww < RS_WARPS; ww++) whist[ww * 256 + t] = 0;
+#pragma unroll
+		for (int r = 0; r < RS_IPT; r++)
+			if (d[r] < 256) sval[rank[r]] = v[r];
+		__syncthreads();
+#pragma unroll
+		for (int r = 0; r < RS_IPT; r++)
+			if (d[r] < 256) v[r] = sval[first + 32 * r];
 		__syncthreads();
 	}
-	for (int p = t; p < cnt; p += RS_THREADS) {
-		uint64_t k = skey[p];
-		uint32_t d = (uint32_t) (k >> shift) & 0xFF;
-		int64_t dest = (int64_t) gstart[d] + (p - (int) dstart[d]);
-		kout[dest] = k;
-		vout[dest] = sval[p];
+#pragma unroll
+	for (int r = 0; r < RS_IPT; r++) {
+		const int idx = first + 32 * r;
+		if (idx < n) {
+			key[idx] = k[r];
+			perm[idx] = v[r];
+		}
 	}
 }
 
@@ -216,7 +298,8 @@ __global__ void k_tie_rank(int64_t n, const uint64_t *__restrict__ hi, const uin
 	const int64_t i = blockIdx.x * (int64_t) blockDim.x + threadIdx.x;
 	if (i >= n) return;
 	const uint64_t h = hi[i];
-	const uint32_t pv = perm[i];
+	// (a pass that gave up leaves places unwritten: keep every index inside)
+	const uint32_t last = (uint32_t) (n - 1), pv = min(perm[i], last);
 	if (!((i > 0 && hi[i - 1] == h) || (i + 1 < n && hi[i + 1] == h))) {
 		out[i] = pv;
 		return;
@@ -227,23 +310,17 @@ __global__ void k_tie_rank(int64_t n, const uint64_t *__restrict__ hi, const uin
 	const uint64_t kv = lo_orig[pv];
 	int64_t r = 0;
 	for (int64_t j = a; j < e; j++) {
-		const uint64_t kj = lo_orig[perm[j]];
+		const uint64_t kj = lo_orig[min(perm[j], last)];
 		r += (kj < kv || (kj == kv && j < i)) ? 1 : 0;
 	}
 	out[a + r] = pv;
 }
 
-__global__ void k_gather_u64(int64_t n, const uint32_t *__restrict__ perm, const uint64_t *__restrict__ in,
-                             uint64_t *__restrict__ out)
-{
-	int64_t i = blockIdx.x * (int64_t) blockDim.x + threadIdx.x;
-	if (i < n) out[i] = in[perm[i]];
-}
-
+// the particle fields and the low key words
 struct GatherList {
-	const void *in[FS_NFIELDS];
-	void *out[FS_NFIELDS];
-	int bytes[FS_NFIELDS];
+	const void *in[FS_NFIELDS + 1];
+	void *out[FS_NFIELDS + 1];
+	int bytes[FS_NFIELDS + 1];
 	int nf;
 };
 
@@ -294,61 +371,59 @@ __global__ void k_gather_fields(int64_t n, const uint32_t *__restrict__ perm, Ga
 	}
 }
 
-// k_radix_scatter's dynamic shared memory (above the 48 KB default) is a
-// function attribute of each device: set it once for every device the
-// process sorts on
-static cudaError_t radix_smem_attr(size_t smem)
+// The eight passes over n keys: kin / kout and the two value buffers alternate,
+// and after the eighth pass the result is back in kin and vb. count: 8 x 256
+// words; st[2]: tile states; tiles: 8 words.
+static cudaError_t radix_passes(cudaStream_t s, int64_t n, const uint64_t *key, uint64_t *kin, uint64_t *kout,
+                                uint32_t *va, uint32_t *vb, uint32_t *count, int32_t *skip,
+                                uint32_t *const st[2], uint32_t *tiles, int *status)
 {
-	static std::mutex mu;
-	static bool done[TVG_MAX_DEVICES] = { false };
-	int device = 0;
-	cudaError_t e = cudaGetDevice(&device);
+	const int64_t ntiles = (n + RS_TILE - 1) / RS_TILE;
+	cudaError_t e = cudaMemsetAsync(count, 0, 4 * 8 * 256, s);
+	if (e == cudaSuccess) e = cudaMemsetAsync(st[0], 0, 4 * 256 * (size_t) ntiles, s);
 	if (e != cudaSuccess) return e;
-	if (device < 0 || device >= TVG_MAX_DEVICES) return cudaErrorInvalidDevice;
-	std::lock_guard<std::mutex> lock(mu);
-	if (done[device]) return cudaSuccess;
-	e = cudaFuncSetAttribute(k_radix_scatter, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
-	if (e == cudaSuccess) done[device] = true;
-	return e;
+	const unsigned nb = (unsigned) (ntiles < 296 ? ntiles : 296);
+	k_digit_counts<<<nb, 512, 0, s>>>(n, key, count);
+	k_digit_offsets<<<8, 256, 0, s>>>(n, count, skip, tiles);
+	const uint32_t *vin = nullptr;
+	const uint64_t *in = key;
+	for (int d = 0; d < 8; d++) {
+		uint64_t *out = d & 1 ? kin : kout;
+		uint32_t *vout = d & 1 ? vb : va;
+		k_radix_pass<<<(unsigned) ntiles, RS_THREADS, 0, s>>>(n, 8 * d, in, vin, out, vout, count + 256 * d,
+		                                                      st[d & 1], st[(d & 1) ^ 1], tiles, skip, status);
+		in = out;
+		vin = vout;
+	}
+	return cudaGetLastError();
 }
+#define RS_LAUNCHES 10
 
 int tvg_impl_sort(tvg_context *ctx, uint32_t *perm_out)
 {
 	const int64_t n = ctx->n;
 	if (n == 0) return TVG_OK;
 	cudaStream_t s = ctx->stream;
-	const int64_t ntiles = (n + RS_TILE - 1) / RS_TILE;
-	k_iota<<<TVG_CNT(ctx, tvg_blocks(n, 256)), 256, 0, s>>>(n, ctx->perm);
-	TVG_CUDA(ctx, cudaMemsetAsync(ctx->digit_count, 0, 4 * 8 * 256, s));
-	k_digit_counts<<<TVG_CNT(ctx, 296), 512, 0, s>>>(n, ctx->key_hi, ctx->digit_count);
-	int32_t *skip = ctx->dc->sort_skip;
-	k_digit_skip<<<TVG_CNT(ctx, 1), 32, 0, s>>>(n, ctx->digit_count, skip);
-	TVG_CUDA(ctx, cudaGetLastError());
-	const size_t smem = RS_TILE * 12 + (RS_WARPS * 256 + 3 * 256 + 33) * 4;
-	TVG_CUDA(ctx, radix_smem_attr(smem));
-	uint64_t *kin = ctx->key_hi, *kout = ctx->key_tmp;
+	uint64_t *kin = ctx->key_hi;
 	uint32_t *vin = ctx->perm, *vout = ctx->perm_tmp;
-	for (int d = 0; d < 8; d++) {
-		const int shift = 8 * d;
-		k_tile_hist<<<TVG_CNT(ctx, (unsigned) ntiles), RS_THREADS, 0, s>>>(n, shift, kin, ctx->sort_hist, ntiles,
-		                                                                   skip);
+	if (n <= RS_TILE) {
+		k_sort_tile<<<TVG_CNT(ctx, 1), RS_THREADS, 0, s>>>((int) n, kin, vin);
 		TVG_CUDA(ctx, cudaGetLastError());
-		TVG_CHECK(tvg_device_scan_i32(ctx, (const int32_t *) ctx->sort_hist, (int32_t *) ctx->sort_off,
-		                              256 * ntiles, nullptr));
-		k_radix_scatter<<<TVG_CNT(ctx, (unsigned) ntiles), RS_THREADS, smem, s>>>(n, shift, kin, vin, kout, vout,
-		                                                            ctx->sort_off, ntiles, skip);
-		TVG_CUDA(ctx, cudaGetLastError());
-		uint64_t *kt = kin; kin = kout; kout = kt;
-		uint32_t *vt = vin; vin = vout; vout = vt;
+	} else {
+		uint32_t *const st[2] = { ctx->sort_hist, ctx->sort_off };
+		ctx->launches += RS_LAUNCHES;
+		TVG_CUDA(ctx, radix_passes(s, n, kin, kin, ctx->key_tmp, vout, vin, ctx->digit_count, ctx->dc->sort_skip,
+		                           st, ctx->dc->sort_tiles, ctx->status));
 	}
-	ctx->key_hi = kin; ctx->key_tmp = kout;
 	// runs of equal high words by the low words, into the other buffer
 	k_tie_rank<<<TVG_CNT(ctx, tvg_blocks(n, 256)), 256, 0, s>>>(n, kin, ctx->key_lo, vin, vout);
 	ctx->perm = vout; ctx->perm_tmp = vin;
-	k_gather_u64<<<TVG_CNT(ctx, tvg_blocks(n, 256)), 256, 0, s>>>(n, ctx->perm, ctx->key_lo, ctx->key_tmp);
-	{ uint64_t *t = ctx->key_lo; ctx->key_lo = ctx->key_tmp; ctx->key_tmp = t; }
 	GatherList g;
-	g.nf = 0;
+	g.in[0] = ctx->key_lo;
+	g.out[0] = ctx->key_tmp;
+	g.bytes[0] = 8;
+	g.nf = 1;
+	{ uint64_t *t = ctx->key_lo; ctx->key_lo = ctx->key_tmp; ctx->key_tmp = t; }
 	for (int f = 0; f < FS_NFIELDS; f++) {
 		g.in[g.nf] = ctx->f[f];
 		g.out[g.nf] = ctx->falt[f];
@@ -378,8 +453,7 @@ int tvg_impl_sort(tvg_context *ctx, uint32_t *perm_out)
 //
 // The array belongs to every GPU that loads this library, for the life of the
 // process (about 6.4 MB). All calls on a device share it and it keeps the
-// last call's contents: each pass rewrites every histogram entry it reads, so
-// nothing has to start at zero. Two calls that overlap on the same GPU (from
+// last call's contents: a call zeroes the counts and states it starts from. Two calls that overlap on the same GPU (from
 // two host threads, or on two streams) corrupt each other's scratch.
 // ------------------------------------------------------------------------
 
@@ -388,50 +462,14 @@ int tvg_impl_sort(tvg_context *ctx, uint32_t *perm_out)
 struct NoallocScratch {
 	uint64_t key[2][TVG_NOALLOC_MAX_KEYS];   // sorted high words, ping-pong
 	uint32_t idx[2][TVG_NOALLOC_MAX_KEYS];   // permutation, ping-pong
-	uint32_t hist[256 * NOALLOC_TILES];      // per-tile digit counts (digit-major)
-	uint32_t off[256 * NOALLOC_TILES];       // their exclusive prefix sum
+	uint32_t state[2][256 * NOALLOC_TILES];  // the passes' tile states
+	uint32_t count[8 * 256];                 // digit counts, then offsets
+	int32_t skip[8];
+	uint32_t tiles[8];
+	int status;
 };
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[sizeof(NoallocScratch)];
-
-// single-block exclusive prefix sum of up to 1024 * 16 counts
-__global__ void __launch_bounds__(1024) k_scan_small(const uint32_t *__restrict__ in, uint32_t *__restrict__ out, int n)
-{
-	__shared__ uint32_t s_warp[32];
-	const int t = threadIdx.x, lane = t & 31, w = t >> 5;
-	uint32_t v[16], sum = 0;
-#pragma unroll
-	for (int k = 0; k < 16; k++) {
-		const int i = t * 16 + k;
-		v[k] = i < n ? in[i] : 0u;
-		sum += v[k];
-	}
-	uint32_t inc = sum;
-#pragma unroll
-	for (int o = 1; o < 32; o <<= 1) {
-		uint32_t u = __shfl_up_sync(0xFFFFFFFFu, inc, o);
-		if (lane >= o) inc += u;
-	}
-	if (lane == 31) s_warp[w] = inc;
-	__syncthreads();
-	if (w == 0) {
-		uint32_t x = s_warp[lane], xi = x;
-#pragma unroll
-		for (int o = 1; o < 32; o <<= 1) {
-			uint32_t u = __shfl_up_sync(0xFFFFFFFFu, xi, o);
-			if (lane >= o) xi += u;
-		}
-		s_warp[lane] = xi - x;
-	}
-	__syncthreads();
-	uint32_t run = inc - sum + s_warp[w];
-#pragma unroll
-	for (int k = 0; k < 16; k++) {
-		const int i = t * 16 + k;
-		if (i < n) out[i] = run;
-		run += v[k];
-	}
-}
 
 // Device address of the scratch array, looked up once per device with that
 // device current (the host-side symbol is not a device address).
@@ -462,25 +500,20 @@ extern "C" int tvg_sort_keys_noalloc(const uint64_t *key_hi, const uint64_t *key
 	if (cudaGetDevice(&device) != cudaSuccess) { cudaGetLastError(); return TVG_E_CUDA; }
 	NoallocScratch *S = noalloc_scratch(device);
 	if (!S) return TVG_E_CUDA;
-	const size_t smem = RS_TILE * 12 + (RS_WARPS * 256 + 3 * 256 + 33) * 4;
-	if (radix_smem_attr(smem) != cudaSuccess) { cudaGetLastError(); return TVG_E_CUDA; }
-	const int64_t ntiles = (n + RS_TILE - 1) / RS_TILE;
 	cudaStream_t s = 0;
-	k_iota<<<tvg_blocks(n, 256), 256, 0, s>>>(n, S->idx[0]);
-	const uint64_t *kin = key_hi;
-	int cur = 0;
-	for (int d = 0; d < 8; d++) {
-		const int shift = 8 * d;
-		uint64_t *kout = S->key[d & 1];
-		k_tile_hist<<<(unsigned) ntiles, RS_THREADS, 0, s>>>(n, shift, kin, S->hist, ntiles);
-		k_scan_small<<<1, 1024, 0, s>>>(S->hist, S->off, (int) (256 * ntiles));
-		k_radix_scatter<<<(unsigned) ntiles, RS_THREADS, smem, s>>>(n, shift, kin, S->idx[cur], kout,
-		                                                            S->idx[cur ^ 1], S->off, ntiles);
-		kin = kout;
-		cur ^= 1;
+	cudaError_t e = cudaMemsetAsync(&S->status, 0, sizeof(int), s);
+	if (e == cudaSuccess) {
+		uint32_t *const st[2] = { S->state[0], S->state[1] };
+		e = radix_passes(s, n, key_hi, S->key[0], S->key[1], S->idx[0], S->idx[1], S->count, S->skip, st, S->tiles,
+		                 &S->status);
 	}
-	k_tie_rank<<<tvg_blocks(n, 256), 256, 0, s>>>(n, kin, key_lo, S->idx[cur], perm);
-	cudaError_t e = cudaGetLastError();
+	if (e == cudaSuccess) {
+		k_tie_rank<<<tvg_blocks(n, 256), 256, 0, s>>>(n, S->key[0], key_lo, S->idx[1], perm);
+		e = cudaGetLastError();
+	}
+	int status = 0;
+	if (e == cudaSuccess) e = cudaMemcpyAsync(&status, &S->status, sizeof(int), cudaMemcpyDeviceToHost, s);
 	if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+	if (e == cudaSuccess && status) return TVG_E_TIMEOUT;
 	return e == cudaSuccess ? TVG_OK : TVG_E_CUDA;
 }
