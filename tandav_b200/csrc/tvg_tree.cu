@@ -31,7 +31,12 @@
 // exact mode, every node are summed sequentially in particle order in Float
 // (tree_build.c:561-572), which reproduces the reference bit for bit; the fast
 // mode sums internal nodes in FP64 with one warp per node.
-// Roofline: HBM/L2 bound (1 B level + 16 B key per particle, ~O(nodes)).
+// Roofline: HBM/L2 bound (1 B level + 16 B key per particle, ~O(nodes)). The
+// searches for a node's end take eight levels or block minima per load and go on
+// from the child's end (k_nodes: 263 -> 44 us for a halo of 400,000, 888 -> 559 us for
+// 256^3), a warp writes its bundles' Tree_Parent together (k_emit_nodes: 1120 -> 605
+// us for 256^3), and the top nodes are made and placed by a block each (60 and
+// 90 -> 6 and 5 us).
 #include "tvg_internal.cuh"
 
 #define TOP_LEVEL 2         // MIN_LEVEL (domain.c:3): the top level on one target
@@ -59,38 +64,48 @@ __global__ void k_top_first(int64_t n, const uint64_t *__restrict__ key_hi, int3
 	if (i == 0 || (int) (key_hi[i - 1] >> 58) != c) first[c] = (int32_t) i;
 }
 
-// one thread: top nodes in descending key order (compare_bunches_by_key,
-// domain.c:678-684), centre from the first particle (domain.c:237-246)
+// a thread per level-2 cell: top nodes in descending key order
+// (compare_bunches_by_key, domain.c:678-684), centre from the first particle
+// (domain.c:237-246)
 template <typename F>
-__global__ void k_make_top(int64_t n, const int32_t *first, const F *x, const F *y, const F *z,
-                           double ox, double oy, double oz, double size, tvg_topnode *top,
-                           int32_t *count, tvg_devcount *dc)
+__global__ void __launch_bounds__(64)
+k_make_top(int64_t n, const int32_t *__restrict__ first, const F *x, const F *y, const F *z,
+           double ox, double oy, double oz, double size, tvg_topnode *top,
+           int32_t *count, tvg_devcount *dc)
 {
-	if (threadIdx.x || blockIdx.x) return;
-	int nt = 0;
-	for (int c = 63; c >= 0; c--) {
-		if (first[c] < 0) { count[c] = 0; continue; }
-		int64_t e = n;
-		for (int d = c + 1; d < 64; d++)
-			if (first[d] >= 0) { e = first[d]; break; }
-		count[c] = (int32_t) (e - first[c]);
-		tvg_topnode t;
-		t.key = ((uint64_t) c << 58) | (0xFFFFFFFFFFFFFFFFULL >> 6);
-		t.target = -1;
-		t.level = TOP_LEVEL;
-		t.first_part = first[c];
-		t.npart = (int32_t) (e - first[c]);
-		int64_t ip = first[c];
-		const double sz = size / (double) (1ULL << TOP_LEVEL);
-		const double px = (double) x[ip] - ox, py = (double) y[ip] - oy, pz = (double) z[ip] - oz;
-		t.pos[0] = (float) __dadd_rn(__dmul_rn(floor(px / sz) + 0.5, sz), ox);
-		t.pos[1] = (float) __dadd_rn(__dmul_rn(floor(py / sz) + 0.5, sz), oy);
-		t.pos[2] = (float) __dadd_rn(__dmul_rn(floor(pz / sz) + 0.5, sz), oz);
-		t.mass = 0;
-		for (int k = 0; k < 3; k++) { t.com[k] = 0; t.dp[k] = 0; }
-		top[nt++] = t;
+	__shared__ int32_t s_first[64];
+	const int c = threadIdx.x;
+	const int32_t f = first[c];
+	s_first[c] = f;
+	__syncthreads();
+	int64_t e = n;
+	int above = 0, all = 0;             // non-empty cells of larger keys, and all
+	for (int d = 63; d >= 0; d--) {
+		const int32_t fd = s_first[d];
+		if (fd < 0) continue;
+		all++;
+		if (d > c) {
+			above++;
+			e = fd;
+		}
 	}
-	dc->ntop = nt;
+	if (c == 0) dc->ntop = all;
+	count[c] = f < 0 ? 0 : (int32_t) (e - f);
+	if (f < 0) return;
+	tvg_topnode t;
+	t.key = ((uint64_t) c << 58) | (0xFFFFFFFFFFFFFFFFULL >> 6);
+	t.target = -1;
+	t.level = TOP_LEVEL;
+	t.first_part = f;
+	t.npart = (int32_t) (e - f);
+	const double sz = size / (double) (1ULL << TOP_LEVEL);
+	const double px = (double) x[f] - ox, py = (double) y[f] - oy, pz = (double) z[f] - oz;
+	t.pos[0] = (float) __dadd_rn(__dmul_rn(floor(px / sz) + 0.5, sz), ox);
+	t.pos[1] = (float) __dadd_rn(__dmul_rn(floor(py / sz) + 0.5, sz), oy);
+	t.pos[2] = (float) __dadd_rn(__dmul_rn(floor(pz / sz) + 0.5, sz), oz);
+	t.mass = 0;
+	for (int k = 0; k < 3; k++) { t.com[k] = 0; t.dp[k] = 0; }
+	top[above] = t;
 }
 
 // top node of every particle: block b takes top nodes b, b + grid, ...
@@ -123,12 +138,12 @@ int tvg_impl_top_nodes(tvg_context *ctx)
 	TVG_CUDA(ctx, cudaMemsetAsync(ctx->top_first, 0xFF, 4 * 64, s));
 	k_top_first<<<TVG_CNT(ctx, tvg_blocks(n, 256)), 256, 0, s>>>(n, ctx->key_hi, ctx->top_first);
 	if (ctx->cfg.float_bytes == 4)
-		k_make_top<float><<<TVG_CNT(ctx, 1), 1, 0, s>>>(n, ctx->top_first, (const float *) ctx->f[FS_POS0],
+		k_make_top<float><<<TVG_CNT(ctx, 1), 64, 0, s>>>(n, ctx->top_first, (const float *) ctx->f[FS_POS0],
 		                                  (const float *) ctx->f[FS_POS1], (const float *) ctx->f[FS_POS2],
 		                                  ctx->origin[0], ctx->origin[1], ctx->origin[2], ctx->dsize,
 		                                  ctx->d_top, ctx->top_count, ctx->dc);
 	else
-		k_make_top<double><<<TVG_CNT(ctx, 1), 1, 0, s>>>(n, ctx->top_first, (const double *) ctx->f[FS_POS0],
+		k_make_top<double><<<TVG_CNT(ctx, 1), 64, 0, s>>>(n, ctx->top_first, (const double *) ctx->f[FS_POS0],
 		                                   (const double *) ctx->f[FS_POS1], (const double *) ctx->f[FS_POS2],
 		                                   ctx->origin[0], ctx->origin[1], ctx->origin[2], ctx->dsize,
 		                                   ctx->d_top, ctx->top_count, ctx->dc);
@@ -193,41 +208,77 @@ __global__ void k_levels(int64_t n, const uint64_t *__restrict__ hi, const uint6
 	if (i == n - 1) ncnt[n] = 0;
 }
 
-// first j > s with lvl[j] < l, or n
-__device__ int64_t next_smaller(const uint8_t *__restrict__ lvl, const uint8_t *__restrict__ m64,
-                                int64_t n, int64_t s, int l)
+// mask of the bytes of an 8-byte word below l: the byte's top bit set
+__device__ __forceinline__ uint64_t bytes_below(uint64_t w, uint32_t l4)
 {
-	int64_t j = s + 1;
-	while (j < n && (j & 63)) {
-		if (lvl[j] < l) return j;
-		j++;
-	}
-	if (j >= n) return n;
-	int64_t b = j >> 6;
-	const int64_t nb = (n + 63) >> 6;
-	while (b < nb && m64[b] >= l) b++;
-	if (b >= nb) return n;
-	j = b << 6;
-	while (j < n && lvl[j] >= l) j++;
-	return j;
+	const uint32_t lo = __vcmpltu4((uint32_t) w, l4), hi = __vcmpltu4((uint32_t) (w >> 32), l4);
+	return ((uint64_t) hi << 32 | lo) & 0x8080808080808080ull;
 }
 
-// last j < s with lvl[j] < l (exists: a top node's first particle has lvl 1)
+// first index >= j of a byte below l in a[0 .. n), or n; eight bytes at a time
+// (the arrays are allocated 64 bytes past their length; what lies there is
+// ignored). stop: the search may end at the first multiple of `stop` (a power of
+// two >= 8) after j without a find, which it returns.
+__device__ __forceinline__ int64_t find_below(const uint8_t *__restrict__ a, int64_t n, int64_t j, int l, int64_t stop)
+{
+	const uint32_t l4 = (uint32_t) l * 0x01010101u;
+	while (j < n) {
+		const int64_t w = j & ~(int64_t) 7;
+		uint64_t m = bytes_below(*(const uint64_t *) (a + w), l4);
+		m &= ~0ull << (8 * (j - w));
+		if (m) return min(n, w + ((__ffsll((long long) m) - 1) >> 3));
+		j = w + 8;
+		if ((j & (stop - 1)) == 0) return min(j, n);
+	}
+	return n;
+}
+
+// last index <= j of a byte below l in a, or a value below the last multiple of
+// `stop` at or below j
+__device__ __forceinline__ int64_t find_below_back(const uint8_t *__restrict__ a, int64_t j, int l, int64_t stop)
+{
+	const uint32_t l4 = (uint32_t) l * 0x01010101u;
+	while (j >= 0) {
+		const int64_t w = j & ~(int64_t) 7;
+		uint64_t m = bytes_below(*(const uint64_t *) (a + w), l4);
+		m &= ~0ull >> (8 * (7 - (j - w)));
+		if (m) return w + ((63 - __clzll((long long) m)) >> 3);
+		j = w - 1;
+		if ((w & (stop - 1)) == 0) return j;
+	}
+	return -1;
+}
+
+#define FIND_ALL ((int64_t) 1 << 62)
+
+// first index >= j with lvl < l, or n: within j's 64-block, then the blocks'
+// minima, then within the block found
+__device__ int64_t next_smaller(const uint8_t *__restrict__ lvl, const uint8_t *__restrict__ m64,
+                                int64_t n, int64_t j, int l)
+{
+	if (j >= n) return n;
+	if (j & 63) {
+		j = find_below(lvl, n, j, l, 64);
+		if (j >= n || lvl[j] < l) return j;
+	}
+	const int64_t nb = (n + 63) >> 6, b = find_below(m64, nb, j >> 6, l, FIND_ALL);
+	if (b >= nb) return n;
+	return find_below(lvl, n, b << 6, l, 64);
+}
+
+// last j < s with lvl[j] < l (exists: a top node's first particle has lvl 0)
 __device__ int64_t prev_smaller(const uint8_t *__restrict__ lvl, const uint8_t *__restrict__ m64,
                                 int64_t s, int l)
 {
 	int64_t j = s - 1;
-	while (j >= 0 && ((j + 1) & 63)) {
-		if (lvl[j] < l) return j;
-		j--;
-	}
 	if (j < 0) return -1;
-	int64_t b = j >> 6;
-	while (b >= 0 && m64[b] >= l) b--;
+	if ((j & 63) != 63) {
+		j = find_below_back(lvl, j, l, 64);
+		if (j < 0 || (j & 63) != 63 || lvl[j] < l) return j;
+	}
+	const int64_t b = find_below_back(m64, j >> 6, l, FIND_ALL);
 	if (b < 0) return -1;
-	j = (b << 6) + 63;
-	while (lvl[j] >= l) j--;
-	return j;
+	return find_below_back(lvl, (b << 6) + 63, l, 64);
 }
 
 enum { UF_COLLAPSED = 1, UF_LEAF = 2, UF_ROOT = 4 };
@@ -256,10 +307,13 @@ __global__ void k_nodes(int64_t n, const uint8_t *__restrict__ lvl, const uint8_
 	if (nc == 0) return;
 	const bool top_start = lvl[s] == LVL_START;
 	const int lo_l = first_level(lvl, top, top_of, s);
-	for (int k = 0; k < nc; k++) {
+	// deepest node first: a node's end lies at or past its child's, so the
+	// search goes on from there
+	int64_t e = s + 1;
+	for (int k = nc - 1; k >= 0; k--) {
 		const int l = lo_l + k;
 		const int64_t u = b0 + k;
-		const int64_t e = next_smaller(lvl, m64, n, s, l);
+		e = next_smaller(lvl, m64, n, e, l);
 		const int32_t cnt = (int32_t) (e - s);
 		uint8_t flag = 0;
 		if (top_start && k == 0) flag |= UF_ROOT;
@@ -274,10 +328,7 @@ __global__ void k_nodes(int64_t n, const uint8_t *__restrict__ lvl, const uint8_
 					// cell A (level l_e+1 holding e-1) must hold > vsize particles
 					int64_t a0 = e - vsize;
 					if (a0 < 0) a0 = 0;
-					bool a_small = false;
-					for (int64_t j = a0; j < e; j++)
-						if (lvl[j] <= le) { a_small = true; break; }
-					if (!a_small) flag |= UF_COLLAPSED;
+					if (find_below(lvl, e, a0, le + 1, FIND_ALL) >= e) flag |= UF_COLLAPSED;
 				}
 			}
 		}
@@ -309,31 +360,58 @@ __global__ void k_survivors(const tvg_devcount *__restrict__ dc, int64_t ucap,
 	surv[u] = (u < nu && excl[u + 1] == 0) ? 1 : 0;
 }
 
-// one thread: subtree placement in top-node order (tree_build.c:59-96); the
-// placement table for the emission and the node count, on the device
-__global__ void k_place_subtrees(tvg_devcount *dc, tvg_topnode *top, const int32_t *__restrict__ base,
-                                 const int32_t *__restrict__ F, int vsize, TopTables tp, int64_t ucap,
-                                 int64_t tcap, int *status)
+// One block: subtree placement in top-node order (tree_build.c:59-96), a
+// prefix sum of the subtrees' sizes; the placement table for the emission and
+// the node count, on the device
+#define PLACE_THREADS 256
+__global__ void __launch_bounds__(PLACE_THREADS)
+k_place_subtrees(tvg_devcount *dc, tvg_topnode *top, const int32_t *__restrict__ base,
+                 const int32_t *__restrict__ F, int vsize, TopTables tp, int64_t ucap,
+                 int64_t tcap, int *status)
 {
-	if (threadIdx.x || blockIdx.x) return;
-	const int ntop = dc->ntop;
+	__shared__ int64_t s_warp[PLACE_THREADS / 32];
+	const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, ntop = dc->ntop;
 	int64_t run = 0;
-	for (int t = 0; t < ntop; t++) {
-		top[t].target = (int32_t) run;       // also for small top nodes (quirk Q3)
-		tp.target[t] = (int32_t) run;
-		tp.end[t] = top[t].first_part + top[t].npart;
-		tp.nsurv[t] = tp.toff[t] = 0;
-		if (top[t].npart > vsize) {
-			int64_t f = top[t].first_part, e = f + top[t].npart;
-			// base <= nu; past the capacity the build has failed (status set)
-			int32_t fs = F[min((int64_t) base[f], ucap)], fe = F[min((int64_t) base[e], ucap)];
-			tp.nsurv[t] = fe - fs;
-			tp.toff[t] = (int32_t) (run - fs);
-			run += (fe - fs) + 1;             // + terminator
+	for (int t0 = 0; t0 < ntop; t0 += PLACE_THREADS) {
+		const int t = t0 + threadIdx.x;
+		int64_t size = 0;
+		int32_t fs = 0, nsurv = 0;
+		if (t < ntop) {
+			const int64_t f = top[t].first_part, e = f + top[t].npart;
+			tp.end[t] = (int32_t) e;
+			if (top[t].npart > vsize) {
+				// base <= nu; past the capacity the build has failed (status set)
+				fs = F[min((int64_t) base[f], ucap)];
+				nsurv = F[min((int64_t) base[e], ucap)] - fs;
+				size = (int64_t) nsurv + 1;       // + terminator
+			}
 		}
+		int64_t inc = size;
+#pragma unroll
+		for (int o = 1; o < 32; o <<= 1) {
+			const int64_t u = __shfl_up_sync(0xFFFFFFFFu, inc, o);
+			if (lane >= o) inc += u;
+		}
+		if (lane == 31) s_warp[w] = inc;
+		__syncthreads();
+		int64_t before = run;
+		for (int k = 0; k < PLACE_THREADS / 32; k++) {
+			if (k < w) before += s_warp[k];
+			run += s_warp[k];
+		}
+		if (t < ntop) {
+			const int64_t at = before + inc - size;
+			top[t].target = (int32_t) at;         // also for small top nodes (quirk Q3)
+			tp.target[t] = (int32_t) at;
+			tp.nsurv[t] = nsurv;
+			tp.toff[t] = size ? (int32_t) (at - fs) : 0;
+		}
+		__syncthreads();
 	}
-	if (run > tcap) atomicOr(status, TVG_ST_TREE_FULL);
-	dc->nnodes = run;
+	if (threadIdx.x == 0) {
+		if (run > tcap) atomicOr(status, TVG_ST_TREE_FULL);
+		dc->nnodes = run;
+	}
 }
 
 
@@ -357,14 +435,27 @@ __global__ void k_emit_nodes(const tvg_devcount *__restrict__ dc, int64_t ucap, 
 {
 	const int64_t nu = min(dc->nu, ucap);
 	const int64_t u = blockIdx.x * (int64_t) blockDim.x + threadIdx.x;
-	if (u >= nu || !surv[u]) return;
-	const int32_t s = u_start[u];
-	const int l = u_level[u];
-	const int32_t cnt = u_count[u];
-	const uint8_t flag = u_flag[u];
-	const int t = top_of[s];
-	const int64_t G = (int64_t) tp.toff[t] + Fidx[u];
-	if (G < 0 || G >= tcap) { atomicOr(status, TVG_ST_TREE_FULL); return; }
+	if (u - (threadIdx.x & 31) >= nu) return;      // whole warps
+	bool live = u < nu && surv[u];
+	const int32_t s = live ? u_start[u] : 0;
+	const int l = live ? u_level[u] : 0;
+	const int32_t cnt = live ? u_count[u] : 0;
+	const uint8_t flag = live ? u_flag[u] : 0;
+	const int t = live ? top_of[s] : 0;
+	const int64_t G = live ? (int64_t) tp.toff[t] + Fidx[u] : 0;
+	if (live && (G < 0 || G >= tcap)) {
+		atomicOr(status, TVG_ST_TREE_FULL);
+		live = false;
+	}
+	// Tree_Parent of the bundles' particles, one bundle of the warp's at a time
+	// with all lanes (a thread for its own 64 wrote as many separate sectors)
+	for (unsigned todo = __ballot_sync(0xFFFFFFFFu, live && (flag & (UF_COLLAPSED | UF_LEAF))); todo; todo &= todo - 1) {
+		const int src = __ffs(todo) - 1;
+		const int32_t bs = __shfl_sync(0xFFFFFFFFu, s, src), bc = __shfl_sync(0xFFFFFFFFu, cnt, src);
+		const int32_t bg = __shfl_sync(0xFFFFFFFFu, (int32_t) G, src);
+		for (int32_t j = threadIdx.x & 31; j < bc; j += 32) tree_parent[bs + j] = bg;
+	}
+	if (!live) return;
 	TNode<F> nd;
 	nd.Npart = cnt;
 	nd.Bitfield = (uint32_t) l | ((uint32_t) triplet_at(hi, lo, s, l) << 6) | (1u << 9)
@@ -394,8 +485,6 @@ __global__ void k_emit_nodes(const tvg_devcount *__restrict__ dc, int64_t ucap, 
 	nd.Mass = 0;
 	tree[G] = nd;
 	tree_u[G] = (int32_t) u;
-	if (flag & (UF_COLLAPSED | UF_LEAF))
-		for (int32_t j = s; j < s + cnt; j++) tree_parent[j] = (int32_t) G;
 }
 
 // particles of top nodes without subtree point to their top node (-t-1),
@@ -675,7 +764,7 @@ __global__ void k_list_big_nodes(const tvg_devcount *__restrict__ dc, int64_t tc
 }
 
 // the listed nodes, a block each, with the FP64 sums of moments_warp_one
-#define MOM_BLOCK_THREADS 256
+#define MOM_BLOCK_THREADS 512
 template <typename F>
 __global__ void __launch_bounds__(MOM_BLOCK_THREADS) k_moments_block(TNode<F> *tree,
                                                                      const int32_t *__restrict__ tree_u,
@@ -795,7 +884,7 @@ static int build_typed(tvg_context *ctx, uint32_t flags)
 	TVG_CUDA(ctx, cudaGetLastError());
 	TVG_CHECK(tvg_device_scan_i32(ctx, ctx->u_diff, ctx->u_final, ucap + 1, nullptr));
 	// placement of the subtrees
-	k_place_subtrees<<<TVG_CNT(ctx, 1), 1, 0, s>>>(dc, ctx->d_top, ctx->ncnt, ctx->u_final, vsize, tp,
+	k_place_subtrees<<<TVG_CNT(ctx, 1), PLACE_THREADS, 0, s>>>(dc, ctx->d_top, ctx->ncnt, ctx->u_final, vsize, tp,
 	                                               ucap, tcap, ctx->status);
 	TVG_CUDA(ctx, cudaGetLastError());
 	TNode<F> *tree = (TNode<F> *) ctx->tree;

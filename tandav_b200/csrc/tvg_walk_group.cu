@@ -362,7 +362,7 @@ __global__ void k_wt_list_big(const tvg_devcount *__restrict__ dc, const int2 *_
 }
 
 // the listed walk nodes, a block each
-#define GW_QUAD_BLOCK_THREADS 256
+#define GW_QUAD_BLOCK_THREADS 512
 __global__ void __launch_bounds__(GW_QUAD_BLOCK_THREADS)
 k_wt_quad_block(const tvg_wnode *__restrict__ wt, const int2 *__restrict__ wrange,
                 const uint32_t *__restrict__ ix, const uint32_t *__restrict__ iy, const uint32_t *__restrict__ iz,
