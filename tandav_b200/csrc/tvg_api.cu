@@ -183,7 +183,8 @@ extern "C" void tvg_finalize(tvg_context *ctx)
 	                 ctx->act_off, ctx->mlp_prm, ctx->mlp_bf16, ctx->ewald_taylor, ctx->dc,
 	                 ctx->d_toptab, ctx->top_of, ctx->dd_scratch, ctx->tu_first, ctx->tu_dp,
 	                 ctx->tu_big, ctx->big_list, ctx->tune_active, ctx->wquad, ctx->wrange,
-	                 ctx->ewald_xyz, ctx->ft_ws, ctx->mlp_ws };
+	                 ctx->ewald_xyz, ctx->ft_ws, ctx->mlp_ws,
+	                 ctx->domain_state };
 	for (void *b : bufs) if (b) cudaFree(b);
 	if (ctx->h_status) cudaFreeHost(ctx->h_status);
 	for (int i = 0; i < 16; i++) if (ctx->ev[i]) cudaEventDestroy(ctx->ev[i]);

@@ -159,6 +159,7 @@ struct tvg_context {
 	int32_t dd_ntask = 1;
 	double dd_part_alloc_factor = 1.1; // Param.Part_Alloc_Factor
 	double dd_imbal_ceil = 0.05;       // DOMAIN_IMBAL_CEIL
+	void *domain_state = nullptr;      // tvg_find_domain's selection state
 	void *dd_scratch = nullptr;        // fill jobs, bunch keys and partial sums
 	int32_t dd_rounds = 0;             // refinement rounds of the last decomposition
 
