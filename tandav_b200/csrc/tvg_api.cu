@@ -178,7 +178,7 @@ extern "C" void tvg_finalize(tvg_context *ctx)
 	                 ctx->ipos[0], ctx->ipos[1], ctx->ipos[2], ctx->wtree, ctx->group_first,
 	                 ctx->work_counter, ctx->counters, ctx->ewald_f[0], ctx->ewald_f[1],
 	                 ctx->ewald_f[2], ctx->ewald_f[3], ctx->ewald_raw, ctx->ewald32,
-	                 ctx->ewald_wide, ctx->wide_list, ctx->wide_part, ctx->active, ctx->kd_x, ctx->kd_kick, ctx->kd_drift,
+	                 ctx->ewald_wide, ctx->wide_list, ctx->part_sums, ctx->active, ctx->kd_x, ctx->kd_kick, ctx->kd_drift,
 	                 ctx->kd_m2k, ctx->kd_m2d, ctx->kd_work, ctx->tl_scratch, ctx->act_flag,
 	                 ctx->act_off, ctx->mlp_prm, ctx->mlp_bf16, ctx->ewald_taylor, ctx->dc,
 	                 ctx->d_toptab, ctx->top_of, ctx->dd_scratch, ctx->tu_first, ctx->tu_dp,

@@ -186,10 +186,8 @@ struct tvg_context {
 	double *ewald_raw = nullptr;
 	float *ewald32 = nullptr;          // FP32 copy for the group form (FP64 builds)
 	float *ewald_wide = nullptr;       // T and 3 derivatives at TVG_WIDE_NODES^3 nodes, 24 floats each
-	// groups that take per-target images (k_ewald_wide): their list, then partial
-	// sums of WIDE_ITEMS items
-	int32_t *wide_list = nullptr;
-	double *wide_part = nullptr;
+	int32_t *wide_list = nullptr;      // groups that take per-target images (k_ewald_wide)
+	void *part_sums = nullptr;         // sums of the parts of split groups (both group walks)
 	float *ewald_taylor = nullptr;     // T and 3 derivatives at TVG_TAYLOR_NODES^3 nodes, 32 floats each
 	// Ewald-walk opening of the group form: the monopole error of the
 	// correction may reach ewald_open_rel |a_old| (relative mode); the limit of

@@ -612,19 +612,30 @@ __device__ __forceinline__ int pop_nodes(const int32_t *stack, int &sp, int *sta
 	return node;
 }
 
-// pushes the children of the lanes' opened internal nodes
+// pushes the children of the lanes' opened internal nodes; with parts > 1 only
+// those that fall to this part (index modulo parts)
 __device__ __forceinline__ void push_children(int32_t *stack, int &sp, bool open_int, int nchild,
-                                              int child)
+                                              int child, int part = 0, int parts = 1)
 {
 	const int lane = threadIdx.x & 31;
-	int c = open_int ? nchild : 0, incl = c;
+	int c = 0, at = child;
+	if (open_int) {
+		c = nchild;
+		if (parts > 1) {
+			// the first child of this part, and how many there are
+			const int skip = (part - child % parts + parts) % parts;
+			at = child + skip;
+			c = skip < nchild ? (nchild - skip + parts - 1) / parts : 0;
+		}
+	}
+	int incl = c;
 #pragma unroll
 	for (int o = 1; o < 32; o <<= 1) {
 		int u = __shfl_up_sync(0xFFFFFFFFu, incl, o);
 		if (lane >= o) incl += u;
 	}
 	const int tot = __shfl_sync(0xFFFFFFFFu, incl, 31);
-	for (int q = 0; q < c; q++) stack[sp + incl - c + q] = child + c - 1 - q;
+	for (int q = 0; q < c; q++) stack[sp + incl - c + q] = at + (c - 1 - q) * parts;
 	sp += tot;
 }
 
@@ -826,14 +837,17 @@ __device__ __forceinline__ void flush_slow(const GroupParams &p, const float4 *l
 }
 
 // gravity walk of one group: 32 * TPL PH-contiguous active particles, lane l
-// holds the particles first + l + 32 k
-template <int MODE, int TPL, bool QUAD>
+// holds the particles first + l + 32 k. With parts > 1 this is one of the parts
+// of the group's walk: every part tests the roots, a root that is accepted or is
+// a bundle belongs to part (root mod parts), and the children of an opened root
+// are dealt out the same way.
+template <int MODE, int TPL, bool QUAD, bool SPLIT>
 __device__ void walk_group(const GroupParams &p, WarpSmem &S, const tvg_wnode *__restrict__ wt,
                            const uint32_t *__restrict__ ix, const uint32_t *__restrict__ iy,
                            const uint32_t *__restrict__ iz, const float *__restrict__ mass_f,
                            const float *__restrict__ last_acc, int64_t first, int cnt,
                            const int32_t *__restrict__ active, Target (&t)[TPL], QuadList *QL,
-                           const float4 *__restrict__ wq, int *status)
+                           const float4 *__restrict__ wq, int part, int parts, int *status)
 {
 	const int lane = threadIdx.x & 31;
 	const unsigned lt = (1u << lane) - 1u;
@@ -869,6 +883,8 @@ __device__ void walk_group(const GroupParams &p, WarpSmem &S, const tvg_wnode *_
 			bool accept = false, open_int = false, open_bundle = false, wrap = false, near = false;
 			float4 entry = make_float4(0.f, 0.f, 0.f, 0.f);
 			int nchild = 0, child = 0;
+			const bool root = SPLIT && node < ntop;
+			const bool mine = !root || node % parts == part;
 			if (node >= 0) {
 				const tvg_wnode nd = wt[node];
 				const float dx = ioff(nd.cx, g.cx, p.scale), dy = ioff(nd.cy, g.cy, p.scale),
@@ -878,7 +894,7 @@ __device__ void walk_group(const GroupParams &p, WarpSmem &S, const tvg_wnode *_
 				                                ioff(nd.gy, g.cy, p.scale), ioff(nd.gz, g.cz, p.scale), r2,
 				                                quad_open);
 				if (!open) {
-					accept = true;
+					accept = mine;
 					entry = make_float4(dx, dy, dz, p.gravity * nd.mass);
 					wrap = per_target && (fabsf(dx) > wlimx || fabsf(dy) > wlimy || fabsf(dz) > wlimz);
 					near = r2 < p.near2;
@@ -887,7 +903,7 @@ __device__ void walk_group(const GroupParams &p, WarpSmem &S, const tvg_wnode *_
 					nchild = nd.nchild;
 					child = nd.child;
 				} else {
-					open_bundle = true;
+					open_bundle = mine;
 					nchild = -nd.nchild;
 					child = nd.child;
 				}
@@ -924,7 +940,8 @@ __device__ void walk_group(const GroupParams &p, WarpSmem &S, const tvg_wnode *_
 			if (QUAD) nq += __popc(bm);
 			else nl += __popc(bm);
 			nw += __popc(bw);
-			push_children(S.stack, sp, open_int, nchild, child);
+			if (SPLIT) push_children(S.stack, sp, open_int, nchild, child, part, root ? parts : 1);
+			else push_children(S.stack, sp, open_int, nchild, child);
 			// opened bundles -> bundle queue
 			const unsigned bb = __ballot_sync(0xFFFFFFFFu, open_bundle);
 			if (open_bundle) S.bq[__popc(bb & lt)] = make_int2(child, nchild);
@@ -976,18 +993,42 @@ __device__ void walk_group(const GroupParams &p, WarpSmem &S, const tvg_wnode *_
 	flush_slow<TPL>(p, S.wlist, nw, t);
 	if (QUAD) flush_quad<TPL>(*QL, nq, t);
 #pragma unroll
-	for (int k = 0; k < TPL; k++) t[k].cost -= 1.f;     // the self pair, which the reference skips
+	for (int k = 0; k < TPL; k++)
+		if (!SPLIT || part == 0) t[k].cost -= 1.f;     // the self pair, which the reference skips
 	__syncwarp();
 }
 
-template <int MODE, int TPL, typename F, bool QUAD>
+// Parts of a group's walk: few groups leave the device idle (a warp each) and a
+// few long ones end alone, so the groups are split until there are WALK_ITEMS
+// warps' worth of them, eight for each of the 16 warps an SM holds, but no further
+// than the 64 level-2 cells' children give even shares. Each part has its own
+// sums, which k_walk_sum adds in order. Gravity walk, one warp per group / so: box
+// of 32^3 2.40 / 0.36 ms, halo of 3001 0.31 / 0.11 ms, box of 64^3 with monopoles 28.1 /
+// 22.5 ms (24.4 with four items a warp, 30.1 with two); Ewald walk of the 32^3 box
+// 0.48 / 0.13 ms. A part tests the roots again, 1 to 2 us, so light groups of a halo's
+// active list gain nothing (130,000 of 200,000 active: 0.38 / 0.42 ms).
+#define WALK_ITEMS (148 * 16 * 8)
+#define WALK_MAX_PARTS 32
+__host__ __device__ __forceinline__ int walk_parts(int64_t ngroups)
+{
+	const int64_t p = WALK_ITEMS / (ngroups > 0 ? ngroups : 1);
+	return p < 1 ? 1 : p > WALK_MAX_PARTS ? WALK_MAX_PARTS : (int) p;
+}
+
+// a target's sums of one part
+struct __align__(16) PartSum {
+	double a[3];
+	float cost, qcost;
+};
+
+template <int MODE, int TPL, typename F, bool QUAD, bool SPLIT>
 __global__ void __launch_bounds__(GW_THREADS, GW_WALK_MINB)
 k_walk_group(GroupParams p, const int32_t *__restrict__ active, const int32_t *__restrict__ gfirst,
              const tvg_wnode *__restrict__ wt, const float4 *__restrict__ wq,
              const uint32_t *__restrict__ ix, const uint32_t *__restrict__ iy,
              const uint32_t *__restrict__ iz, const float *__restrict__ mass_f,
              const float *__restrict__ last_acc, F *acc0, F *acc1, F *acc2, F *gacc0, F *gacc1,
-             F *gacc2, F *cost_out, int32_t *work, double *counter, int *status)
+             F *gacc2, F *cost_out, int32_t *work, double *counter, PartSum *sums, int *status)
 {
 	extern __shared__ __align__(16) unsigned char smem_raw[];
 	WarpSmem &S = ((WarpSmem *) smem_raw)[threadIdx.x >> 5];
@@ -996,11 +1037,14 @@ k_walk_group(GroupParams p, const int32_t *__restrict__ active, const int32_t *_
 	const int lane = threadIdx.x & 31;
 	double cnt_acc = 0, qcnt_acc = 0;
 	const int64_t ngroups = p.dc->ngroups;
+	const int parts = SPLIT ? walk_parts(ngroups) : 1;
 	for (;;) {
-		int64_t g = 0;
-		if (lane == 0) g = atomicAdd(work, 1);
-		g = __shfl_sync(0xFFFFFFFFu, g, 0);
-		if (g >= ngroups) break;
+		int64_t item = 0;
+		if (lane == 0) item = atomicAdd(work, 1);
+		item = __shfl_sync(0xFFFFFFFFu, item, 0);
+		if (item >= ngroups * parts) break;
+		const int64_t g = SPLIT ? item / parts : item;
+		const int part = SPLIT ? (int) (item % parts) : 0;
 		int64_t first;
 		int cnt;
 		if (gfirst) {
@@ -1011,12 +1055,16 @@ k_walk_group(GroupParams p, const int32_t *__restrict__ active, const int32_t *_
 			cnt = (int) min((int64_t) p.gsize, p.n - first);
 		}
 		Target t[TPL];
-		walk_group<MODE, TPL, QUAD>(p, S, wt, ix, iy, iz, mass_f, last_acc, first, cnt, active, t, QL, wq,
-		                            status);
+		walk_group<MODE, TPL, QUAD, SPLIT>(p, S, wt, ix, iy, iz, mass_f, last_acc, first, cnt, active, t, QL, wq,
+		                            part, parts, status);
 #pragma unroll
 		for (int k = 0; k < TPL; k++) {
-			if (!t[k].valid) continue;
 			const int slot = lane + 32 * k;
+			if (SPLIT && parts > 1) {
+				sums[item * p.gsize + slot] = { { t[k].ax, t[k].ay, t[k].az }, t[k].cost, t[k].qcost };
+				continue;
+			}
+			if (!t[k].valid) continue;
 			const int64_t i = active ? (int64_t) active[first + slot] : first + slot;
 			acc0[i] += (F) t[k].ax;
 			acc1[i] += (F) t[k].ay;
@@ -1036,6 +1084,55 @@ k_walk_group(GroupParams p, const int32_t *__restrict__ active, const int32_t *_
 	}
 	if (lane == 0 && cnt_acc != 0) atomicAdd(counter, cnt_acc);
 	if (QUAD && lane == 0 && qcnt_acc != 0) atomicAdd(counter + 2, qcnt_acc);
+}
+
+// the parts' sums of each target, in order
+template <typename F>
+__global__ void __launch_bounds__(256)
+k_walk_sum(GroupParams p, const int32_t *__restrict__ active, const int32_t *__restrict__ gfirst,
+           const PartSum *__restrict__ sums, F *acc0, F *acc1, F *acc2, F *gacc0, F *gacc1, F *gacc2, F *cost_out,
+           double *counter)
+{
+	const int64_t ngroups = p.dc->ngroups;
+	const int parts = walk_parts(ngroups);
+	if (parts == 1) return;
+	double cnt = 0, qcnt = 0;
+	for (int64_t e = blockIdx.x * (int64_t) blockDim.x + threadIdx.x; e < ngroups * p.gsize;
+	     e += (int64_t) gridDim.x * blockDim.x) {
+		const int64_t g = e / p.gsize;
+		const int slot = (int) (e % p.gsize);
+		const int64_t first = gfirst ? (int64_t) gfirst[g] : g * p.gsize;
+		const int64_t last = gfirst ? (int64_t) gfirst[g + 1] : min(first + p.gsize, p.n);
+		if (first + slot >= last) continue;
+		PartSum s = { { 0, 0, 0 }, 0, 0 };
+		for (int q = 0; q < parts; q++) {
+			const PartSum v = sums[(g * parts + q) * p.gsize + slot];
+			s.a[0] += v.a[0];
+			s.a[1] += v.a[1];
+			s.a[2] += v.a[2];
+			s.cost += v.cost;
+			s.qcost += v.qcost;
+		}
+		const int64_t i = active ? (int64_t) active[first + slot] : first + slot;
+		acc0[i] += (F) s.a[0];
+		acc1[i] += (F) s.a[1];
+		acc2[i] += (F) s.a[2];
+		gacc0[i] = (F) s.a[0];
+		gacc1[i] = (F) s.a[1];
+		gacc2[i] = (F) s.a[2];
+		cost_out[i] = (F) s.cost;
+		cnt += s.cost;
+		qcnt += s.qcost;
+	}
+#pragma unroll
+	for (int o = 16; o; o >>= 1) {
+		cnt += __shfl_xor_sync(0xFFFFFFFFu, cnt, o);
+		qcnt += __shfl_xor_sync(0xFFFFFFFFu, qcnt, o);
+	}
+	if ((threadIdx.x & 31) == 0) {
+		if (cnt != 0) atomicAdd(counter, cnt);
+		if (qcnt != 0) atomicAdd(counter + 2, qcnt);
+	}
 }
 
 // ------------------------------------------------------ the Ewald walk
@@ -1372,7 +1469,36 @@ __device__ __forceinline__ void ewald_batch(const GroupParams &p, const float *t
 	}
 }
 
-template <int TPL, bool MLP>
+// The targets' part of a group's Ewald walk: K(d_c - t) ~ K - J t + H:tt / 2 from
+// the group's sums (K 3, J xx yy zz xy xz yz, H xxx xxy xxz xyy xyz xzz yyy yyz yzz
+// zzz), and the uniform background's remainder
+#define EW_SUMS 19
+template <int TPL>
+__device__ __forceinline__ void ewald_expand(const GroupParams &p, const double *q, Target (&t)[TPL])
+{
+	const double *K = q, *J = q + 3, *H = q + 9;
+#pragma unroll
+	for (int k = 0; k < TPL; k++) {
+		const double x = t[k].tx, y = t[k].ty, z = t[k].tz;
+		const double xx = 0.5 * x * x, yy = 0.5 * y * y, zz = 0.5 * z * z, xy = x * y, xz = x * z, yz = y * z;
+		double out[3];
+		out[0] = K[0] - (J[0] * x + J[3] * y + J[4] * z)
+		       + (H[0] * xx + H[3] * yy + H[5] * zz + H[1] * xy + H[2] * xz + H[4] * yz);
+		out[1] = K[1] - (J[3] * x + J[1] * y + J[5] * z)
+		       + (H[1] * xx + H[6] * yy + H[8] * zz + H[3] * xy + H[4] * xz + H[7] * yz);
+		out[2] = K[2] - (J[4] * x + J[5] * y + J[2] * z)
+		       + (H[2] * xx + H[7] * yy + H[9] * zz + H[4] * xy + H[5] * xz + H[8] * yz);
+		double rem[3];
+		uniform_remainder(p, x, y, z, rem);
+		t[k].ax = out[0] + rem[0];
+		t[k].ay = out[1] + rem[1];
+		t[k].az = out[2] + rem[2];
+	}
+}
+
+// SPLIT: one of `parts` parts of the group's walk (the roots and the opened
+// roots' children dealt out as in walk_group), whose sums go to `sums`
+template <int TPL, bool MLP, bool SPLIT>
 __device__ void ewald_group(const GroupParams &p, EwaldSmem &S, const tvg_wnode *__restrict__ wt,
                             const uint32_t *__restrict__ ix, const uint32_t *__restrict__ iy,
                             const uint32_t *__restrict__ iz, const float *__restrict__ mass_f,
@@ -1380,7 +1506,7 @@ __device__ void ewald_group(const GroupParams &p, EwaldSmem &S, const tvg_wnode 
                             const float *mlp, const uint32_t *w2b,
                             int64_t first, int cnt, const int32_t *__restrict__ active,
                             Target (&t)[TPL], float &nev, int *status, const float4 *__restrict__ wq_all,
-                            int64_t group, int32_t *wide)
+                            int64_t group, int32_t *wide, int part, int parts, double *sums)
 {
 	const int lane = threadIdx.x & 31;
 	const unsigned lt = (1u << lane) - 1u;
@@ -1391,7 +1517,7 @@ __device__ void ewald_group(const GroupParams &p, EwaldSmem &S, const tvg_wnode 
 	const bool per_target = hmax >= p.taylor_h;
 	// with the table such groups are left to k_ewald_wide (wide[0] counts them)
 	if (!MLP && per_target) {
-		if (lane == 0) wide[1 + atomicAdd(&wide[0], 1)] = (int32_t) group;
+		if (lane == 0 && (!SPLIT || part == 0)) wide[1 + atomicAdd(&wide[0], 1)] = (int32_t) group;
 		return;
 	}
 	// node quadrupoles (TVG_CFG_QUADRUPOLE) in the expansion about the group
@@ -1446,6 +1572,8 @@ __device__ void ewald_group(const GroupParams &p, EwaldSmem &S, const tvg_wnode 
 				bool accept = false, open_int = false, open_bundle = false;
 				float4 entry = make_float4(0.f, 0.f, 0.f, 0.f);
 				int nchild = 0, child = 0;
+				const bool root = SPLIT && node < ntop;
+				const bool mine = !root || node % parts == part;
 				if (node >= 0) {
 					const tvg_wnode nd = wt[node];
 					const float dx = ioff(nd.cx, g.cx, p.scale), dy = ioff(nd.cy, g.cy, p.scale),
@@ -1473,14 +1601,14 @@ __device__ void ewald_group(const GroupParams &p, EwaldSmem &S, const tvg_wnode 
 						} else open = nd.mass * hs2 * 0.125f * l2 > p.ew_rel * g.fac;
 					}
 					if (!open) {
-						accept = true;
+						accept = mine;
 						entry = make_float4(dx, dy, dz, p.gravity * nd.mass);
 					} else if (nd.nchild > 0) {
 						open_int = true;
 						nchild = nd.nchild;
 						child = nd.child;
 					} else {
-						open_bundle = true;
+						open_bundle = mine;
 						nchild = -nd.nchild;
 						child = nd.child;
 					}
@@ -1491,7 +1619,8 @@ __device__ void ewald_group(const GroupParams &p, EwaldSmem &S, const tvg_wnode 
 					S.lnode[nl + __popc(bm & lt)] = node;
 				}
 				nl += __popc(bm);       // below 64: the drain left fewer than 32
-				push_children(S.stack, sp, open_int, nchild, child);
+				if (SPLIT) push_children(S.stack, sp, open_int, nchild, child, part, root ? parts : 1);
+				else push_children(S.stack, sp, open_int, nchild, child);
 				const unsigned bb = __ballot_sync(0xFFFFFFFFu, open_bundle);
 				if (open_bundle) S.bq[__popc(bb & lt)] = make_int2(child, nchild);
 				nb = __popc(bb);
@@ -1537,45 +1666,27 @@ __device__ void ewald_group(const GroupParams &p, EwaldSmem &S, const tvg_wnode 
 	}
 	if (per_target) return;
 	// sum over lanes (FP64), then K(d_c - t) ~ K - J t + H:tt / 2 per target
-	double K[3], J[6], H[10];
+	double q[EW_SUMS];
 #pragma unroll
-	for (int a = 0; a < 3; a++) K[a] = c.k[a];
+	for (int a = 0; a < 3; a++) q[a] = c.k[a];
 #pragma unroll
-	for (int a = 0; a < 6; a++) J[a] = c.j[a];
+	for (int a = 0; a < 6; a++) q[3 + a] = c.j[a];
 #pragma unroll
-	for (int a = 0; a < 10; a++) H[a] = c.h[a];
+	for (int a = 0; a < 10; a++) q[9 + a] = c.h[a];
 #pragma unroll
-	for (int o = 16; o; o >>= 1) {
+	for (int o = 16; o; o >>= 1)
 #pragma unroll
-		for (int a = 0; a < 3; a++) K[a] += __shfl_xor_sync(0xFFFFFFFFu, K[a], o);
+		for (int a = 0; a < EW_SUMS; a++) q[a] += __shfl_xor_sync(0xFFFFFFFFu, q[a], o);
+	if (SPLIT && parts > 1) {
 #pragma unroll
-		for (int a = 0; a < 6; a++) J[a] += __shfl_xor_sync(0xFFFFFFFFu, J[a], o);
-#pragma unroll
-		for (int a = 0; a < 10; a++) H[a] += __shfl_xor_sync(0xFFFFFFFFu, H[a], o);
+		for (int a = 0; a < EW_SUMS; a++)
+			if (lane == a) sums[a] = q[a];
+		return;
 	}
-#pragma unroll
-	for (int k = 0; k < TPL; k++) {
-		const double x = t[k].tx, y = t[k].ty, z = t[k].tz;
-		const double xx = 0.5 * x * x, yy = 0.5 * y * y, zz = 0.5 * z * z, xy = x * y, xz = x * z, yz = y * z;
-		double out[3];
-		out[0] = K[0] - (J[0] * x + J[3] * y + J[4] * z)
-		       + (H[0] * xx + H[3] * yy + H[5] * zz + H[1] * xy + H[2] * xz + H[4] * yz);
-		out[1] = K[1] - (J[3] * x + J[1] * y + J[5] * z)
-		       + (H[1] * xx + H[6] * yy + H[8] * zz + H[3] * xy + H[4] * xz + H[7] * yz);
-		out[2] = K[2] - (J[4] * x + J[5] * y + J[2] * z)
-		       + (H[2] * xx + H[7] * yy + H[9] * zz + H[4] * xy + H[5] * xz + H[8] * yz);
-		double rem[3];
-		uniform_remainder(p, x, y, z, rem);
-		out[0] += rem[0];
-		out[1] += rem[1];
-		out[2] += rem[2];
-		t[k].ax = out[0];
-		t[k].ay = out[1];
-		t[k].az = out[2];
-	}
+	ewald_expand<TPL>(p, q, t);
 }
 
-template <int TPL, bool MLP, typename F>
+template <int TPL, bool MLP, typename F, bool SPLIT>
 __global__ void __launch_bounds__(GE_THREADS, MLP ? 1 : GW_EWALD_MINB)
 k_ewald_group(GroupParams p, const int32_t *__restrict__ active, const int32_t *__restrict__ gfirst,
               const tvg_wnode *__restrict__ wt,
@@ -1584,7 +1695,7 @@ k_ewald_group(GroupParams p, const int32_t *__restrict__ active, const int32_t *
               const float *__restrict__ last_acc, const float *__restrict__ tay,
               const __nv_bfloat16 *__restrict__ mlp_w, const float *__restrict__ mlp_f32, F *acc0, F *acc1,
               F *acc2, F *gacc0, F *gacc1, F *gacc2, int32_t *work, double *counter, int *status,
-              const float4 *__restrict__ wq, int32_t *wide)
+              const float4 *__restrict__ wq, int32_t *wide, double *sums)
 {
 	extern __shared__ __align__(16) unsigned char smem_raw[];
 	EwaldSmem &S = ((EwaldSmem *) smem_raw)[threadIdx.x >> 5];
@@ -1599,11 +1710,13 @@ k_ewald_group(GroupParams p, const int32_t *__restrict__ active, const int32_t *
 	const int lane = threadIdx.x & 31;
 	double ev_acc = 0;
 	const int64_t ngroups = p.dc->ngroups;
+	const int parts = SPLIT ? walk_parts(ngroups) : 1;
 	for (;;) {
-		int64_t g = 0;
-		if (lane == 0) g = atomicAdd(work, 1);
-		g = __shfl_sync(0xFFFFFFFFu, g, 0);
-		if (g >= ngroups) break;
+		int64_t item = 0;
+		if (lane == 0) item = atomicAdd(work, 1);
+		item = __shfl_sync(0xFFFFFFFFu, item, 0);
+		if (item >= ngroups * parts) break;
+		const int64_t g = SPLIT ? item / parts : item;
 		int64_t first;
 		int cnt;
 		if (gfirst) {
@@ -1615,9 +1728,11 @@ k_ewald_group(GroupParams p, const int32_t *__restrict__ active, const int32_t *
 		}
 		Target t[TPL];
 		float nev = 0.f;
-		ewald_group<TPL, MLP>(p, S, wt, ix, iy, iz, mass_f, last_acc, tay, mlp, w2b, first, cnt, active, t, nev,
-		                      status, wq, g, wide);
+		ewald_group<TPL, MLP, SPLIT>(p, S, wt, ix, iy, iz, mass_f, last_acc, tay, mlp, w2b, first, cnt, active, t, nev,
+		                             status, wq, g, wide, SPLIT ? (int) (item % parts) : 0, parts,
+		                             sums + EW_SUMS * item);
 		ev_acc += nev;
+		if (SPLIT && parts > 1) continue;          // k_ewald_sum
 #pragma unroll
 		for (int k = 0; k < TPL; k++) {
 			if (!t[k].valid) continue;
@@ -1647,7 +1762,7 @@ k_ewald_group(GroupParams p, const int32_t *__restrict__ active, const int32_t *
 #define WIDE_ITEMS 4736
 __device__ __forceinline__ int wide_parts(int nwide, int ntop)
 {
-	return max(1, min(ntop, WIDE_ITEMS / max(nwide, 1)));
+	return max(1, min(min(ntop, 64), WIDE_ITEMS / max(nwide, 1)));
 }
 
 template <int TPL>
@@ -1862,6 +1977,47 @@ __global__ void k_ewald_wide_sum(GroupParams p, const int32_t *__restrict__ acti
 	}
 }
 
+// split groups without per-target images: a warp per group adds the parts' sums in
+// order and expands them for the targets
+template <int TPL, typename F>
+__global__ void __launch_bounds__(GE_THREADS)
+k_ewald_sum(GroupParams p, const int32_t *__restrict__ active, const int32_t *__restrict__ gfirst,
+            const uint32_t *__restrict__ ix, const uint32_t *__restrict__ iy, const uint32_t *__restrict__ iz,
+            const float *__restrict__ last_acc, const double *__restrict__ sums, F *acc0, F *acc1, F *acc2,
+            F *gacc0, F *gacc1, F *gacc2)
+{
+	const int64_t ngroups = p.dc->ngroups;
+	const int parts = walk_parts(ngroups), lane = threadIdx.x & 31;
+	if (parts == 1) return;
+	for (int64_t gi = (blockIdx.x * (int64_t) blockDim.x + threadIdx.x) >> 5; gi < ngroups;
+	     gi += ((int64_t) gridDim.x * blockDim.x) >> 5) {
+		const int64_t first = gfirst ? (int64_t) gfirst[gi] : gi * p.gsize;
+		const int64_t last = gfirst ? (int64_t) gfirst[gi + 1] : min(first + p.gsize, p.n);
+		Target t[TPL];
+		GroupBox g;
+		group_setup<TPL>(p, ix, iy, iz, last_acc, active, first, (int) (last - first), t, g);
+		if (fmaxf(g.hx, fmaxf(g.hy, g.hz)) >= p.taylor_h) continue;      // k_ewald_wide
+		double mine = 0, q[EW_SUMS];
+		if (lane < EW_SUMS)
+			for (int k = 0; k < parts; k++) mine += sums[EW_SUMS * (gi * parts + k) + lane];
+#pragma unroll
+		for (int a = 0; a < EW_SUMS; a++) q[a] = __shfl_sync(0xFFFFFFFFu, mine, a);
+		ewald_expand<TPL>(p, q, t);
+#pragma unroll
+		for (int k = 0; k < TPL; k++) {
+			if (!t[k].valid) continue;
+			const int slot = lane + 32 * k;
+			const int64_t i = active ? (int64_t) active[first + slot] : first + slot;
+			acc0[i] += (F) t[k].ax;
+			acc1[i] += (F) t[k].ay;
+			acc2[i] += (F) t[k].az;
+			gacc0[i] += (F) t[k].ax;
+			gacc1[i] += (F) t[k].ay;
+			gacc2[i] += (F) t[k].az;
+		}
+	}
+}
+
 template <typename F>
 __global__ void k_to_float(int64_t n, const F *__restrict__ a, float *__restrict__ b)
 {
@@ -2011,7 +2167,7 @@ static int blocks_for(tvg_context *ctx, K kernel, size_t smem, int *cache, int t
 	return TVG_OK;
 }
 
-template <int MODE, int TPL, typename F, bool QUAD>
+template <int MODE, int TPL, typename F, bool QUAD, bool SPLIT>
 static int launch_walk_q(tvg_context *ctx, GroupParams p, const float *mass_f, const float *last_f,
                          double *counter)
 {
@@ -2019,26 +2175,44 @@ static int launch_walk_q(tvg_context *ctx, GroupParams p, const float *mass_f, c
 	TVG_CHECK(device_slot(ctx));
 	int &nblk = nblk_dev[ctx->device];
 	const size_t smem = (sizeof(WarpSmem) + (QUAD ? sizeof(QuadList) : 0)) * GW_WARPS;
-	TVG_CHECK(blocks_for(ctx, k_walk_group<MODE, TPL, F, QUAD>, smem, &nblk));
-	k_walk_group<MODE, TPL, F, QUAD><<<TVG_CNT(ctx, nblk), GW_THREADS, smem, ctx->stream>>>(
-	    p, ctx->use_active ? ctx->active : nullptr, ctx->use_active ? ctx->group_first : nullptr,
-	    ctx->wtree, ctx->wquad, ctx->ipos[0], ctx->ipos[1],
-	    ctx->ipos[2], mass_f, last_f, (F *) ctx->f[FS_ACC0], (F *) ctx->f[FS_ACC1],
-	    (F *) ctx->f[FS_ACC2], (F *) ctx->f[FS_GACC0], (F *) ctx->f[FS_GACC1], (F *) ctx->f[FS_GACC2],
-	    (F *) ctx->f[FS_COST], ctx->work_counter, counter, ctx->status);
+	TVG_CHECK(blocks_for(ctx, k_walk_group<MODE, TPL, F, QUAD, SPLIT>, smem, &nblk));
+	const int32_t *act = ctx->use_active ? ctx->active : nullptr, *gf = ctx->use_active ? ctx->group_first : nullptr;
+	F *a[7] = { (F *) ctx->f[FS_ACC0], (F *) ctx->f[FS_ACC1], (F *) ctx->f[FS_ACC2], (F *) ctx->f[FS_GACC0],
+	            (F *) ctx->f[FS_GACC1], (F *) ctx->f[FS_GACC2], (F *) ctx->f[FS_COST] };
+	k_walk_group<MODE, TPL, F, QUAD, SPLIT><<<TVG_CNT(ctx, nblk), GW_THREADS, smem, ctx->stream>>>(
+	    p, act, gf, ctx->wtree, ctx->wquad, ctx->ipos[0], ctx->ipos[1], ctx->ipos[2], mass_f, last_f, a[0], a[1],
+	    a[2], a[3], a[4], a[5], a[6], ctx->work_counter, counter, (PartSum *) ctx->part_sums, ctx->status);
+	if (SPLIT)
+		k_walk_sum<F><<<TVG_CNT(ctx, 148 * 4), 256, 0, ctx->stream>>>(
+		    p, act, gf, (const PartSum *) ctx->part_sums, a[0], a[1], a[2], a[3], a[4], a[5], a[6], counter);
 	TVG_CUDA(ctx, cudaGetLastError());
 	return TVG_OK;
+}
+
+// whether the groups may be split: from the number of groups, or, for an active
+// list, whose length the device knows, always (its kernels then decide). FP64
+// contexts keep a warp per group: they return the FP32 sums at full width, and a
+// split changes the sums' order (1e-7 of the force).
+static bool may_split(const tvg_context *ctx, const GroupParams &p)
+{
+	return ctx->cfg.float_bytes == 4 && (ctx->use_active || walk_parts((ctx->n + p.gsize - 1) / p.gsize) > 1);
 }
 
 template <int MODE, int TPL, typename F>
 static int launch_walk(tvg_context *ctx, GroupParams p, const float *mass_f, const float *last_f,
                        double *counter)
 {
-	if (p.quad) return launch_walk_q<MODE, TPL, F, true>(ctx, p, mass_f, last_f, counter);
-	return launch_walk_q<MODE, TPL, F, false>(ctx, p, mass_f, last_f, counter);
+	if constexpr (sizeof(F) == 4) {
+		if (may_split(ctx, p)) {
+			if (p.quad) return launch_walk_q<MODE, TPL, F, true, true>(ctx, p, mass_f, last_f, counter);
+			return launch_walk_q<MODE, TPL, F, false, true>(ctx, p, mass_f, last_f, counter);
+		}
+	}
+	if (p.quad) return launch_walk_q<MODE, TPL, F, true, false>(ctx, p, mass_f, last_f, counter);
+	return launch_walk_q<MODE, TPL, F, false, false>(ctx, p, mass_f, last_f, counter);
 }
 
-template <int TPL, bool MLP, typename F>
+template <int TPL, bool MLP, typename F, bool SPLIT>
 static int launch_ewald(tvg_context *ctx, GroupParams p, const float *mass_f, const float *last_f,
                         double *counter)
 {
@@ -2047,30 +2221,30 @@ static int launch_ewald(tvg_context *ctx, GroupParams p, const float *mass_f, co
 	int &nblk = nblk_dev[ctx->device];
 	const size_t smem = sizeof(EwaldSmem) * GE_WARPS
 	                  + (MLP ? 4 * MLP_NPARAM + 2 * MLP_H * MLP_H : 0);
-	TVG_CHECK(blocks_for(ctx, k_ewald_group<TPL, MLP, F>, smem, &nblk, GE_THREADS));
-	k_ewald_group<TPL, MLP, F><<<TVG_CNT(ctx, nblk), GE_THREADS, smem, ctx->stream>>>(
-	    p, ctx->use_active ? ctx->active : nullptr, ctx->use_active ? ctx->group_first : nullptr,
-	    ctx->wtree, ctx->ipos[0], ctx->ipos[1],
-	    ctx->ipos[2], mass_f, last_f, ctx->ewald_taylor, (const __nv_bfloat16 *) ctx->mlp_bf16, ctx->mlp_prm,
-	    (F *) ctx->f[FS_ACC0],
-	    (F *) ctx->f[FS_ACC1], (F *) ctx->f[FS_ACC2], (F *) ctx->f[FS_GACC0], (F *) ctx->f[FS_GACC1],
-	    (F *) ctx->f[FS_GACC2], ctx->work_counter + 1, counter, ctx->status,
-	    p.quad ? (const float4 *) ctx->wquad : nullptr, ctx->wide_list);
+	TVG_CHECK(blocks_for(ctx, k_ewald_group<TPL, MLP, F, SPLIT>, smem, &nblk, GE_THREADS));
+	const int32_t *act = ctx->use_active ? ctx->active : nullptr, *gf = ctx->use_active ? ctx->group_first : nullptr;
+	F *a[6] = { (F *) ctx->f[FS_ACC0], (F *) ctx->f[FS_ACC1], (F *) ctx->f[FS_ACC2],
+	            (F *) ctx->f[FS_GACC0], (F *) ctx->f[FS_GACC1], (F *) ctx->f[FS_GACC2] };
+	double *sums = (double *) ctx->part_sums;
+	k_ewald_group<TPL, MLP, F, SPLIT><<<TVG_CNT(ctx, nblk), GE_THREADS, smem, ctx->stream>>>(
+	    p, act, gf, ctx->wtree, ctx->ipos[0], ctx->ipos[1], ctx->ipos[2], mass_f, last_f, ctx->ewald_taylor,
+	    (const __nv_bfloat16 *) ctx->mlp_bf16, ctx->mlp_prm, a[0], a[1], a[2], a[3], a[4], a[5],
+	    ctx->work_counter + 1, counter, ctx->status, p.quad ? (const float4 *) ctx->wquad : nullptr,
+	    ctx->wide_list, sums);
 	TVG_CUDA(ctx, cudaGetLastError());
 	if constexpr (!MLP) {
+		if (SPLIT)
+			k_ewald_sum<TPL, F><<<TVG_CNT(ctx, 148 * 4), GE_THREADS, 0, ctx->stream>>>(
+			    p, act, gf, ctx->ipos[0], ctx->ipos[1], ctx->ipos[2], last_f, sums, a[0], a[1], a[2], a[3], a[4], a[5]);
 		static int nwide_dev[TVG_MAX_DEVICES] = { 0 };
 		int &nb = nwide_dev[ctx->device];
 		const size_t sm = sizeof(EwaldSmem) * GE_WARPS;
 		TVG_CHECK(blocks_for(ctx, k_ewald_wide<TPL, F>, sm, &nb, GE_THREADS));
-		const int32_t *act = ctx->use_active ? ctx->active : nullptr, *gf = ctx->use_active ? ctx->group_first : nullptr;
-		F *a[6] = { (F *) ctx->f[FS_ACC0], (F *) ctx->f[FS_ACC1], (F *) ctx->f[FS_ACC2],
-		            (F *) ctx->f[FS_GACC0], (F *) ctx->f[FS_GACC1], (F *) ctx->f[FS_GACC2] };
 		k_ewald_wide<TPL, F><<<TVG_CNT(ctx, nb), GE_THREADS, sm, ctx->stream>>>(
 		    p, act, gf, ctx->wtree, ctx->ipos[0], ctx->ipos[1], ctx->ipos[2], mass_f, last_f, ctx->ewald_wide,
-		    a[0], a[1], a[2], a[3], a[4], a[5], ctx->wide_list, ctx->wide_part, ctx->work_counter + 2, counter,
-		    ctx->status);
+		    a[0], a[1], a[2], a[3], a[4], a[5], ctx->wide_list, sums, ctx->work_counter + 2, counter, ctx->status);
 		k_ewald_wide_sum<F><<<TVG_CNT(ctx, 148), 256, 0, ctx->stream>>>(
-		    p, act, gf, ctx->wide_list, ctx->wide_part, a[0], a[1], a[2], a[3], a[4], a[5]);
+		    p, act, gf, ctx->wide_list, sums, a[0], a[1], a[2], a[3], a[4], a[5]);
 		TVG_CUDA(ctx, cudaGetLastError());
 	}
 	return TVG_OK;
@@ -2096,9 +2270,11 @@ static int launch_pair(tvg_context *ctx, const GroupParams &p, bool ewald, bool 
 	if (ewald) TVG_CHECK((launch_walk<GM_CENTRE, TPL, F>(ctx, p, mass_f, last_f, cnt)));
 	else TVG_CHECK((launch_walk<GM_NEAREST, TPL, F>(ctx, p, mass_f, last_f, cnt)));
 	TVG_CUDA(ctx, tvg_record(ctx, ctx->ev[1]));
-	if (ewald && mlp) TVG_CHECK((launch_ewald<TPL, true, F>(ctx, p, mass_f, last_f, cnt + 1)));
-	else if (ewald) TVG_CHECK((launch_ewald<TPL, false, F>(ctx, p, mass_f, last_f, cnt + 1)));
-	return TVG_OK;
+	if (!ewald) return TVG_OK;
+	if (mlp) return launch_ewald<TPL, true, F, false>(ctx, p, mass_f, last_f, cnt + 1);
+	if constexpr (sizeof(F) == 4)
+		if (may_split(ctx, p)) return launch_ewald<TPL, false, F, true>(ctx, p, mass_f, last_f, cnt + 1);
+	return launch_ewald<TPL, false, F, false>(ctx, p, mass_f, last_f, cnt + 1);
 }
 
 template <typename F>
@@ -2122,13 +2298,17 @@ static int walk_group_typed(tvg_context *ctx, int use_bh, uint32_t parts, int ew
 		                "the table (tvg_ewald_mlp_validate)");
 	cudaStream_t s = ctx->stream;
 	if (!ctx->have_walktree) TVG_CHECK(prepare_typed<F>(ctx));
+	// the parts' sums of both walks, for the largest groups: at most WALK_ITEMS
+	// items, and no more than the capacity's groups in 64 parts
+	if (!ctx->part_sums) {
+		const int64_t most = (ctx->cap / 32 + 1) * 64, items = most < WALK_ITEMS ? most : WALK_ITEMS;
+		TVG_CUDA(ctx, cudaMalloc(&ctx->part_sums, sizeof(PartSum) * 128 * (size_t) items));
+	}
 	if (ewald && !mlp) {
 		if (!ctx->ewald_wide) TVG_CHECK(tvg_impl_ewald_wide(ctx));
-		// the list holds every group (at most one per 32 particles), the partial
-		// sums WIDE_ITEMS items of the largest groups
+		// the list holds every group (at most one per 32 particles)
 		if (!ctx->wide_list)
 			TVG_CUDA(ctx, cudaMalloc((void **) &ctx->wide_list, 4 * (size_t) (ctx->cap / 32 + 1024)));
-		if (!ctx->wide_part) TVG_CUDA(ctx, cudaMalloc((void **) &ctx->wide_part, 24 * (size_t) WIDE_ITEMS * 128));
 		TVG_CUDA(ctx, cudaMemsetAsync(ctx->wide_list, 0, 4, s));
 	}
 	if (ewald && !ctx->ewald_taylor) TVG_CHECK(tvg_impl_ewald_taylor(ctx));

@@ -333,3 +333,34 @@ def test_wide_groups_split(fsize, flags, use_bh):
         assert 0 < tot < ew_all
     if not use_bh:
         assert err["rms"] < 1e-2
+
+
+@pytest.mark.parametrize("periodic", [False, True])
+@pytest.mark.parametrize("flags", [0, G.CFG_QUADRUPOLE])
+def test_split_groups(periodic, flags):
+    """Few groups are split into parts (k_walk_sum, k_ewald_sum): 700,000
+    particles make 10,938 groups, one warp each; active windows of the same
+    order make few groups of the same particles in 2 to 32 parts. Forces equal
+    up to the order of FP32 sums carried in FP64 (1e-4 of the largest component,
+    as for the wide groups), counts exactly."""
+    n = 700_000
+    p = ics.random_box(n, box=1000.0, seed=91, clumps=6)
+    parts = G.WALK_GRAVITY | (G.WALK_EWALD if periodic else 0)
+    with G.GravityContext(n, periodic=periodic, boxsize=1000.0 if periodic else 0.0, softening=p.softening,
+                          flags=flags, open_rel=8e-3) as ctx:
+        ctx.upload(p.pos, p.mass, last_acc=np.full(n, 3.0))
+        ctx.set_domain((0.0, 0.0, 0.0), 1000.0)
+        ctx.set_ewald_opening(1e-2)
+        ctx.force_step(form=G.FORM_GROUP, use_bh=False, parts=parts)
+        full = ctx.download(G.F_GRAV_ACC | G.F_COST)
+        acc, cost = full["grav_acc"].astype(np.float64), full["cost"]
+        for windows in (np.arange(1), np.arange(3, 200, 2), np.arange(0, 10_000, 2), np.arange(10_937, 10_938)):
+            active = (64 * windows[:, None] + np.arange(64)[None]).reshape(-1)
+            active = active[active < n]
+            ctx.set_active(active)
+            ctx.walk(G.FORM_GROUP, use_bh=False, parts=parts)
+            got = ctx.download(G.F_GRAV_ACC | G.F_COST)
+            np.testing.assert_array_equal(got["cost"][active], cost[active])
+            d = np.abs(got["grav_acc"].astype(np.float64)[:, active] - acc[:, active])
+            assert d.max() < 1e-4 * np.abs(acc).max()
+            assert ctx.walk_counters()[0] == cost[active].astype(np.float64).sum()
