@@ -450,15 +450,19 @@ struct GroupParams {
 // float4 slots lxy[q] = (x0, x1, y0, y1) and lzw[q] = (z0, z1, w0, w1), so that
 // each lane meets two sources with one packed f32x2 instruction per operation
 // while its target's coordinates stay in registers as (t, t) pairs.
-struct WarpSmem {
-	int32_t stack[GW_STACK];
-	float4 lxy[GW_LIST / 2];   // far sources (bare 1/r^2 kernel): x, y of a pair
-	float4 lzw[GW_LIST / 2];   // far sources: z, G m of a pair
+template <int STACK, int LIST> struct WarpSmemT {
+	static constexpr int kStack = STACK, kList = LIST;
+	int32_t stack[STACK];
+	float4 lxy[LIST / 2];      // far sources (bare 1/r^2 kernel): x, y of a pair
+	float4 lzw[LIST / 2];      // far sources: z, G m of a pair
 	float4 wlist[GW_WLIST];    // near sources (w > 0) and, per-target image, half-box-plane sources (w < 0)
 	int2 bq[GW_BQ];
 };
 
-__device__ __forceinline__ void far_put(WarpSmem &S, int i, float4 e)
+typedef WarpSmemT<GW_STACK, GW_LIST> WarpSmem;
+
+template <typename SM>
+__device__ __forceinline__ void far_put(SM &S, int i, float4 e)
 {
 	float *a = (float *) &S.lxy[i >> 1], *b = (float *) &S.lzw[i >> 1];
 	const int o = i & 1;
@@ -593,14 +597,15 @@ __device__ __forceinline__ bool gravity_opens(const GroupParams &p, const GroupB
 // node at a time: from there on the stack holds at most 7 siblings per level
 // of the current path (<= 40 levels below the top nodes), which the reserve
 // covers, so the stack cannot overflow.
+template <int STACK = GW_STACK>
 __device__ __forceinline__ int pop_nodes(const int32_t *stack, int &sp, int *status, bool &stop)
 {
 	const int lane = threadIdx.x & 31;
 	int k = min(32, sp);
-	const int room = (GW_STACK - GW_RESERVE - sp) / 7;
+	const int room = (STACK - GW_RESERVE - sp) / 7;
 	if (room < k) k = max(room, 1);
 	stop = false;
-	if (sp + 7 * k > GW_STACK) {
+	if (sp + 7 * k > STACK) {
 		atomicOr(status, TVG_ST_LIST_OVERFLOW);
 		stop = true;
 		return -1;
@@ -662,8 +667,8 @@ __device__ __forceinline__ void pair_full(const GroupParams &p, float dx, float 
 // loop is bound by the FMA pipe rather than by instruction issue. The even
 // and odd sources are summed separately and added at the end of the flush.
 // An odd count is padded with a massless source far away (adds exactly 0).
-template <int TPL>
-__device__ __forceinline__ void flush_far(WarpSmem &S, int nl, Target (&t)[TPL])
+template <int TPL, typename SM>
+__device__ __forceinline__ void flush_far(SM &S, int nl, Target (&t)[TPL])
 {
 	if (nl & 1) {
 		if ((threadIdx.x & 31) == 0) far_put(S, nl, make_float4(1.0e15f, 0.f, 0.f, 0.f));
@@ -841,8 +846,8 @@ __device__ __forceinline__ void flush_slow(const GroupParams &p, const float4 *l
 // of the group's walk: every part tests the roots, a root that is accepted or is
 // a bundle belongs to part (root mod parts), and the children of an opened root
 // are dealt out the same way.
-template <int MODE, int TPL, bool QUAD, bool SPLIT>
-__device__ void walk_group(const GroupParams &p, WarpSmem &S, const tvg_wnode *__restrict__ wt,
+template <int MODE, int TPL, bool QUAD, bool SPLIT, bool FREE, typename SM>
+__device__ void walk_group(const GroupParams &p, SM &S, const tvg_wnode *__restrict__ wt,
                            const uint32_t *__restrict__ ix, const uint32_t *__restrict__ iy,
                            const uint32_t *__restrict__ iz, const float *__restrict__ mass_f,
                            const float *__restrict__ last_acc, int64_t first, int cnt,
@@ -878,7 +883,7 @@ __device__ void walk_group(const GroupParams &p, WarpSmem &S, const tvg_wnode *_
 		while (sp > 0) {
 			if (++guard > p.max_iter) { atomicOr(status, TVG_ST_TIMEOUT); halt = true; break; }
 			bool stop;
-			const int node = pop_nodes(S.stack, sp, status, stop);
+			const int node = pop_nodes<SM::kStack>(S.stack, sp, status, stop);
 			if (stop) { halt = true; break; }
 			bool accept = false, open_int = false, open_bundle = false, wrap = false, near = false;
 			float4 entry = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -922,8 +927,8 @@ __device__ void walk_group(const GroupParams &p, WarpSmem &S, const tvg_wnode *_
 					nq = 0;
 					__syncwarp();
 				}
-			} else if (nl + __popc(bm) > GW_LIST) {
-				flush_far<TPL>(S, nl, t);
+			} else if (nl + __popc(bm) > SM::kList) {
+				flush_far<TPL, SM>(S, nl, t);
 				nl = 0;
 				__syncwarp();
 			}
@@ -943,53 +948,81 @@ __device__ void walk_group(const GroupParams &p, WarpSmem &S, const tvg_wnode *_
 			if (SPLIT) push_children(S.stack, sp, open_int, nchild, child, part, root ? parts : 1);
 			else push_children(S.stack, sp, open_int, nchild, child);
 			// opened bundles -> bundle queue
+			if (FREE && nchild <= 0) open_bundle = false;
 			const unsigned bb = __ballot_sync(0xFFFFFFFFu, open_bundle);
-			if (open_bundle) S.bq[__popc(bb & lt)] = make_int2(child, nchild);
-			__syncwarp();
-			const int nb = __popc(bb);
-			for (int b = 0; b < nb; b++) {
-				const int2 q = S.bq[b];
-				for (int o = 0; o < q.y; o += 32) {
-					const int j = o + lane;
-					const bool have = j < q.y;
-					float4 e = make_float4(0.f, 0.f, 0.f, 0.f);
-					bool wr = false, nr = false;
-					if (have) {
-						const int64_t jp = (int64_t) q.x + j;
-						e.x = ioff(ix[jp], g.cx, p.scale);
-						e.y = ioff(iy[jp], g.cy, p.scale);
-						e.z = ioff(iz[jp], g.cz, p.scale);
-						e.w = p.gravity * mass_f[jp];
-						const float ax = fmaxf(fabsf(e.x) - g.hx, 0.f), ay = fmaxf(fabsf(e.y) - g.hy, 0.f),
-						            az = fmaxf(fabsf(e.z) - g.hz, 0.f);
-						nr = ax * ax + ay * ay + az * az < p.near2;
-						wr = per_target && (fabsf(e.x) > wlimx || fabsf(e.y) > wlimy || fabsf(e.z) > wlimz);
-					}
-					const bool tm = have && !wr && !nr, tw = have && (wr || nr);
-					if (wr) e.w = -e.w;
-					const unsigned m1 = __ballot_sync(0xFFFFFFFFu, tm), m2 = __ballot_sync(0xFFFFFFFFu, tw);
-					if (nl + __popc(m1) > GW_LIST) {
-						flush_far<TPL>(S, nl, t);
-						nl = 0;
-						__syncwarp();
-					}
-					if (nw + __popc(m2) > GW_WLIST) {
-						flush_slow<TPL>(p, S.wlist, nw, t);
-						nw = 0;
-						__syncwarp();
-					}
-					if (tm) far_put(S, nl + __popc(m1 & lt), e);
-					if (tw) S.wlist[nw + __popc(m2 & lt)] = e;
-					nl += __popc(m1);
-					nw += __popc(m2);
+			auto particle = [&](bool have, int64_t jp) {
+				float4 e = make_float4(0.f, 0.f, 0.f, 0.f);
+				bool wr = false, nr = false;
+				if (have) {
+					e.x = ioff(ix[jp], g.cx, p.scale);
+					e.y = ioff(iy[jp], g.cy, p.scale);
+					e.z = ioff(iz[jp], g.cz, p.scale);
+					e.w = p.gravity * mass_f[jp];
+					const float ax = fmaxf(fabsf(e.x) - g.hx, 0.f), ay = fmaxf(fabsf(e.y) - g.hy, 0.f),
+					            az = fmaxf(fabsf(e.z) - g.hz, 0.f);
+					nr = ax * ax + ay * ay + az * az < p.near2;
+					wr = per_target && (fabsf(e.x) > wlimx || fabsf(e.y) > wlimy || fabsf(e.z) > wlimz);
+				}
+				const bool tm = have && !wr && !nr, tw = have && (wr || nr);
+				if (wr) e.w = -e.w;
+				const unsigned m1 = __ballot_sync(0xFFFFFFFFu, tm), m2 = __ballot_sync(0xFFFFFFFFu, tw);
+				if (nl + __popc(m1) > SM::kList) {
+					flush_far<TPL, SM>(S, nl, t);
+					nl = 0;
 					__syncwarp();
+				}
+				if (nw + __popc(m2) > GW_WLIST) {
+					flush_slow<TPL>(p, S.wlist, nw, t);
+					nw = 0;
+					__syncwarp();
+				}
+				if (tm) far_put(S, nl + __popc(m1 & lt), e);
+				if (tw) S.wlist[nw + __popc(m2 & lt)] = e;
+				nl += __popc(m1);
+				nw += __popc(m2);
+				__syncwarp();
+			};
+			if (FREE) {
+				// the bundles' particles in one run, 32 at a time: lane l of the chunk
+				// at o takes particle o + l of the run, in the bundle whose start is the
+				// last at or before it. Most bundles hold far fewer than 32: one round
+				// a bundle left most lanes idle (256^3 box, walk 153.3 -> 148.0
+				// ms; 32^3 box 0.40 -> 0.32)
+				if (bb) {
+					const int c = open_bundle ? nchild : 0;
+					int incl = c;
+#pragma unroll
+					for (int o = 1; o < 32; o <<= 1) {
+						const int u = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+						if (lane >= o) incl += u;
+					}
+					const int start = incl - c, total = __shfl_sync(0xFFFFFFFFu, incl, 31);
+					if (open_bundle) S.bq[__popc(bb & lt)] = make_int2(child - start, 0);
+					__syncwarp();
+					int before = 0;                // bundles that start before the chunk
+					for (int o = 0; o < total; o += 32) {
+						const bool in = open_bundle && start >= o && start < o + 32;
+						const unsigned starts = __reduce_or_sync(0xFFFFFFFFu, in ? 1u << (start - o) : 0u);
+						const int b = before + __popc(starts & (lt | 1u << lane)) - 1;
+						const bool have = o + lane < total;
+						particle(have, have ? (int64_t) S.bq[b].x + o + lane : 0);
+						before += __popc(starts);
+					}
+				}
+			} else {
+				if (open_bundle) S.bq[__popc(bb & lt)] = make_int2(child, nchild);
+				__syncwarp();
+				const int nb = __popc(bb);
+				for (int b = 0; b < nb; b++) {
+					const int2 q = S.bq[b];
+					for (int o = 0; o < q.y; o += 32) particle(o + lane < q.y, (int64_t) q.x + o + lane);
 				}
 			}
 			__syncwarp();
 		}
 	}
 	__syncwarp();
-	flush_far<TPL>(S, nl, t);
+	flush_far<TPL, SM>(S, nl, t);
 	flush_slow<TPL>(p, S.wlist, nw, t);
 	if (QUAD) flush_quad<TPL>(*QL, nq, t);
 #pragma unroll
@@ -1015,6 +1048,20 @@ __host__ __device__ __forceinline__ int walk_parts(int64_t ngroups)
 	return p < 1 ? 1 : p > WALK_MAX_PARTS ? WALK_MAX_PARTS : (int) p;
 }
 
+// The warp's memory. A pop takes at most 1/7 of the stack's free room, so a short
+// stack empties the batches, and what an SM's shared memory does not hold is L1,
+// on which the traversal lives. With quadrupoles the far list holds only bundles'
+// particles, so FP32 contexts shorten it and deepen the stack: 256^3 box, walk
+// 148.0 ms with 1024 entries + 256 sources, 146.1 with 1536 + 128 (768 + 128:
+// 184; 1024 + 64: 149.2; 2048 + 128: 145.8, but 12.6 instead of 12.4 ms on the
+// 100^3 box). FP64 contexts keep the flush points of the longer lists, and with
+// them the bits of their sums.
+#define GW_STACK_QUAD 1536
+#define GW_LIST_QUAD 128
+template <typename F, bool QUAD> struct walk_smem_of { typedef WarpSmem type; };
+template <> struct walk_smem_of<float, true> { typedef WarpSmemT<GW_STACK_QUAD, GW_LIST_QUAD> type; };
+template <typename F, bool QUAD> using walk_smem = typename walk_smem_of<F, QUAD>::type;
+
 // a target's sums of one part
 struct __align__(16) PartSum {
 	double a[3];
@@ -1031,8 +1078,9 @@ k_walk_group(GroupParams p, const int32_t *__restrict__ active, const int32_t *_
              F *gacc2, F *cost_out, int32_t *work, double *counter, PartSum *sums, int *status)
 {
 	extern __shared__ __align__(16) unsigned char smem_raw[];
-	WarpSmem &S = ((WarpSmem *) smem_raw)[threadIdx.x >> 5];
-	QuadList *QL = QUAD ? ((QuadList *) (smem_raw + sizeof(WarpSmem) * GW_WARPS)) + (threadIdx.x >> 5)
+	typedef walk_smem<F, QUAD> SM;
+	SM &S = ((SM *) smem_raw)[threadIdx.x >> 5];
+	QuadList *QL = QUAD ? ((QuadList *) (smem_raw + sizeof(SM) * GW_WARPS)) + (threadIdx.x >> 5)
 	                    : nullptr;
 	const int lane = threadIdx.x & 31;
 	double cnt_acc = 0, qcnt_acc = 0;
@@ -1055,8 +1103,8 @@ k_walk_group(GroupParams p, const int32_t *__restrict__ active, const int32_t *_
 			cnt = (int) min((int64_t) p.gsize, p.n - first);
 		}
 		Target t[TPL];
-		walk_group<MODE, TPL, QUAD, SPLIT>(p, S, wt, ix, iy, iz, mass_f, last_acc, first, cnt, active, t, QL, wq,
-		                            part, parts, status);
+		walk_group<MODE, TPL, QUAD, SPLIT, sizeof(F) == 4>(p, S, wt, ix, iy, iz, mass_f, last_acc, first, cnt,
+		                                               active, t, QL, wq, part, parts, status);
 #pragma unroll
 		for (int k = 0; k < TPL; k++) {
 			const int slot = lane + 32 * k;
@@ -1856,7 +1904,7 @@ __device__ void ewald_wide_item(const GroupParams &p, EwaldSmem &S, const tvg_wn
 		if (accept) S.list[nl + __popc(bm & lt)] = entry;
 		nl += __popc(bm);               // below 64: fewer than 32 were left
 		push_children(S.stack, sp, open_int, nchild, child);
-		const unsigned bb = __ballot_sync(0xFFFFFFFFu, open_bundle);
+			const unsigned bb = __ballot_sync(0xFFFFFFFFu, open_bundle);
 		if (open_bundle) S.bq[__popc(bb & lt)] = make_int2(child, nchild);
 		__syncwarp();
 		if (nl >= 32) {
@@ -2174,7 +2222,7 @@ static int launch_walk_q(tvg_context *ctx, GroupParams p, const float *mass_f, c
 	static int nblk_dev[TVG_MAX_DEVICES] = { 0 };
 	TVG_CHECK(device_slot(ctx));
 	int &nblk = nblk_dev[ctx->device];
-	const size_t smem = (sizeof(WarpSmem) + (QUAD ? sizeof(QuadList) : 0)) * GW_WARPS;
+	const size_t smem = (sizeof(walk_smem<F, QUAD>) + (QUAD ? sizeof(QuadList) : 0)) * GW_WARPS;
 	TVG_CHECK(blocks_for(ctx, k_walk_group<MODE, TPL, F, QUAD, SPLIT>, smem, &nblk));
 	const int32_t *act = ctx->use_active ? ctx->active : nullptr, *gf = ctx->use_active ? ctx->group_first : nullptr;
 	F *a[7] = { (F *) ctx->f[FS_ACC0], (F *) ctx->f[FS_ACC1], (F *) ctx->f[FS_ACC2], (F *) ctx->f[FS_GACC0],

@@ -364,3 +364,27 @@ def test_split_groups(periodic, flags):
             d = np.abs(got["grav_acc"].astype(np.float64)[:, active] - acc[:, active])
             assert d.max() < 1e-4 * np.abs(acc).max()
             assert ctx.walk_counters()[0] == cost[active].astype(np.float64).sum()
+
+
+@pytest.mark.parametrize("vsize", [1, 2, 31, 32, 33, 64])
+@pytest.mark.parametrize("n", [1, 33, 3001])
+def test_bundle_runs(n, vsize):
+    """FP32 contexts read the opened bundles' particles as one run of chunks of
+    32, FP64 contexts bundle by bundle, with the same FP32 pair arithmetic. With
+    every node opened each target meets each particle once: equal counts, and
+    forces equal up to the order of FP32 sums of at most 256 entries (256 ulps
+    at most, 3e-5 of the largest component)."""
+    p = ics.random_box(n, box=100.0, seed=17, clumps=3 if n > 100 else 0)
+    out = []
+    for fsize in (4, 8):
+        for flags in (0, G.CFG_QUADRUPOLE):
+            with G.GravityContext(n, float_bytes=fsize, softening=p.softening, vector_size=vsize,
+                                  open_bh=1e-6, flags=flags) as ctx:
+                ctx.upload(np.asarray(p.pos, np.float32), np.asarray(p.mass, np.float32))
+                ctx.set_domain((0.0, 0.0, 0.0), 100.0)
+                ctx.force_step(form=G.FORM_GROUP, use_bh=True, parts=G.WALK_GRAVITY)
+                d = ctx.download(G.F_GRAV_ACC | G.F_COST)
+                out.append((d["grav_acc"].astype(np.float64), d["cost"].astype(np.float64)))
+    for acc, cost in out[:2]:
+        np.testing.assert_array_equal(cost, out[2][1])
+        assert np.abs(acc - out[2][0]).max() <= 3e-5 * np.abs(out[2][0]).max()
