@@ -21,9 +21,22 @@ int tvg_fail(tvg_context *ctx, int code, const char *fmt, ...)
 // Reads the device status word after a phase and maps it to an error code.
 int tvg_sync_status(tvg_context *ctx, const char *phase)
 {
+	TVG_CHECK(tvg_fetch_status(ctx));
+	TVG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+	return tvg_check_status(ctx, phase);
+}
+
+// The two halves of the above for callers that synchronise anyway: the copy of
+// the status word, enqueued, and the look at it once the stream has passed it.
+int tvg_fetch_status(tvg_context *ctx)
+{
 	TVG_CUDA(ctx, cudaMemcpyAsync(ctx->h_status, ctx->status, sizeof(int), cudaMemcpyDeviceToHost,
 	                              ctx->stream));
-	TVG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+	return TVG_OK;
+}
+
+int tvg_check_status(tvg_context *ctx, const char *phase)
+{
 	int st = *ctx->h_status;
 	if (!st) return TVG_OK;
 	TVG_CUDA(ctx, cudaMemsetAsync(ctx->status, 0, sizeof(int), ctx->stream));
@@ -111,6 +124,8 @@ extern "C" int tvg_init(int device, const tvg_config *cfg, tvg_context **out)
 	TVG_CHECK(dalloc(ctx, (void **) &ctx->status, sizeof(int)));
 	TVG_CUDA(ctx, cudaMemset(ctx->status, 0, sizeof(int)));
 	TVG_CUDA(ctx, cudaMallocHost((void **) &ctx->h_status, sizeof(int)));
+	TVG_CUDA(ctx, cudaMallocHost((void **) &ctx->h_dc, sizeof(tvg_devcount)));
+	TVG_CUDA(ctx, cudaMallocHost((void **) &ctx->h_counts, 3 * sizeof(double)));
 	TVG_CHECK(dalloc(ctx, (void **) &ctx->d_top, sizeof(tvg_topnode) * TVG_MAX_TOP));
 	TVG_CHECK(dalloc(ctx, (void **) &ctx->top_first, 4 * TVG_MAX_TOP));
 	TVG_CHECK(dalloc(ctx, (void **) &ctx->top_count, 4 * TVG_MAX_TOP));
@@ -146,20 +161,16 @@ extern "C" int tvg_init(int device, const tvg_config *cfg, tvg_context **out)
 	return TVG_OK;
 }
 
-// the device counts of the last step into the host mirrors
+// the device counts of the last step into the host mirrors, and the status word
 int tvg_read_counts(tvg_context *ctx)
 {
-	tvg_devcount h;
-	cudaStream_t s = ctx->stream;
-	TVG_CUDA(ctx, cudaMemcpyAsync(&h, ctx->dc, sizeof(h), cudaMemcpyDeviceToHost, s));
-	TVG_CUDA(ctx, cudaStreamSynchronize(s));
-	ctx->ntop = h.ntop;
-	ctx->nu = h.nu;
-	ctx->nnodes = h.nnodes;
-	if (ctx->ntop > 0)
-		TVG_CUDA(ctx, cudaMemcpyAsync(ctx->h_top, ctx->d_top, sizeof(tvg_topnode) * ctx->ntop,
-		                              cudaMemcpyDeviceToHost, s));
-	TVG_CUDA(ctx, cudaStreamSynchronize(s));
+	TVG_CUDA(ctx, cudaMemcpyAsync(ctx->h_dc, ctx->dc, sizeof(tvg_devcount), cudaMemcpyDeviceToHost,
+	                              ctx->stream));
+	TVG_CHECK(tvg_fetch_status(ctx));
+	TVG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+	ctx->ntop = ctx->h_dc->ntop;
+	ctx->nu = ctx->h_dc->nu;
+	ctx->nnodes = ctx->h_dc->nnodes;
 	return TVG_OK;
 }
 
@@ -187,6 +198,8 @@ extern "C" void tvg_finalize(tvg_context *ctx)
 	                 ctx->domain_state };
 	for (void *b : bufs) if (b) cudaFree(b);
 	if (ctx->h_status) cudaFreeHost(ctx->h_status);
+	if (ctx->h_dc) cudaFreeHost(ctx->h_dc);
+	if (ctx->h_counts) cudaFreeHost(ctx->h_counts);
 	for (int i = 0; i < 16; i++) if (ctx->ev[i]) cudaEventDestroy(ctx->ev[i]);
 	for (int i = 0; i < 3; i++) if (ctx->xev[i]) cudaEventDestroy(ctx->xev[i]);
 	if (ctx->copy_stream) cudaStreamDestroy(ctx->copy_stream);
@@ -352,6 +365,7 @@ extern "C" int tvg_top_nodes(tvg_context *ctx, int32_t *ntop)
 		return tvg_fail(ctx, TVG_E_STATE, "top_nodes: particles not sorted by standard keys");
 	TVG_CUDA(ctx, cudaSetDevice(ctx->device));
 	TVG_CHECK(tvg_impl_top_nodes(ctx));
+	TVG_CHECK(tvg_read_counts(ctx));
 	ctx->have_top = true;
 	if (ntop) *ntop = ctx->ntop;
 	return TVG_OK;

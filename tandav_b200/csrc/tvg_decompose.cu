@@ -370,8 +370,7 @@ int tvg_impl_top_nodes_balanced(tvg_context *ctx)
 	}
 	const int rc = ctx->cfg.float_bytes == 4 ? decompose_typed<float>(ctx) : decompose_typed<double>(ctx);
 	if (rc != TVG_OK) return rc;
-	TVG_CHECK(tvg_impl_top_of(ctx));
-	return tvg_read_counts(ctx);
+	return tvg_impl_top_of(ctx);
 }
 
 extern "C" int tvg_set_domain_decomposition(tvg_context *ctx, int32_t ntask, double part_alloc_factor,

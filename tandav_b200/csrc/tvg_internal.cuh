@@ -147,11 +147,12 @@ struct tvg_context {
 	size_t scan_tmp_bytes = 0;
 	int *status = nullptr;             // device status word
 	int *h_status = nullptr;           // pinned mirror
+	tvg_devcount *h_dc = nullptr;      // pinned mirror of dc
+	double *h_counts = nullptr;        // pinned mirror of the group walk's counters
 
 	// top nodes
 	int32_t ntop = 0;
 	tvg_topnode *d_top = nullptr;
-	tvg_topnode h_top[TVG_MAX_TOP];
 	int32_t *top_first = nullptr;      // [64] first particle of level-2 cell c
 	int32_t *top_count = nullptr;      // [64]
 	int32_t *top_of = nullptr;         // top node of every particle (cap)
@@ -267,6 +268,8 @@ struct tvg_context {
 
 int tvg_fail(tvg_context *ctx, int code, const char *fmt, ...);
 int tvg_sync_status(tvg_context *ctx, const char *phase);
+int tvg_fetch_status(tvg_context *ctx);
+int tvg_check_status(tvg_context *ctx, const char *phase);
 int tvg_device_scan_i32(tvg_context *ctx, const int32_t *in, int32_t *out, int64_t n,
                         int64_t *total);
 // as tvg_device_scan_i32, the total written to device memory (no host read)

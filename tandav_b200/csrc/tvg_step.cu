@@ -80,9 +80,10 @@ extern "C" int tvg_force_step(tvg_context *ctx, int32_t form, int32_t use_bh, ui
 		return tvg_fail(ctx, TVG_E_STATE, "force_step: domain not set");
 	TVG_CUDA(ctx, cudaSetDevice(ctx->device));
 	TVG_CHECK(force_phases(ctx, form, use_bh, parts, ewald_kind, nullptr));
-	TVG_CUDA(ctx, cudaEventSynchronize(ctx->ev[13]));
+	TVG_CHECK(tvg_fetch_status(ctx));
+	TVG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
 	TVG_CHECK(force_times(ctx));
-	return tvg_sync_status(ctx, "force_step");
+	return tvg_check_status(ctx, "force_step");
 }
 
 // Fields that the steps after the sort never write: a force step from host
@@ -154,10 +155,11 @@ extern "C" int tvg_force_step_host(tvg_context *ctx, int64_t n, const tvg_partic
 		TVG_CUDA(ctx, cudaMemcpyAsync(tvg_host_field(out, f), ctx->f[f], tvg_field_bytes(ctx, f) * n,
 		                              cudaMemcpyDeviceToHost, (bit & kWrittenByStep) ? s : cs));
 	}
+	TVG_CHECK(tvg_fetch_status(ctx));
 	TVG_CUDA(ctx, cudaStreamSynchronize(cs));
 	TVG_CUDA(ctx, cudaStreamSynchronize(s));
 	TVG_CHECK(force_times(ctx));
-	return tvg_sync_status(ctx, "force_step_host");
+	return tvg_check_status(ctx, "force_step_host");
 }
 
 // The launches of Compute_Acceleration (accel.c:15-71) after the single-rank
@@ -256,8 +258,10 @@ extern "C" int tvg_compute_acceleration(tvg_context *ctx, int32_t form, uint32_t
 		ctx->have_ewald = true;
 	}
 	TVG_CHECK(accel_phases(ctx, form, parts, ewald_kind, prepare));
+	TVG_CHECK(tvg_fetch_status(ctx));
+	TVG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
 	TVG_CHECK(accel_times(ctx));
-	return tvg_sync_status(ctx, "compute_acceleration");
+	return tvg_check_status(ctx, "compute_acceleration");
 }
 
 // ------------------------------------------------------------- CUDA graph
@@ -451,7 +455,7 @@ extern "C" int tvg_step_graph(tvg_context *ctx, uint32_t parts, int32_t ewald_ki
 	set_ptrs(ctx, e->end);
 	ctx->keys_std = ctx->sorted = ctx->have_top = ctx->have_tree = ctx->have_walktree = true;
 	ctx->use_active = ctx->have_timeline;
-	// host mirrors of the step's counts and times (one synchronisation)
+	// host mirrors of the step's counts and times
 	TVG_CHECK(accel_times(ctx));
 	TVG_CHECK(tvg_walk_group_results(ctx));
 	TVG_CHECK(tvg_read_counts(ctx));
@@ -461,7 +465,7 @@ extern "C" int tvg_step_graph(tvg_context *ctx, uint32_t parts, int32_t ewald_ki
 		ctx->n_active = na;
 		ctx->tl.state.n_active = na;
 	}
-	return tvg_sync_status(ctx, "step_graph");
+	return tvg_check_status(ctx, "step_graph");    // as tvg_read_counts fetched it
 }
 
 extern "C" int tvg_step_graph_reset(tvg_context *ctx)

@@ -148,9 +148,7 @@ int tvg_impl_top_nodes(tvg_context *ctx)
 		                                   ctx->origin[0], ctx->origin[1], ctx->origin[2], ctx->dsize,
 		                                   ctx->d_top, ctx->top_count, ctx->dc);
 	TVG_CUDA(ctx, cudaGetLastError());
-	TVG_CHECK(tvg_impl_top_of(ctx));
-	if (ctx->capturing) return TVG_OK;
-	return tvg_read_counts(ctx);
+	return tvg_impl_top_of(ctx);
 }
 
 // ----------------------------------------------------- build: levels
@@ -869,7 +867,10 @@ static int build_typed(tvg_context *ctx, uint32_t flags)
 	                                                          ctx->top_of, vsize, ctx->lvl, ctx->ncnt,
 	                                                          ctx->lvl_min64, ctx->status);
 	TVG_CUDA(ctx, cudaGetLastError());
-	if (!ctx->capturing) TVG_CHECK(tvg_sync_status(ctx, "tree_build(levels)"));
+	if (!ctx->capturing) {                  // the top node count comes with it
+		TVG_CHECK(tvg_read_counts(ctx));
+		TVG_CHECK(tvg_check_status(ctx, "tree_build(levels)"));
+	}
 	TVG_CHECK(tvg_device_scan_i32_dev(ctx, ctx->ncnt, ctx->ncnt, n + 1, &dc->nu));
 	TVG_CUDA(ctx, cudaMemsetAsync(ctx->u_diff, 0, 4 * (ucap + 1), s));
 	k_nodes<<<TVG_CNT(ctx, tvg_blocks(n, 128)), 128, 0, s>>>(n, ctx->lvl, ctx->lvl_min64, ctx->ncnt,
@@ -926,7 +927,7 @@ static int build_typed(tvg_context *ctx, uint32_t flags)
 	if (ctx->nnodes > tcap)
 		return tvg_fail(ctx, TVG_E_TREE_FULL, "tree_build: %lld nodes > capacity %lld",
 		                (long long) ctx->nnodes, (long long) tcap);
-	return tvg_sync_status(ctx, "tree_build");
+	return tvg_check_status(ctx, "tree_build");
 }
 
 int tvg_impl_tree_build(tvg_context *ctx, uint32_t flags)

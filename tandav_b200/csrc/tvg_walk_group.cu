@@ -2432,17 +2432,14 @@ static int walk_group_typed(tvg_context *ctx, int use_bh, uint32_t parts, int ew
 // (synchronises)
 int tvg_walk_group_results(tvg_context *ctx)
 {
-	TVG_CUDA(ctx, cudaEventSynchronize(ctx->ev[2]));
+	TVG_CUDA(ctx, cudaMemcpyAsync(ctx->h_counts, ctx->counters, 24, cudaMemcpyDeviceToHost, ctx->stream));
+	TVG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
 	float ms = 0, ms_e = 0;
 	TVG_CUDA(ctx, cudaEventElapsedTime(&ms, ctx->ev[0], ctx->ev[1]));
 	TVG_CUDA(ctx, cudaEventElapsedTime(&ms_e, ctx->ev[1], ctx->ev[2]));
 	ctx->phase_ms[4] = ms;
 	ctx->phase_ms[5] = ms_e;
-	double c[3];
-	TVG_CUDA(ctx, cudaMemcpy(c, ctx->counters, 24, cudaMemcpyDeviceToHost));
-	ctx->last_counts[0] = c[0];
-	ctx->last_counts[1] = c[1];
-	ctx->last_counts[2] = c[2];
+	for (int i = 0; i < 3; i++) ctx->last_counts[i] = ctx->h_counts[i];
 	return TVG_OK;
 }
 
