@@ -115,9 +115,8 @@ extern "C" int tvg_init(int device, const tvg_config *cfg, tvg_context **out)
 	TVG_CHECK(dalloc(ctx, (void **) &ctx->key_tmp, 8 * cap));
 	TVG_CHECK(dalloc(ctx, (void **) &ctx->perm, 4 * cap));
 	TVG_CHECK(dalloc(ctx, (void **) &ctx->perm_tmp, 4 * cap));
-	const int64_t ntiles = (cap + 4095) / 4096;
-	TVG_CHECK(dalloc(ctx, (void **) &ctx->sort_hist, 4 * 256 * (ntiles + 1)));
-	TVG_CHECK(dalloc(ctx, (void **) &ctx->sort_off, 4 * 256 * (ntiles + 1)));
+	TVG_CHECK(dalloc(ctx, (void **) &ctx->sort_hist, 4 * tvg_sort_state_words(cap)));
+	TVG_CHECK(dalloc(ctx, (void **) &ctx->sort_off, 4 * tvg_sort_state_words(cap)));
 	TVG_CHECK(dalloc(ctx, (void **) &ctx->digit_count, 4 * 8 * 256));
 	ctx->scan_tmp_bytes = 8 * ((cap * 3) / 512 + 4096);
 	TVG_CHECK(dalloc(ctx, &ctx->scan_tmp, ctx->scan_tmp_bytes));

@@ -17,7 +17,7 @@
 // keeps it. The three axes go together, and the last block of a pass picks the
 // buckets on the device, so a pass is one launch and the host waits once, for
 // the result (with a launch and a wait per byte and axis: 0.30 ms for 200,000
-// particles in FP32; so: 0.07 ms).
+// particles in FP32; so: 0.05 ms).
 // Roofline: HBM bound, one read of the positions per byte of the Float (4 or 8
 // passes) plus one for the distance.
 #include <stddef.h>
@@ -64,6 +64,12 @@ struct DomainState {
 };
 
 #define DS_THREADS 256
+// Few particles a thread, loaded together: a pass is as long as one thread's chain.
+// 400,000 particles in FP64, whole search with 16 one by one / 8 / 4: 165 / 95 / 94
+// us (200,000 in FP32: 75 / 64 / 54; 4M in FP64 with one block a SM 437, two 264,
+// four 203).
+#define DS_IPT 4
+#define DS_BLOCKS 4
 
 // One byte of the three selections: counts the byte at `shift` of the ordered
 // values of particles 1 .. n-1 that have the prefix; the last block picks the
@@ -83,11 +89,34 @@ k_select(int64_t n, const F *__restrict__ x, const F *__restrict__ y, const F *_
 	U prefix[3];
 #pragma unroll
 	for (int d = 0; d < 3; d++) prefix[d] = (U) st->prefix[d];
-	for (int64_t i = 1 + blockIdx.x * (int64_t) DS_THREADS + threadIdx.x; i < n; i += (int64_t) gridDim.x * DS_THREADS) {
+	const unsigned lane_bit = 1u << (threadIdx.x & 31);
+	for (int64_t base = 1 + blockIdx.x * (int64_t) (DS_IPT * DS_THREADS); base < n;
+	     base += (int64_t) gridDim.x * (DS_IPT * DS_THREADS)) {
+		F v[3][DS_IPT];
 #pragma unroll
-		for (int d = 0; d < 3; d++) {
-			const U u = ordered(X[d][i]);
-			if ((u & mask) == prefix[d]) atomicAdd(&h[d][(u >> shift) & 0xFF], 1u);
+		for (int r = 0; r < DS_IPT; r++) {
+			const int64_t i = base + r * DS_THREADS + threadIdx.x;
+#pragma unroll
+			for (int d = 0; d < 3; d++) v[d][r] = i < n ? X[d][i] : (F) 0;
+		}
+#pragma unroll
+		for (int r = 0; r < DS_IPT; r++) {
+			const bool have = base + r * DS_THREADS + threadIdx.x < n;
+#pragma unroll
+			for (int d = 0; d < 3; d++) {
+				const U u = ordered(v[d][r]);
+				const bool in = have && (u & mask) == prefix[d];
+				const unsigned m = __ballot_sync(0xFFFFFFFFu, in);
+				if (m == 0) continue;
+				// the lanes with the first lane's byte count once, together:
+				// the top bytes are nearly all the same
+				const uint32_t byte = (uint32_t) (u >> shift) & 0xFF;
+				const int first = __ffs(m) - 1;
+				const uint32_t lead = __shfl_sync(0xFFFFFFFFu, byte, first);
+				const unsigned same = __ballot_sync(0xFFFFFFFFu, in && byte == lead);
+				if (lane_bit == 1u << first) atomicAdd(&h[d][lead], (uint32_t) __popc(same));
+				else if (in && byte != lead) atomicAdd(&h[d][byte], 1u);
+			}
 		}
 	}
 	__syncthreads();
@@ -177,8 +206,8 @@ int find_domain_typed(tvg_context *ctx, double origin[3], double *size)
 	const F *x = (const F *) ctx->f[FS_POS0], *y = (const F *) ctx->f[FS_POS1], *z = (const F *) ctx->f[FS_POS2];
 	if (!ctx->domain_state) TVG_CUDA(ctx, cudaMalloc(&ctx->domain_state, sizeof(DomainState)));
 	DomainState *st = (DomainState *) ctx->domain_state;
-	// a block per 4096 particles, up to eight a SM
-	const unsigned grid = tvg_blocks(n, 16 * DS_THREADS) < 148u * 8u ? tvg_blocks(n, 16 * DS_THREADS) : 148u * 8u;
+	// up to DS_BLOCKS blocks a SM
+	const unsigned need = tvg_blocks(n, DS_IPT * DS_THREADS), grid = need < 148u * DS_BLOCKS ? need : 148u * DS_BLOCKS;
 	k_select_start<F><<<TVG_CNT(ctx, 1), DS_THREADS, 0, s>>>(n, x, y, z, st);
 	if (n > 1)
 		for (int pass = 0; pass < (int) sizeof(F); pass++)

@@ -296,6 +296,7 @@ int tvg_impl_tree_drift(tvg_context *ctx, double dt);
 
 // phase implementations (one translation unit each)
 int tvg_impl_keys(tvg_context *ctx, bool reversed);
+size_t tvg_sort_state_words(int64_t n);
 int tvg_impl_sort(tvg_context *ctx, uint32_t *perm_out);
 int tvg_impl_top_nodes(tvg_context *ctx);
 // Domain_Decomposition's cost-driven top nodes for NTask > 1 (tvg_decompose.cu)

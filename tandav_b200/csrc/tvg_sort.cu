@@ -5,10 +5,11 @@
 //  1. LSD radix sort of (key_hi, index) on the 64-bit high key word: 8-bit
 //     digits, one kernel per digit (k_radix_pass). All eight digit histograms are
 //     counted in one pass over the keys beforehand; a pass takes tiles of 4096 keys
-//     in the order of a device counter, ranks a tile's keys stably with warp
-//     matches, finds the tile's place among the equal digits of earlier tiles by
-//     looking back over their published counts, and writes through a
-//     shared-memory staging sort (coalesced runs per digit). A digit that is
+//     (few keys: 1024) in the order of a device counter, ranks a tile's keys
+//     stably with warp ballots, finds the tile's place among the equal digits of
+//     earlier tiles by looking back over their published counts, four tiles at a
+//     time, and writes through a shared-memory staging sort (coalesced runs per
+//     digit). A digit that is
 //     equal for every key (decided on the device) is not ranked: its pass copies
 //     the keys through, so the number of passes, and with it the buffer a step
 //     ends in, never depends on the data. Up to one tile of keys is sorted by one
@@ -24,16 +25,17 @@
 // unspecified order).
 // Roofline: HBM bound; per pass 12 B read + 12 B write per key. Histogram, scan
 // and scatter kernels per digit (three to five launches, 20 B read) took, with
-// the gather of the fields, 4.65 ms for 16.7M particles, 0.47 ms for 400,000 and
-// 0.28 ms for 3001; this 2.80, 0.22 and 0.06 ms (a pass over 16.7M keys 243 us, 1.7
-// TB/s, bound by the warp matches of the ranking).
+// the gather of the fields, 4.65 ms for 16.7M particles, 0.47 ms for 400,000,
+// 0.27 ms for 32,768 and 0.28 ms for 3001; this 2.44, 0.20, 0.10 and 0.06 ms. A
+// pass over many keys waits on shared memory (ranking and staging, 16 keys a
+// thread) at the 32 warps an SM holds (4M keys: 61 us, 0.9 TB/s of DRAM traffic,
+// as the L2 holds both buffers).
 #include <mutex>
 
 #include "tvg_internal.cuh"
 
 #define RS_THREADS 256
-#define RS_IPT 16
-#define RS_TILE (RS_THREADS * RS_IPT)
+#define RS_TILE (RS_THREADS * 16)
 #define RS_WARPS (RS_THREADS / 32)
 
 // global histogram of all 8 digits of key_hi (to skip constant digits)
@@ -95,12 +97,27 @@ __device__ __forceinline__ uint32_t scan256(uint32_t v, uint32_t *s_warp)
 	return base + inc - v;
 }
 
-// Ranks a tile's digits: a warp holds RS_IPT x 32 consecutive keys, key r of
+// lanes that hold the digit d of this one (256: none), by a ballot per bit (with
+// a match instruction the sort of 16.7M keys took 2.80 ms instead of 2.48)
+__device__ __forceinline__ unsigned equal_digits(uint32_t d)
+{
+	unsigned peers = __ballot_sync(0xFFFFFFFFu, d < 256);
+#pragma unroll
+	for (int b = 0; b < 8; b++) {
+		const bool one = (d >> b) & 1;
+		const unsigned m = __ballot_sync(0xFFFFFFFFu, one);
+		peers &= one ? m : ~m;
+	}
+	return peers;
+}
+
+// Ranks a tile's digits: a warp holds IPT x 32 consecutive keys, key r of
 // lane l at r * 32 + l; whist[w][d] counts digit d of warp w as it goes, so that
 // rank[r] is the key's place among the equal digits of its warp. Returns with
 // whist holding, per digit, the offset of each warp among the tile's equal
 // digits, and in thread t the tile's count of digit t.
-__device__ __forceinline__ uint32_t rank_tile(const uint32_t (&d)[RS_IPT], uint32_t (&rank)[RS_IPT],
+template <int IPT>
+__device__ __forceinline__ uint32_t rank_tile(const uint32_t (&d)[IPT], uint32_t (&rank)[IPT],
                                               uint32_t (*whist)[256])
 {
 	const int t = threadIdx.x, lane = t & 31, w = t >> 5;
@@ -109,8 +126,8 @@ __device__ __forceinline__ uint32_t rank_tile(const uint32_t (&d)[RS_IPT], uint3
 	for (int k = 0; k < RS_WARPS; k++) whist[k][t] = 0;
 	__syncthreads();
 #pragma unroll
-	for (int r = 0; r < RS_IPT; r++) {
-		const unsigned peers = __match_any_sync(0xFFFFFFFFu, d[r]);
+	for (int r = 0; r < IPT; r++) {
+		const unsigned peers = equal_digits(d[r]);
 		const int leader = __ffs(peers) - 1;
 		uint32_t old = 0;
 		if (lane == leader && d[r] < 256) {
@@ -140,24 +157,28 @@ __device__ __forceinline__ uint32_t rank_tile(const uint32_t (&d)[RS_IPT], uint3
 // polls of one predecessor's state before the pass gives up (about a second);
 // tiles are taken in order, so the predecessors run or have run
 #define RS_SPIN (1 << 21)
+// predecessors looked at together
+#define RS_LOOK 4
 
 // One digit's pass. state: ntiles x 256 words of this pass, zero at its start;
 // next: those of the next pass, zeroed here. vin null: the values are the
 // indices.
-__global__ void __launch_bounds__(RS_THREADS, 3)
+template <int IPT>
+__global__ void __launch_bounds__(RS_THREADS, IPT > 4 ? 4 : 6)
 k_radix_pass(int64_t n, int shift, const uint64_t *__restrict__ kin, const uint32_t *__restrict__ vin,
              uint64_t *__restrict__ kout, uint32_t *__restrict__ vout, const uint32_t *__restrict__ offsets,
              volatile uint32_t *state, uint32_t *__restrict__ next, uint32_t *tiles,
              const int32_t *__restrict__ skip, int *status)
 {
-	__shared__ __align__(16) uint64_t skey[RS_TILE];     // keys, then values
+	constexpr int TILE = RS_THREADS * IPT;
+	__shared__ __align__(16) uint64_t skey[TILE];     // keys, then values
 	__shared__ uint32_t whist[RS_WARPS][256];
 	__shared__ uint32_t dstart[256], gstart[256], s_warp[RS_WARPS], s_tile;
 	const int t = threadIdx.x, lane = t & 31, w = t >> 5;
 	next[(int64_t) blockIdx.x * 256 + t] = 0;
 	if (skip[shift >> 3]) {                              // constant digit: the order stays
-		const int64_t b0 = (int64_t) blockIdx.x * RS_TILE;
-		const int c0 = (int) min((int64_t) RS_TILE, n - b0);
+		const int64_t b0 = (int64_t) blockIdx.x * TILE;
+		const int c0 = (int) min((int64_t) TILE, n - b0);
 		for (int p = t; p < c0; p += RS_THREADS) {
 			kout[b0 + p] = kin[b0 + p];
 			vout[b0 + p] = vin ? vin[b0 + p] : (uint32_t) (b0 + p);
@@ -166,13 +187,13 @@ k_radix_pass(int64_t n, int shift, const uint64_t *__restrict__ kin, const uint3
 	}
 	if (t == 0) s_tile = atomicAdd(&tiles[shift >> 3], 1u);
 	__syncthreads();
-	const int64_t tile = s_tile, base = tile * RS_TILE;
-	const int cnt = (int) min((int64_t) RS_TILE, n - base);
-	uint64_t k[RS_IPT];
-	uint32_t d[RS_IPT], rank[RS_IPT];
-	const int first = w * (32 * RS_IPT) + lane;
+	const int64_t tile = s_tile, base = tile * TILE;
+	const int cnt = (int) min((int64_t) TILE, n - base);
+	uint64_t k[IPT];
+	uint32_t d[IPT], rank[IPT];
+	const int first = w * (32 * IPT) + lane;
 #pragma unroll
-	for (int r = 0; r < RS_IPT; r++) {
+	for (int r = 0; r < IPT; r++) {
 		const int idx = first + 32 * r;
 		k[r] = idx < cnt ? kin[base + idx] : 0;
 		d[r] = idx < cnt ? (uint32_t) (k[r] >> shift) & 0xFF : 256u;
@@ -182,33 +203,41 @@ k_radix_pass(int64_t n, int shift, const uint64_t *__restrict__ kin, const uint3
 	dstart[t] = scan256(count, s_warp);
 	// look back: thread t sums digit t's counts of the earlier tiles
 	uint32_t before = 0;
-	for (int64_t q = tile - 1; q >= 0; q--) {
-		uint32_t v = state[q * 256 + t];
-		for (int spin = 0; v == 0; spin++) {
-			if (spin > RS_SPIN) {
-				atomicOr(status, TVG_ST_TIMEOUT);
-				v = RS_TOTAL;
-				break;
+	for (int64_t q = tile - 1; q >= 0; q -= RS_LOOK) {
+		uint32_t v[RS_LOOK];
+#pragma unroll
+		for (int j = 0; j < RS_LOOK; j++) v[j] = q - j >= 0 ? state[(q - j) * 256 + t] : RS_TOTAL;
+		bool done = false;
+#pragma unroll
+		for (int j = 0; j < RS_LOOK; j++) {
+			if (done) continue;
+			for (int spin = 0; v[j] == 0; spin++) {
+				if (spin > RS_SPIN) {
+					atomicOr(status, TVG_ST_TIMEOUT);
+					v[j] = RS_TOTAL;
+					break;
+				}
+				v[j] = state[(q - j) * 256 + t];
 			}
-			v = state[q * 256 + t];
+			before += v[j] & RS_VALUE;
+			done = v[j] & RS_TOTAL;
 		}
-		before += v & RS_VALUE;
-		if (v & RS_TOTAL) break;
+		if (done) break;
 	}
 	if (tile > 0) state[tile * 256 + t] = RS_TOTAL | ((before + count) & RS_VALUE);
 	gstart[t] = offsets[t] + before - dstart[t];
 	__syncthreads();
 #pragma unroll
-	for (int r = 0; r < RS_IPT; r++) {
+	for (int r = 0; r < IPT; r++) {
 		if (d[r] < 256) {
 			rank[r] += dstart[d[r]] + whist[w][d[r]];
 			skey[rank[r]] = k[r];
 		}
 	}
 	__syncthreads();
-	uint32_t dest[RS_IPT];
+	uint32_t dest[IPT];
 #pragma unroll
-	for (int r = 0; r < RS_IPT; r++) {
+	for (int r = 0; r < IPT; r++) {
 		const int p = t + RS_THREADS * r;
 		dest[r] = 0xFFFFFFFFu;
 		if (p < cnt) {
@@ -220,13 +249,13 @@ k_radix_pass(int64_t n, int shift, const uint64_t *__restrict__ kin, const uint3
 	__syncthreads();
 	uint32_t *sval = (uint32_t *) skey;
 #pragma unroll
-	for (int r = 0; r < RS_IPT; r++) {
+	for (int r = 0; r < IPT; r++) {
 		const int idx = first + 32 * r;
 		if (idx < cnt) sval[rank[r]] = vin ? vin[base + idx] : (uint32_t) (base + idx);
 	}
 	__syncthreads();
 #pragma unroll
-	for (int r = 0; r < RS_IPT; r++) {
+	for (int r = 0; r < IPT; r++) {
 		const int p = t + RS_THREADS * r;
 		if (dest[r] < n) vout[dest[r]] = sval[p];
 	}
@@ -237,48 +266,49 @@ k_radix_pass(int64_t n, int shift, const uint64_t *__restrict__ kin, const uint3
 __global__ void __launch_bounds__(RS_THREADS)
 k_sort_tile(int n, uint64_t *__restrict__ key, uint32_t *__restrict__ perm)
 {
+	constexpr int IPT = RS_TILE / RS_THREADS;
 	__shared__ __align__(16) uint64_t skey[RS_TILE];
 	__shared__ uint32_t whist[RS_WARPS][256];
 	__shared__ uint32_t dstart[256], s_warp[RS_WARPS];
 	uint32_t *sval = (uint32_t *) skey;
-	const int t = threadIdx.x, lane = t & 31, w = t >> 5, first = w * (32 * RS_IPT) + lane;
-	uint64_t k[RS_IPT];
-	uint32_t v[RS_IPT], d[RS_IPT], rank[RS_IPT];
+	const int t = threadIdx.x, lane = t & 31, w = t >> 5, first = w * (32 * IPT) + lane;
+	uint64_t k[IPT];
+	uint32_t v[IPT], d[IPT], rank[IPT];
 #pragma unroll
-	for (int r = 0; r < RS_IPT; r++) {
+	for (int r = 0; r < IPT; r++) {
 		const int idx = first + 32 * r;
 		k[r] = idx < n ? key[idx] : 0;
 		v[r] = (uint32_t) idx;
 	}
 	for (int shift = 0; shift < 64; shift += 8) {
 #pragma unroll
-		for (int r = 0; r < RS_IPT; r++) d[r] = first + 32 * r < n ? (uint32_t) (k[r] >> shift) & 0xFF : 256u;
+		for (int r = 0; r < IPT; r++) d[r] = first + 32 * r < n ? (uint32_t) (k[r] >> shift) & 0xFF : 256u;
 		const uint32_t count = rank_tile(d, rank, whist);
 		if (__syncthreads_or(count == (uint32_t) n)) continue;
 		dstart[t] = scan256(count, s_warp);
 		__syncthreads();
 #pragma unroll
-		for (int r = 0; r < RS_IPT; r++)
+		for (int r = 0; r < IPT; r++)
 			if (d[r] < 256) {
 				rank[r] += dstart[d[r]] + whist[w][d[r]];
 				skey[rank[r]] = k[r];
 			}
 		__syncthreads();
 #pragma unroll
-		for (int r = 0; r < RS_IPT; r++)
+		for (int r = 0; r < IPT; r++)
 			if (d[r] < 256) k[r] = skey[first + 32 * r];
 		__syncthreads();
 #pragma unroll
-		for (int r = 0; r < RS_IPT; r++)
+		for (int r = 0; r < IPT; r++)
 			if (d[r] < 256) sval[rank[r]] = v[r];
 		__syncthreads();
 #pragma unroll
-		for (int r = 0; r < RS_IPT; r++)
+		for (int r = 0; r < IPT; r++)
 			if (d[r] < 256) v[r] = sval[first + 32 * r];
 		__syncthreads();
 	}
 #pragma unroll
-	for (int r = 0; r < RS_IPT; r++) {
+	for (int r = 0; r < IPT; r++) {
 		const int idx = first + 32 * r;
 		if (idx < n) {
 			key[idx] = k[r];
@@ -374,15 +404,17 @@ __global__ void k_gather_fields(int64_t n, const uint32_t *__restrict__ perm, Ga
 // The eight passes over n keys: kin / kout and the two value buffers alternate,
 // and after the eighth pass the result is back in kin and vb. count: 8 x 256
 // words; st[2]: tile states; tiles: 8 words.
+template <int IPT>
 static cudaError_t radix_passes(cudaStream_t s, int64_t n, const uint64_t *key, uint64_t *kin, uint64_t *kout,
                                 uint32_t *va, uint32_t *vb, uint32_t *count, int32_t *skip,
                                 uint32_t *const st[2], uint32_t *tiles, int *status)
 {
-	const int64_t ntiles = (n + RS_TILE - 1) / RS_TILE;
+	constexpr int TILE = RS_THREADS * IPT;
+	const int64_t ntiles = (n + TILE - 1) / TILE, ncount = (n + RS_TILE - 1) / RS_TILE;
 	cudaError_t e = cudaMemsetAsync(count, 0, 4 * 8 * 256, s);
 	if (e == cudaSuccess) e = cudaMemsetAsync(st[0], 0, 4 * 256 * (size_t) ntiles, s);
 	if (e != cudaSuccess) return e;
-	const unsigned nb = (unsigned) (ntiles < 296 ? ntiles : 296);
+	const unsigned nb = (unsigned) (ncount < 296 ? ncount : 296);
 	k_digit_counts<<<nb, 512, 0, s>>>(n, key, count);
 	k_digit_offsets<<<8, 256, 0, s>>>(n, count, skip, tiles);
 	const uint32_t *vin = nullptr;
@@ -390,7 +422,7 @@ static cudaError_t radix_passes(cudaStream_t s, int64_t n, const uint64_t *key, 
 	for (int d = 0; d < 8; d++) {
 		uint64_t *out = d & 1 ? kin : kout;
 		uint32_t *vout = d & 1 ? vb : va;
-		k_radix_pass<<<(unsigned) ntiles, RS_THREADS, 0, s>>>(n, 8 * d, in, vin, out, vout, count + 256 * d,
+		k_radix_pass<IPT><<<(unsigned) ntiles, RS_THREADS, 0, s>>>(n, 8 * d, in, vin, out, vout, count + 256 * d,
 		                                                      st[d & 1], st[(d & 1) ^ 1], tiles, skip, status);
 		in = out;
 		vin = vout;
@@ -398,6 +430,20 @@ static cudaError_t radix_passes(cudaStream_t s, int64_t n, const uint64_t *key, 
 	return cudaGetLastError();
 }
 #define RS_LAUNCHES 10
+
+// Up to this many keys the tiles are of 1024 keys instead of 4096: a pass is then
+// one wave of blocks, as long as one block's chain of loads, ranks and look-back.
+// Sort and gather, tiles of 4096 / 1024: 5000 keys 156 / 109 us, 32768 172 / 126,
+// 200,000 212 / 176, 400,000 224 / 214, 700,000 288 / 291, 1,000,000 333 / 360.
+#define RS_SMALL_KEYS (1 << 19)
+
+// words of one pass's tile states for up to n keys
+size_t tvg_sort_state_words(int64_t n)
+{
+	const int64_t large = (n + RS_TILE - 1) / RS_TILE, few = n < RS_SMALL_KEYS ? n : RS_SMALL_KEYS;
+	const int64_t small = (few + RS_THREADS * 4 - 1) / (RS_THREADS * 4);
+	return 256 * (size_t) ((large > small ? large : small) + 1);
+}
 
 int tvg_impl_sort(tvg_context *ctx, uint32_t *perm_out)
 {
@@ -412,8 +458,9 @@ int tvg_impl_sort(tvg_context *ctx, uint32_t *perm_out)
 	} else {
 		uint32_t *const st[2] = { ctx->sort_hist, ctx->sort_off };
 		ctx->launches += RS_LAUNCHES;
-		TVG_CUDA(ctx, radix_passes(s, n, kin, kin, ctx->key_tmp, vout, vin, ctx->digit_count, ctx->dc->sort_skip,
-		                           st, ctx->dc->sort_tiles, ctx->status));
+		const auto passes = n <= RS_SMALL_KEYS ? radix_passes<4> : radix_passes<16>;
+		TVG_CUDA(ctx, passes(s, n, kin, kin, ctx->key_tmp, vout, vin, ctx->digit_count, ctx->dc->sort_skip, st,
+		                     ctx->dc->sort_tiles, ctx->status));
 	}
 	// runs of equal high words by the low words, into the other buffer
 	k_tie_rank<<<TVG_CNT(ctx, tvg_blocks(n, 256)), 256, 0, s>>>(n, kin, ctx->key_lo, vin, vout);
@@ -504,7 +551,7 @@ extern "C" int tvg_sort_keys_noalloc(const uint64_t *key_hi, const uint64_t *key
 	cudaError_t e = cudaMemsetAsync(&S->status, 0, sizeof(int), s);
 	if (e == cudaSuccess) {
 		uint32_t *const st[2] = { S->state[0], S->state[1] };
-		e = radix_passes(s, n, key_hi, S->key[0], S->key[1], S->idx[0], S->idx[1], S->count, S->skip, st, S->tiles,
+		e = radix_passes<16>(s, n, key_hi, S->key[0], S->key[1], S->idx[0], S->idx[1], S->count, S->skip, st, S->tiles,
 		                 &S->status);
 	}
 	if (e == cudaSuccess) {

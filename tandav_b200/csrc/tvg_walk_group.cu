@@ -1134,7 +1134,8 @@ k_walk_group(GroupParams p, const int32_t *__restrict__ active, const int32_t *_
 	if (QUAD && lane == 0 && qcnt_acc != 0) atomicAdd(counter + 2, qcnt_acc);
 }
 
-// the parts' sums of each target, in order
+// the parts' sums of each target, in order, eight in flight (few groups, so few
+// blocks, each as long as a thread's chain of loads)
 template <typename F>
 __global__ void __launch_bounds__(256)
 k_walk_sum(GroupParams p, const int32_t *__restrict__ active, const int32_t *__restrict__ gfirst,
@@ -1153,6 +1154,7 @@ k_walk_sum(GroupParams p, const int32_t *__restrict__ active, const int32_t *__r
 		const int64_t last = gfirst ? (int64_t) gfirst[g + 1] : min(first + p.gsize, p.n);
 		if (first + slot >= last) continue;
 		PartSum s = { { 0, 0, 0 }, 0, 0 };
+#pragma unroll 8
 		for (int q = 0; q < parts; q++) {
 			const PartSum v = sums[(g * parts + q) * p.gsize + slot];
 			s.a[0] += v.a[0];
@@ -2046,8 +2048,10 @@ k_ewald_sum(GroupParams p, const int32_t *__restrict__ active, const int32_t *__
 		group_setup<TPL>(p, ix, iy, iz, last_acc, active, first, (int) (last - first), t, g);
 		if (fmaxf(g.hx, fmaxf(g.hy, g.hz)) >= p.taylor_h) continue;      // k_ewald_wide
 		double mine = 0, q[EW_SUMS];
-		if (lane < EW_SUMS)
+		if (lane < EW_SUMS) {
+#pragma unroll 8
 			for (int k = 0; k < parts; k++) mine += sums[EW_SUMS * (gi * parts + k) + lane];
+		}
 #pragma unroll
 		for (int a = 0; a < EW_SUMS; a++) q[a] = __shfl_sync(0xFFFFFFFFu, mine, a);
 		ewald_expand<TPL>(p, q, t);

@@ -40,3 +40,22 @@ def test_sort_tiles(kind, n):
             np.testing.assert_array_equal(out["key"], keys[order])
             np.testing.assert_array_equal(out["id"], order)
             np.testing.assert_array_equal(out["pos"], pos[:, order])
+
+
+@pytest.mark.parametrize("kind", ["random", "few", "corner"])
+@pytest.mark.parametrize("n", [5119, 5121, (1 << 19) - 1, 1 << 19, (1 << 19) + 1])
+def test_small_tiles(kind, n):
+    """Tiles of 1024 keys below 2^19 + 1 keys, of 4096 above, in a context that
+    has room for just these keys."""
+    rng = np.random.default_rng(n)
+    pos = positions(kind, n, rng)
+    with G.GravityContext(n, float_bytes=8, periodic=True, boxsize=1000.0) as ctx:
+        ctx.upload(pos, np.ones(n))
+        ctx.set_domain((0.0, 0.0, 0.0), 1000.0)
+        ctx.peano_keys()
+        keys = ctx.download(G.F_KEY)["key"]
+        perm = ctx.sort_particles()
+        out = ctx.download(G.F_KEY)
+        order = np.lexsort((keys[:, 1], keys[:, 0]))
+        np.testing.assert_array_equal(perm, order)
+        np.testing.assert_array_equal(out["key"], keys[order])
