@@ -18,7 +18,7 @@ against an FP64 Ewald-summed direct sum over all particles for 10^4 random
 particles); the step is one captured CUDA graph with the particles resident
 in HBM (`value`), and the same step through the C ABI from and to pinned host
 buffers with the copies overlapped (`e2e`, tvg_force_step_host). Beside it:
-the plain GPU form (the reference algorithm, one thread per particle, FP64,
+the plain GPU form (the reference algorithm for each particle, FP64,
 exact moments, the reference's TREE_OPEN_PARAM_REL 0.005) over all particles
 with its own measured error, the group form at the plain form's opening, the
 group form with monopoles, and the learned Ewald correction.
@@ -735,7 +735,7 @@ def main():
                 accuracy["plain"] = {k: float(f"{v:.4e}") for k, v in err64.items()}
             t_plain = pre_ms * 1e-3 + w_ms * 1e-3 * n / len(act)
             plain = {"value": n / t_plain, "unit": UNIT,
-                     "form": "plain: reference walk, one thread per particle, FP64, table Ewald",
+                     "form": "plain: reference walk, FP64, table Ewald",
                      "sample": ("keys, sort, build and the relative walk (incl. Ewald) of all "
                                 f"{n} particles, measured" if args.plain_stride == 1 else
                                 f"walk of every {args.plain_stride}th particle ({len(act)}), "
@@ -790,7 +790,7 @@ def main():
             "ewald_walk": {"kernel": f"k_ewald_group<{tune_choice}, false, float>",
                            "ms_per_step": round(ew_ms / args.steps, 2),
                            "evaluations_per_group": round(ew_i / args.steps / (n / (32 * tune_choice)), 1),
-                           "evaluation": "Taylor-table K, dK, d2K: 15 float4 loads, ~200 FP32 ops"},
+                           "evaluation": "Taylor-table K, dK, d2K: 8 float4 loads, ~200 FP32 ops"},
             "plain_form": plain,
             "group_form_monopole": monopole,
             "group_form_at_plain_opening": matched,

@@ -216,7 +216,7 @@ int tvg_download_tree(tvg_context *ctx, void *tree, int64_t tree_cap, int64_t *n
 /* ----------------------------------------------------------- tree walk */
 
 enum {
-	/* the reference algorithm, one thread per active particle, in Float */
+	/* the reference algorithm for each active particle, in Float */
 	TVG_FORM_PLAIN = 0,
 	/* one warp per PH group, FP32 on integer-offset positions */
 	TVG_FORM_GROUP = 1
@@ -335,7 +335,8 @@ int tvg_fp32_peak(tvg_context *ctx, double ms_target, double *tflops);
  * which keeps the last call's contents; calls that overlap on the same GPU
  * (from several host threads) race and give wrong results.
  * Returns TVG_E_BADINPUT for n < 0 or n > TVG_NOALLOC_MAX_KEYS, TVG_E_CUDA
- * on a CUDA error. */
+ * on a CUDA error, TVG_E_TIMEOUT if a pass gave up waiting for its earlier
+ * tiles (perm then holds no order, but only indices below n). */
 int tvg_sort_keys_noalloc(const uint64_t *key_hi, const uint64_t *key_lo, int64_t n, uint32_t *perm);
 
 /* Counters of the last walk: total gravity and Ewald interactions. */

@@ -30,14 +30,14 @@ int tvg_sync_status(tvg_context *ctx, const char *phase)
 // the status word, enqueued, and the look at it once the stream has passed it.
 int tvg_fetch_status(tvg_context *ctx)
 {
-	TVG_CUDA(ctx, cudaMemcpyAsync(ctx->h_status, ctx->status, sizeof(int), cudaMemcpyDeviceToHost,
+	TVG_CUDA(ctx, cudaMemcpyAsync(&ctx->host->status, ctx->status, sizeof(int), cudaMemcpyDeviceToHost,
 	                              ctx->stream));
 	return TVG_OK;
 }
 
 int tvg_check_status(tvg_context *ctx, const char *phase)
 {
-	int st = *ctx->h_status;
+	int st = ctx->host->status;
 	if (!st) return TVG_OK;
 	TVG_CUDA(ctx, cudaMemsetAsync(ctx->status, 0, sizeof(int), ctx->stream));
 	if (st & TVG_ST_COINCIDENT)
@@ -122,9 +122,7 @@ extern "C" int tvg_init(int device, const tvg_config *cfg, tvg_context **out)
 	TVG_CHECK(dalloc(ctx, &ctx->scan_tmp, ctx->scan_tmp_bytes));
 	TVG_CHECK(dalloc(ctx, (void **) &ctx->status, sizeof(int)));
 	TVG_CUDA(ctx, cudaMemset(ctx->status, 0, sizeof(int)));
-	TVG_CUDA(ctx, cudaMallocHost((void **) &ctx->h_status, sizeof(int)));
-	TVG_CUDA(ctx, cudaMallocHost((void **) &ctx->h_dc, sizeof(tvg_devcount)));
-	TVG_CUDA(ctx, cudaMallocHost((void **) &ctx->h_counts, 3 * sizeof(double)));
+	TVG_CUDA(ctx, cudaMallocHost((void **) &ctx->host, sizeof(tvg_mirror)));
 	TVG_CHECK(dalloc(ctx, (void **) &ctx->d_top, sizeof(tvg_topnode) * TVG_MAX_TOP));
 	TVG_CHECK(dalloc(ctx, (void **) &ctx->top_first, 4 * TVG_MAX_TOP));
 	TVG_CHECK(dalloc(ctx, (void **) &ctx->top_count, 4 * TVG_MAX_TOP));
@@ -163,13 +161,13 @@ extern "C" int tvg_init(int device, const tvg_config *cfg, tvg_context **out)
 // the device counts of the last step into the host mirrors, and the status word
 int tvg_read_counts(tvg_context *ctx)
 {
-	TVG_CUDA(ctx, cudaMemcpyAsync(ctx->h_dc, ctx->dc, sizeof(tvg_devcount), cudaMemcpyDeviceToHost,
+	TVG_CUDA(ctx, cudaMemcpyAsync(&ctx->host->dc, ctx->dc, sizeof(tvg_devcount), cudaMemcpyDeviceToHost,
 	                              ctx->stream));
 	TVG_CHECK(tvg_fetch_status(ctx));
 	TVG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-	ctx->ntop = ctx->h_dc->ntop;
-	ctx->nu = ctx->h_dc->nu;
-	ctx->nnodes = ctx->h_dc->nnodes;
+	ctx->ntop = ctx->host->dc.ntop;
+	ctx->nu = ctx->host->dc.nu;
+	ctx->nnodes = ctx->host->dc.nnodes;
 	return TVG_OK;
 }
 
@@ -196,9 +194,7 @@ extern "C" void tvg_finalize(tvg_context *ctx)
 	                 ctx->ewald_xyz, ctx->ft_ws, ctx->mlp_ws,
 	                 ctx->domain_state };
 	for (void *b : bufs) if (b) cudaFree(b);
-	if (ctx->h_status) cudaFreeHost(ctx->h_status);
-	if (ctx->h_dc) cudaFreeHost(ctx->h_dc);
-	if (ctx->h_counts) cudaFreeHost(ctx->h_counts);
+	if (ctx->host) cudaFreeHost(ctx->host);
 	for (int i = 0; i < 16; i++) if (ctx->ev[i]) cudaEventDestroy(ctx->ev[i]);
 	for (int i = 0; i < 3; i++) if (ctx->xev[i]) cudaEventDestroy(ctx->xev[i]);
 	if (ctx->copy_stream) cudaStreamDestroy(ctx->copy_stream);

@@ -88,6 +88,13 @@ struct tvg_devcount {
 	int64_t nwchild;         // walk nodes below the top nodes (TVG_CFG_QUADRUPOLE)
 };
 
+// What a step reads back, in one pinned allocation
+struct tvg_mirror {
+	int status;
+	tvg_devcount dc;
+	double counts[3];        // interactions of the group walk
+};
+
 // Per top node tables of the tree build, on the device (TVG_MAX_TOP
 // entries each, one allocation): the subtree's first node and node count,
 // the offset from a node's rank among the build's survivors to its tree
@@ -146,9 +153,7 @@ struct tvg_context {
 	void *scan_tmp = nullptr;
 	size_t scan_tmp_bytes = 0;
 	int *status = nullptr;             // device status word
-	int *h_status = nullptr;           // pinned mirror
-	tvg_devcount *h_dc = nullptr;      // pinned mirror of dc
-	double *h_counts = nullptr;        // pinned mirror of the group walk's counters
+	tvg_mirror *host = nullptr;        // pinned mirrors
 
 	// top nodes
 	int32_t ntop = 0;

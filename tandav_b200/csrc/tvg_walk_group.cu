@@ -2352,7 +2352,7 @@ static int walk_group_typed(tvg_context *ctx, int use_bh, uint32_t parts, int ew
 	if (!ctx->have_walktree) TVG_CHECK(prepare_typed<F>(ctx));
 	// the parts' sums of both walks, for the largest groups: at most WALK_ITEMS
 	// items, and no more than the capacity's groups in 64 parts
-	if (!ctx->part_sums) {
+	if (!ctx->part_sums && (sizeof(F) == 4 || (ewald && !mlp))) {
 		const int64_t most = (ctx->cap / 32 + 1) * 64, items = most < WALK_ITEMS ? most : WALK_ITEMS;
 		TVG_CUDA(ctx, cudaMalloc(&ctx->part_sums, sizeof(PartSum) * 128 * (size_t) items));
 	}
@@ -2436,14 +2436,14 @@ static int walk_group_typed(tvg_context *ctx, int use_bh, uint32_t parts, int ew
 // (synchronises)
 int tvg_walk_group_results(tvg_context *ctx)
 {
-	TVG_CUDA(ctx, cudaMemcpyAsync(ctx->h_counts, ctx->counters, 24, cudaMemcpyDeviceToHost, ctx->stream));
+	TVG_CUDA(ctx, cudaMemcpyAsync(ctx->host->counts, ctx->counters, 24, cudaMemcpyDeviceToHost, ctx->stream));
 	TVG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
 	float ms = 0, ms_e = 0;
 	TVG_CUDA(ctx, cudaEventElapsedTime(&ms, ctx->ev[0], ctx->ev[1]));
 	TVG_CUDA(ctx, cudaEventElapsedTime(&ms_e, ctx->ev[1], ctx->ev[2]));
 	ctx->phase_ms[4] = ms;
 	ctx->phase_ms[5] = ms_e;
-	for (int i = 0; i < 3; i++) ctx->last_counts[i] = ctx->h_counts[i];
+	for (int i = 0; i < 3; i++) ctx->last_counts[i] = ctx->host->counts[i];
 	return TVG_OK;
 }
 

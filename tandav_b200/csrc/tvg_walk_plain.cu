@@ -1,5 +1,5 @@
-// tvg_walk_plain.cu -- the plain GPU form: the reference tree walk, one
-// thread per active particle, in the host's Float width.
+// tvg_walk_plain.cu -- the plain GPU form: the reference tree walk of each
+// active particle, in the host's Float width.
 //
 // Gravity part: Gravity_Tree_Acceleration (tree_accel.c:32-394) -- every top
 // node (interact_with_topnode), then the subtree walk with the BH or the
