@@ -43,3 +43,31 @@ def test_tree_edges_vs_oracle(n, vsize, fsize, one_cell):
     assert_struct_equal(top, top_o, TOP_FIELDS, "topnodes")
     assert_struct_equal(tree, tree_o, TREE_FIELDS, "tree")
     assert np.array_equal(parent, parent_o)
+
+
+@pytest.mark.parametrize("n", [3000, 65_535, 65_536, 65_537])
+def test_tree_at_capacities(n):
+    """The build's scans run over the capacity (2 c + 4097 items), the active
+    set's over n: with one launch up to 16 tiles of 4096 items, two up to 2048,
+    and a scan of the sums beyond. The same particles give the same tree, the
+    same forces and the same window groups at capacities on both sides."""
+    pos, mass = clumps(n, 5, False)
+    caps = [c for c in (n, 30_719, 30_720, 4_192_255, 4_192_256) if c >= n]
+    active = np.arange(0, n, 3)
+    out = []
+    for cap in caps:
+        with G.GravityContext(cap, softening=1.0, vector_size=16, flags=G.CFG_QUADRUPOLE) as ctx:
+            ctx.upload(pos.astype(np.float32), mass.astype(np.float32))
+            ctx.set_domain((0.0, 0.0, 0.0), 1000.0)
+            ctx.force_step(form=G.FORM_GROUP, use_bh=True, parts=G.WALK_GRAVITY)
+            ctx.set_active(active)
+            ctx.walk(G.FORM_GROUP, use_bh=True, parts=G.WALK_GRAVITY)
+            tree, top = ctx.download_tree()
+            d = ctx.download(G.F_GRAV_ACC | G.F_COST | G.F_TREE_PARENT)
+            out.append((tree, top, d["cost"], d["tree_parent"], d["grav_acc"]))
+    for tree, top, cost, parent, acc in out[1:]:
+        np.testing.assert_array_equal(tree, out[0][0])
+        np.testing.assert_array_equal(top, out[0][1])
+        np.testing.assert_array_equal(cost, out[0][2])
+        np.testing.assert_array_equal(parent, out[0][3])
+        np.testing.assert_array_equal(acc, out[0][4])
