@@ -1032,20 +1032,29 @@ __device__ void walk_group(const GroupParams &p, SM &S, const tvg_wnode *__restr
 }
 
 // Parts of a group's walk: few groups leave the device idle (a warp each) and a
-// few long ones end alone, so the groups are split until there are WALK_ITEMS
-// warps' worth of them, eight for each of the 16 warps an SM holds, but no further
-// than the 64 level-2 cells' children give even shares. Each part has its own
-// sums, which k_walk_sum adds in order. Gravity walk, one warp per group / so: box
-// of 32^3 2.40 / 0.36 ms, halo of 3001 0.31 / 0.11 ms, box of 64^3 with monopoles 28.1 /
-// 22.5 ms (24.4 with four items a warp, 30.1 with two); Ewald walk of the 32^3 box
-// 0.48 / 0.13 ms. A part tests the roots again, 1 to 2 us, so light groups of a halo's
-// active list gain nothing (130,000 of 200,000 active: 0.38 / 0.42 ms).
-#define WALK_ITEMS (148 * 16 * 8)
+// few long ones end alone, so the groups are split until there are walk_items()
+// warps' worth of them, eight or sixteen for each of the 16 warps an SM holds, but
+// no further than the 64 level-2 cells' children give even shares. Each part has
+// its own sums, which k_walk_sum adds in order. Gravity walk, one warp per group /
+// with eight: box of 32^3 2.40 / 0.36 ms, halo of 3001 0.31 / 0.11 ms, box of 64^3
+// with monopoles 28.1 / 22.5 ms (24.4 with four, 30.1 with two); Ewald walk of the
+// 32^3 box 0.48 / 0.13 ms. A part tests the roots again, 1 to 2 us. The groups of a
+// periodic box are long (8000 interactions a target and more) and end unevenly:
+// with sixteen its walks gain (8 / 16 / 32 a warp, gravity walk: 100^3 12.8 / 12.0 /
+// 11.5 ms, 72^3 5.5 / 4.9 / 4.8, 64^3 with monopoles 22.9 / 22.1 / 22.1; Ewald walks
+// of 100^3 1.06 / 1.12 / 1.20, of 72^3 2.9 / 2.9 / 3.1). Those of an isolated halo are
+// light (130,000 of 200,000 active: one warp per group 0.38, 8 0.41, 16 0.49 ms).
+#define WALK_WARPS (148 * 16)
 #define WALK_MAX_PARTS 32
-__host__ __device__ __forceinline__ int walk_parts(int64_t ngroups)
+__host__ __device__ __forceinline__ int64_t walk_items(int periodic)
 {
-	const int64_t p = WALK_ITEMS / (ngroups > 0 ? ngroups : 1);
-	return p < 1 ? 1 : p > WALK_MAX_PARTS ? WALK_MAX_PARTS : (int) p;
+	return (int64_t) WALK_WARPS * (periodic ? 16 : 8);
+}
+
+__host__ __device__ __forceinline__ int walk_parts(const GroupParams &p, int64_t ngroups)
+{
+	const int64_t k = walk_items(p.periodic) / (ngroups > 0 ? ngroups : 1);
+	return k < 1 ? 1 : k > WALK_MAX_PARTS ? WALK_MAX_PARTS : (int) k;
 }
 
 // The warp's memory. A pop takes at most 1/7 of the stack's free room, so a short
@@ -1085,7 +1094,7 @@ k_walk_group(GroupParams p, const int32_t *__restrict__ active, const int32_t *_
 	const int lane = threadIdx.x & 31;
 	double cnt_acc = 0, qcnt_acc = 0;
 	const int64_t ngroups = p.dc->ngroups;
-	const int parts = SPLIT ? walk_parts(ngroups) : 1;
+	const int parts = SPLIT ? walk_parts(p, ngroups) : 1;
 	for (;;) {
 		int64_t item = 0;
 		if (lane == 0) item = atomicAdd(work, 1);
@@ -1143,7 +1152,7 @@ k_walk_sum(GroupParams p, const int32_t *__restrict__ active, const int32_t *__r
            double *counter)
 {
 	const int64_t ngroups = p.dc->ngroups;
-	const int parts = walk_parts(ngroups);
+	const int parts = walk_parts(p, ngroups);
 	if (parts == 1) return;
 	double cnt = 0, qcnt = 0;
 	for (int64_t e = blockIdx.x * (int64_t) blockDim.x + threadIdx.x; e < ngroups * p.gsize;
@@ -1760,7 +1769,7 @@ k_ewald_group(GroupParams p, const int32_t *__restrict__ active, const int32_t *
 	const int lane = threadIdx.x & 31;
 	double ev_acc = 0;
 	const int64_t ngroups = p.dc->ngroups;
-	const int parts = SPLIT ? walk_parts(ngroups) : 1;
+	const int parts = SPLIT ? walk_parts(p, ngroups) : 1;
 	for (;;) {
 		int64_t item = 0;
 		if (lane == 0) item = atomicAdd(work, 1);
@@ -2037,7 +2046,7 @@ k_ewald_sum(GroupParams p, const int32_t *__restrict__ active, const int32_t *__
             F *gacc0, F *gacc1, F *gacc2)
 {
 	const int64_t ngroups = p.dc->ngroups;
-	const int parts = walk_parts(ngroups), lane = threadIdx.x & 31;
+	const int parts = walk_parts(p, ngroups), lane = threadIdx.x & 31;
 	if (parts == 1) return;
 	for (int64_t gi = (blockIdx.x * (int64_t) blockDim.x + threadIdx.x) >> 5; gi < ngroups;
 	     gi += ((int64_t) gridDim.x * blockDim.x) >> 5) {
@@ -2247,7 +2256,7 @@ static int launch_walk_q(tvg_context *ctx, GroupParams p, const float *mass_f, c
 // split changes the sums' order (1e-7 of the force).
 static bool may_split(const tvg_context *ctx, const GroupParams &p)
 {
-	return ctx->cfg.float_bytes == 4 && (ctx->use_active || walk_parts((ctx->n + p.gsize - 1) / p.gsize) > 1);
+	return ctx->cfg.float_bytes == 4 && (ctx->use_active || walk_parts(p, (ctx->n + p.gsize - 1) / p.gsize) > 1);
 }
 
 template <int MODE, int TPL, typename F>
@@ -2350,10 +2359,11 @@ static int walk_group_typed(tvg_context *ctx, int use_bh, uint32_t parts, int ew
 		                "the table (tvg_ewald_mlp_validate)");
 	cudaStream_t s = ctx->stream;
 	if (!ctx->have_walktree) TVG_CHECK(prepare_typed<F>(ctx));
-	// the parts' sums of both walks, for the largest groups: at most WALK_ITEMS
+	// the parts' sums of both walks, for the largest groups: at most walk_items()
 	// items, and no more than the capacity's groups in 64 parts
 	if (!ctx->part_sums && (sizeof(F) == 4 || (ewald && !mlp))) {
-		const int64_t most = (ctx->cap / 32 + 1) * 64, items = most < WALK_ITEMS ? most : WALK_ITEMS;
+		const int64_t most = (ctx->cap / 32 + 1) * 64, full = walk_items(ctx->cfg.periodic);
+		const int64_t items = most < full ? most : full;
 		TVG_CUDA(ctx, cudaMalloc(&ctx->part_sums, sizeof(PartSum) * 128 * (size_t) items));
 	}
 	if (ewald && !mlp) {
