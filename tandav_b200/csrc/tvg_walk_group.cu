@@ -1143,8 +1143,8 @@ k_walk_group(GroupParams p, const int32_t *__restrict__ active, const int32_t *_
 	if (QUAD && lane == 0 && qcnt_acc != 0) atomicAdd(counter + 2, qcnt_acc);
 }
 
-// the parts' sums of each target, in order, eight in flight (few groups, so few
-// blocks, each as long as a thread's chain of loads)
+// the parts' sums of each target, in order (32,768 targets in 32 parts: 22 us,
+// unrolled or not)
 template <typename F>
 __global__ void __launch_bounds__(256)
 k_walk_sum(GroupParams p, const int32_t *__restrict__ active, const int32_t *__restrict__ gfirst,
