@@ -86,6 +86,7 @@ template <typename F> struct PlainCtx {
 	F r2min, r2max;            // FP32: range of the branch-free root (inv_sqrt)
 	F box;                     // FP32: boxsize as a float, 0 if it is not one
 	int64_t tree_cap;          // node capacity: the walks never read past it
+	int64_t n;                 // particles
 	PlainParams p;
 };
 
@@ -356,6 +357,26 @@ __device__ __forceinline__ void gravity_bundle(const PlainCtx<double> &c, const 
 	}
 }
 
+// The particles of an opened small top node: the reference takes them from
+// Target on, a running node count, which passes the last particle when nodes
+// outnumber particles (bundles of one). add(f, np) takes those that exist;
+// past(d) says whether a particle at the origin, d from the target, counts: what
+// lies past the last particle is such a particle without mass, which adds nothing
+// but its count.
+template <typename F, typename Add, typename Past>
+__device__ __forceinline__ void small_top(const PlainCtx<F> &c, const tvg_topnode &t, const F sp[3], Sums &s,
+                                          Add add, Past past)
+{
+	const int64_t f = c.p.fix_small ? t.first_part : t.target;
+	const int np = (int) max((int64_t) 0, min((int64_t) t.npart, c.n - f));
+	add(f, np);
+	if (np < t.npart) {
+		F d[3] = { -sp[0], -sp[1], -sp[2] };
+		nearest(c, d);
+		if (past(d)) s.n += t.npart - np;
+	}
+}
+
 // one node of a subtree for one target; returns the node it goes to next
 // (INT_MAX at the subtree's terminator, DNext = 0; a valid tree ends every
 // subtree with one well inside the capacity, the bound keeps a damaged one in
@@ -413,7 +434,10 @@ __device__ void walk_gravity(const PlainCtx<F> &c, const Lanes<S> &l, bool have,
 			}
 		}
 		if (t.npart <= c.p.vsize) {
-			if (open) gravity_bundle<POT, S>(c, l, c.p.fix_small ? t.first_part : t.target, t.npart, sp, s);
+			if (open)
+				small_top(
+				    c, t, sp, s, [&](int64_t f, int np) { gravity_bundle<POT, S>(c, l, f, np, sp, s); },
+				    [](const F d[3]) { return d[0] * d[0] + d[1] * d[1] + d[2] * d[2] != 0; });
 			if (COH) __syncwarp();
 			continue;
 		}
@@ -631,7 +655,10 @@ __device__ void walk_ewald(const PlainCtx<F> &c, const Lanes<S> &l, bool have, c
 			if (!open) ewald_add_node<POT>(c, dr, (F) t.mass, s);
 		}
 		if (t.npart <= c.p.vsize) {
-			if (open) ewald_bundle<POT, S>(c, l, c.p.fix_small ? t.first_part : t.target, t.npart, sp, s);
+			if (open)
+				small_top(
+				    c, t, sp, s, [&](int64_t f, int np) { ewald_bundle<POT, S>(c, l, f, np, sp, s); },
+				    [](const F d[3]) { return d[0] != 0 && d[1] != 0 && d[2] != 0; });
 			if (COH) __syncwarp();
 			continue;
 		}
@@ -810,6 +837,7 @@ static int walk_typed(tvg_context *ctx, int use_bh, uint32_t parts)
 	c.top = ctx->d_top;
 	c.tree = (const WNode<F> *) ctx->tree;
 	c.tree_cap = ctx->tcap;
+	c.n = n;
 	const tvg_config &cf = ctx->cfg;
 	c.p.gravity = cf.gravity;
 	c.p.domain_size = ctx->dsize;
