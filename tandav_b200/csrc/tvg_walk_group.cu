@@ -443,6 +443,7 @@ struct GroupParams {
 	float taylor_h;     // groups with a larger half extent take per-target images (with Ewald)
 	float wide_grid;    // node spacings per length of the table for single points
 	float tay_grid;     // Taylor-table node spacings per length (2 (TVG_TAYLOR_NODES - 1) / L)
+	int items;          // items of a split walk (walk_items)
 	double uniform_g;   // G / L^2: times the total mass, the scale of the uniform-background remainder
 };
 
@@ -1033,27 +1034,28 @@ __device__ void walk_group(const GroupParams &p, SM &S, const tvg_wnode *__restr
 
 // Parts of a group's walk: few groups leave the device idle (a warp each) and a
 // few long ones end alone, so the groups are split until there are walk_items()
-// warps' worth of them, eight or sixteen for each of the 16 warps an SM holds, but
-// no further than the 64 level-2 cells' children give even shares. Each part has
-// its own sums, which k_walk_sum adds in order. Gravity walk, one warp per group /
-// with eight: box of 32^3 2.40 / 0.36 ms, halo of 3001 0.31 / 0.11 ms, box of 64^3
-// with monopoles 28.1 / 22.5 ms (24.4 with four, 30.1 with two); Ewald walk of the
-// 32^3 box 0.48 / 0.13 ms. A part tests the roots again, 1 to 2 us. The groups of a
-// periodic box are long (8000 interactions a target and more) and end unevenly:
-// with sixteen its walks gain (8 / 16 / 32 a warp, gravity walk: 100^3 12.8 / 12.0 /
-// 11.5 ms, 72^3 5.5 / 4.9 / 4.8, 64^3 with monopoles 22.9 / 22.1 / 22.1; Ewald walks
-// of 100^3 1.06 / 1.12 / 1.20, of 72^3 2.9 / 2.9 / 3.1). Those of an isolated halo are
-// light (130,000 of 200,000 active: one warp per group 0.38, 8 0.41, 16 0.49 ms).
+// warps' worth of them, but no further than the 64 level-2 cells' children give even
+// shares. Each part has its own sums, which k_walk_sum adds in order. A part tests
+// the roots again and has lists of its own to flush, a few us, so how many
+// items the 16 warps an SM holds should have depends on how long the walks are. All
+// particles of a periodic box are long (8000 interactions a target and more) and end
+// unevenly: sixteen a warp (8 / 16 / 32, gravity walk: 100^3 12.8 / 12.0 / 11.5 ms,
+// 72^3 5.5 / 4.9 / 4.8, 64^3 with monopoles 22.9 / 22.1 / 22.1; Ewald walks of 100^3
+// 1.06 / 1.12 / 1.20, of 72^3 2.9 / 2.9 / 3.1). Those of an isolated halo are
+// lighter: eight (one warp per group / 8, both of 64 particles: box of 32^3 2.40 /
+// 0.36 ms, halo of 3001 0.31 / 0.11, of 100,000 2.6 / 1.9). The groups of an active
+// list may be of any kind, among them light ones, in any number: two (walks of lists,
+// ms with unsplit groups / 2 / 16 a warp: of a clumpy box of 10^6 1000 particles
+// spread 0.10 / 0.10 / 0.25, 100,000 neighbours 0.24 / 0.26 / 0.49; of a 128^3 box
+// 1000 spread 4.7 / 2.3 / 2.2, 20,000 neighbours 5.5 / 1.0 / 1.0; of a halo of 10^6
+// 1000 spread 0.18 / 0.12 / 0.19, 100,000 neighbours 0.35 / 0.30 / 0.42).
 #define WALK_WARPS (148 * 16)
 #define WALK_MAX_PARTS 32
-__host__ __device__ __forceinline__ int64_t walk_items(int periodic)
-{
-	return (int64_t) WALK_WARPS * (periodic ? 16 : 8);
-}
+static int walk_items(bool periodic, bool list) { return WALK_WARPS * (list ? 2 : periodic ? 16 : 8); }
 
 __host__ __device__ __forceinline__ int walk_parts(const GroupParams &p, int64_t ngroups)
 {
-	const int64_t k = walk_items(p.periodic) / (ngroups > 0 ? ngroups : 1);
+	const int64_t k = p.items / (ngroups > 0 ? ngroups : 1);
 	return k < 1 ? 1 : k > WALK_MAX_PARTS ? WALK_MAX_PARTS : (int) k;
 }
 
@@ -2362,7 +2364,7 @@ static int walk_group_typed(tvg_context *ctx, int use_bh, uint32_t parts, int ew
 	// the parts' sums of both walks, for the largest groups: at most walk_items()
 	// items, and no more than the capacity's groups in 64 parts
 	if (!ctx->part_sums && (sizeof(F) == 4 || (ewald && !mlp))) {
-		const int64_t most = (ctx->cap / 32 + 1) * 64, full = walk_items(ctx->cfg.periodic);
+		const int64_t most = (ctx->cap / 32 + 1) * 64, full = walk_items(ctx->cfg.periodic, false);
 		const int64_t items = most < full ? most : full;
 		TVG_CUDA(ctx, cudaMalloc(&ctx->part_sums, sizeof(PartSum) * 128 * (size_t) items));
 	}
@@ -2399,6 +2401,7 @@ static int walk_group_typed(tvg_context *ctx, int use_bh, uint32_t parts, int ew
 		TVG_CUDA(ctx, cudaGetLastError());
 	}
 	p.periodic = cf.periodic;
+	p.items = walk_items(cf.periodic, ctx->use_active);
 	p.use_bh = use_bh;
 	p.open_bundles = (cf.flags & TVG_CFG_OPEN_BUNDLES) ? 1 : 0;
 	p.scale = (float) (cf.periodic ? ctx->dsize / 4294967296.0 : ctx->dsize / 2147483648.0);
