@@ -62,7 +62,8 @@ int tvg_check_status(tvg_context *ctx, const char *phase)
 	return tvg_fail(ctx, TVG_E_CUDA, "%s: device status 0x%x", phase, st);
 }
 
-static int dalloc(tvg_context *ctx, void **p, size_t bytes)
+// device memory, TVG_E_NOMEM when there is none
+int tvg_alloc(tvg_context *ctx, void **p, size_t bytes)
 {
 	if (bytes == 0) bytes = 16;
 	cudaError_t e = cudaMalloc(p, bytes);
@@ -106,54 +107,54 @@ extern "C" int tvg_init(int device, const tvg_config *cfg, tvg_context **out)
 	const int64_t cap = ctx->cap;
 	for (int s = 0; s < FS_NFIELDS; s++) {
 		size_t b = tvg_field_bytes(ctx, s) * (size_t) cap;
-		TVG_CHECK(dalloc(ctx, &ctx->f[s], b));
-		TVG_CHECK(dalloc(ctx, &ctx->falt[s], b));
+		TVG_CHECK(tvg_alloc(ctx, &ctx->f[s], b));
+		TVG_CHECK(tvg_alloc(ctx, &ctx->falt[s], b));
 		TVG_CUDA(ctx, cudaMemset(ctx->f[s], 0, b));
 	}
-	TVG_CHECK(dalloc(ctx, (void **) &ctx->key_hi, 8 * cap));
-	TVG_CHECK(dalloc(ctx, (void **) &ctx->key_lo, 8 * cap));
-	TVG_CHECK(dalloc(ctx, (void **) &ctx->key_tmp, 8 * cap));
-	TVG_CHECK(dalloc(ctx, (void **) &ctx->perm, 4 * cap));
-	TVG_CHECK(dalloc(ctx, (void **) &ctx->perm_tmp, 4 * cap));
-	TVG_CHECK(dalloc(ctx, (void **) &ctx->sort_hist, 4 * tvg_sort_state_words(cap)));
-	TVG_CHECK(dalloc(ctx, (void **) &ctx->sort_off, 4 * tvg_sort_state_words(cap)));
-	TVG_CHECK(dalloc(ctx, (void **) &ctx->digit_count, 4 * 8 * 256));
+	TVG_CHECK(tvg_alloc(ctx, (void **) &ctx->key_hi, 8 * cap));
+	TVG_CHECK(tvg_alloc(ctx, (void **) &ctx->key_lo, 8 * cap));
+	TVG_CHECK(tvg_alloc(ctx, (void **) &ctx->key_tmp, 8 * cap));
+	TVG_CHECK(tvg_alloc(ctx, (void **) &ctx->perm, 4 * cap));
+	TVG_CHECK(tvg_alloc(ctx, (void **) &ctx->perm_tmp, 4 * cap));
+	TVG_CHECK(tvg_alloc(ctx, (void **) &ctx->sort_hist, 4 * tvg_sort_state_words(cap)));
+	TVG_CHECK(tvg_alloc(ctx, (void **) &ctx->sort_off, 4 * tvg_sort_state_words(cap)));
+	TVG_CHECK(tvg_alloc(ctx, (void **) &ctx->digit_count, 4 * 8 * 256));
 	ctx->scan_tmp_bytes = 8 * ((cap * 3) / 512 + 4096);
-	TVG_CHECK(dalloc(ctx, &ctx->scan_tmp, ctx->scan_tmp_bytes));
-	TVG_CHECK(dalloc(ctx, (void **) &ctx->status, sizeof(int)));
+	TVG_CHECK(tvg_alloc(ctx, &ctx->scan_tmp, ctx->scan_tmp_bytes));
+	TVG_CHECK(tvg_alloc(ctx, (void **) &ctx->status, sizeof(int)));
 	TVG_CUDA(ctx, cudaMemset(ctx->status, 0, sizeof(int)));
 	TVG_CUDA(ctx, cudaMallocHost((void **) &ctx->host, sizeof(tvg_mirror)));
-	TVG_CHECK(dalloc(ctx, (void **) &ctx->d_top, sizeof(tvg_topnode) * TVG_MAX_TOP));
-	TVG_CHECK(dalloc(ctx, (void **) &ctx->top_first, 4 * TVG_MAX_TOP));
-	TVG_CHECK(dalloc(ctx, (void **) &ctx->top_count, 4 * TVG_MAX_TOP));
-	TVG_CHECK(dalloc(ctx, (void **) &ctx->lvl, cap + 64));
-	TVG_CHECK(dalloc(ctx, (void **) &ctx->lvl_min64, cap / 64 + 64));
-	TVG_CHECK(dalloc(ctx, (void **) &ctx->ncnt, 4 * (cap + 1)));
+	TVG_CHECK(tvg_alloc(ctx, (void **) &ctx->d_top, sizeof(tvg_topnode) * TVG_MAX_TOP));
+	TVG_CHECK(tvg_alloc(ctx, (void **) &ctx->top_first, 4 * TVG_MAX_TOP));
+	TVG_CHECK(tvg_alloc(ctx, (void **) &ctx->top_count, 4 * TVG_MAX_TOP));
+	TVG_CHECK(tvg_alloc(ctx, (void **) &ctx->lvl, cap + 64));
+	TVG_CHECK(tvg_alloc(ctx, (void **) &ctx->lvl_min64, cap / 64 + 64));
+	TVG_CHECK(tvg_alloc(ctx, (void **) &ctx->ncnt, 4 * (cap + 1)));
 	// uncollapsed nodes: at most ~2 per particle for non-degenerate inputs;
 	// the build checks the bound and fails with TVG_E_TREE_FULL otherwise
 	ctx->ucap = 2 * cap + 4096;
-	TVG_CHECK(dalloc(ctx, (void **) &ctx->u_start, 4 * ctx->ucap));
-	TVG_CHECK(dalloc(ctx, (void **) &ctx->u_count, 4 * ctx->ucap));
-	TVG_CHECK(dalloc(ctx, (void **) &ctx->u_endu, 4 * ctx->ucap));
-	TVG_CHECK(dalloc(ctx, (void **) &ctx->u_diff, 4 * (ctx->ucap + 1)));
-	TVG_CHECK(dalloc(ctx, (void **) &ctx->u_final, 4 * (ctx->ucap + 1)));
-	TVG_CHECK(dalloc(ctx, (void **) &ctx->u_level, ctx->ucap));
-	TVG_CHECK(dalloc(ctx, (void **) &ctx->u_flag, ctx->ucap));
+	TVG_CHECK(tvg_alloc(ctx, (void **) &ctx->u_start, 4 * ctx->ucap));
+	TVG_CHECK(tvg_alloc(ctx, (void **) &ctx->u_count, 4 * ctx->ucap));
+	TVG_CHECK(tvg_alloc(ctx, (void **) &ctx->u_endu, 4 * ctx->ucap));
+	TVG_CHECK(tvg_alloc(ctx, (void **) &ctx->u_diff, 4 * (ctx->ucap + 1)));
+	TVG_CHECK(tvg_alloc(ctx, (void **) &ctx->u_final, 4 * (ctx->ucap + 1)));
+	TVG_CHECK(tvg_alloc(ctx, (void **) &ctx->u_level, ctx->ucap));
+	TVG_CHECK(tvg_alloc(ctx, (void **) &ctx->u_flag, ctx->ucap));
 	ctx->tcap = cap + 2 * TVG_MAX_TOP + 4096;
 	size_t node_bytes = 16 + 10 * tvg_fsize(ctx);
-	TVG_CHECK(dalloc(ctx, &ctx->tree, node_bytes * ctx->tcap));
-	TVG_CHECK(dalloc(ctx, (void **) &ctx->tree_u, 4 * ctx->tcap));
-	TVG_CHECK(dalloc(ctx, (void **) &ctx->pref, 8 * 4 * (cap + 1)));
-	for (int k = 0; k < 3; k++) TVG_CHECK(dalloc(ctx, (void **) &ctx->ipos[k], 4 * cap));
-	TVG_CHECK(dalloc(ctx, (void **) &ctx->wtree, sizeof(tvg_wnode) * ctx->tcap));
-	TVG_CHECK(dalloc(ctx, (void **) &ctx->big_list, 4 * (ctx->tcap + 2)));
-	TVG_CHECK(dalloc(ctx, (void **) &ctx->group_first, 4 * (cap / 8 + 1024)));
-	TVG_CHECK(dalloc(ctx, (void **) &ctx->work_counter, 64));
-	TVG_CHECK(dalloc(ctx, (void **) &ctx->counters, 8 * 8));
-	TVG_CHECK(dalloc(ctx, (void **) &ctx->dc, sizeof(tvg_devcount)));
-	TVG_CHECK(dalloc(ctx, (void **) &ctx->d_toptab, 4 * sizeof(int32_t) * TVG_MAX_TOP));
+	TVG_CHECK(tvg_alloc(ctx, &ctx->tree, node_bytes * ctx->tcap));
+	TVG_CHECK(tvg_alloc(ctx, (void **) &ctx->tree_u, 4 * ctx->tcap));
+	TVG_CHECK(tvg_alloc(ctx, (void **) &ctx->pref, 8 * 4 * (cap + 1)));
+	for (int k = 0; k < 3; k++) TVG_CHECK(tvg_alloc(ctx, (void **) &ctx->ipos[k], 4 * cap));
+	TVG_CHECK(tvg_alloc(ctx, (void **) &ctx->wtree, sizeof(tvg_wnode) * ctx->tcap));
+	TVG_CHECK(tvg_alloc(ctx, (void **) &ctx->big_list, 4 * (ctx->tcap + 2)));
+	TVG_CHECK(tvg_alloc(ctx, (void **) &ctx->group_first, 4 * (cap / 8 + 1024)));
+	TVG_CHECK(tvg_alloc(ctx, (void **) &ctx->work_counter, 64));
+	TVG_CHECK(tvg_alloc(ctx, (void **) &ctx->counters, 8 * 8));
+	TVG_CHECK(tvg_alloc(ctx, (void **) &ctx->dc, sizeof(tvg_devcount)));
+	TVG_CHECK(tvg_alloc(ctx, (void **) &ctx->d_toptab, 4 * sizeof(int32_t) * TVG_MAX_TOP));
 	TVG_CUDA(ctx, cudaMemset(ctx->d_toptab, 0, 4 * sizeof(int32_t) * TVG_MAX_TOP));
-	TVG_CHECK(dalloc(ctx, (void **) &ctx->top_of, 4 * cap));
+	TVG_CHECK(tvg_alloc(ctx, (void **) &ctx->top_of, 4 * cap));
 	TVG_CUDA(ctx, cudaMemset(ctx->dc, 0, sizeof(tvg_devcount)));
 	return TVG_OK;
 }

@@ -204,7 +204,7 @@ int find_domain_typed(tvg_context *ctx, double origin[3], double *size)
 	const int64_t n = ctx->n;
 	cudaStream_t s = ctx->stream;
 	const F *x = (const F *) ctx->f[FS_POS0], *y = (const F *) ctx->f[FS_POS1], *z = (const F *) ctx->f[FS_POS2];
-	if (!ctx->domain_state) TVG_CUDA(ctx, cudaMalloc(&ctx->domain_state, sizeof(DomainState)));
+	if (!ctx->domain_state) TVG_CHECK(tvg_alloc(ctx, &ctx->domain_state, sizeof(DomainState)));
 	DomainState *st = (DomainState *) ctx->domain_state;
 	// up to DS_BLOCKS blocks a SM
 	const unsigned need = tvg_blocks(n, DS_IPT * DS_THREADS), grid = need < 148u * DS_BLOCKS ? need : 148u * DS_BLOCKS;

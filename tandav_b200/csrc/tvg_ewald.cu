@@ -216,16 +216,18 @@ static int make_table(tvg_context *ctx, int nodes, size_t record, void (*kernel)
 	const int nf = fine_points(nodes);
 	const int64_t n = (int64_t) nodes * nodes * nodes, nfine = (int64_t) nf * nf * nf;
 	double *fine = nullptr;
-	TVG_CUDA(ctx, cudaMalloc((void **) &fine, 24 * (size_t) nfine));
 	float *tab = nullptr;
-	cudaError_t e = cudaMalloc((void **) &tab, record * (size_t) n);
-	if (e == cudaSuccess) {
-		k_ewald_fine<<<TVG_CNT(ctx, tvg_blocks(nfine, 128)), 128, 0, ctx->stream>>>(nodes, fine);
-		kernel<<<TVG_CNT(ctx, tvg_blocks(n, 128)), 128, 0, ctx->stream>>>(fine, tab);
-		e = cudaGetLastError();
-		const cudaError_t es = cudaStreamSynchronize(ctx->stream);
-		if (e == cudaSuccess) e = es;
+	TVG_CHECK(tvg_alloc(ctx, (void **) &fine, 24 * (size_t) nfine));
+	const int rc = tvg_alloc(ctx, (void **) &tab, record * (size_t) n);
+	if (rc != TVG_OK) {
+		cudaFree(fine);
+		return rc;
 	}
+	k_ewald_fine<<<TVG_CNT(ctx, tvg_blocks(nfine, 128)), 128, 0, ctx->stream>>>(nodes, fine);
+	kernel<<<TVG_CNT(ctx, tvg_blocks(n, 128)), 128, 0, ctx->stream>>>(fine, tab);
+	cudaError_t e = cudaGetLastError();
+	const cudaError_t es = cudaStreamSynchronize(ctx->stream);
+	if (e == cudaSuccess) e = es;
 	cudaFree(fine);
 	if (e != cudaSuccess) {
 		cudaFree(tab);

@@ -194,6 +194,7 @@ struct tvg_context {
 	float *ewald_wide = nullptr;       // T and 3 derivatives at TVG_WIDE_NODES^3 nodes, 24 floats each
 	int32_t *wide_list = nullptr;      // groups that take per-target images (k_ewald_wide)
 	void *part_sums = nullptr;         // sums of the parts of split groups (both group walks)
+	size_t part_bytes = 0;
 	float *ewald_taylor = nullptr;     // T and 3 derivatives at TVG_TAYLOR_NODES^3 nodes, 32 floats each
 	// Ewald-walk opening of the group form: the monopole error of the
 	// correction may reach ewald_open_rel |a_old| (relative mode); the limit of
@@ -272,6 +273,7 @@ struct tvg_context {
 
 
 int tvg_fail(tvg_context *ctx, int code, const char *fmt, ...);
+int tvg_alloc(tvg_context *ctx, void **p, size_t bytes);
 int tvg_sync_status(tvg_context *ctx, const char *phase);
 int tvg_fetch_status(tvg_context *ctx);
 int tvg_check_status(tvg_context *ctx, const char *phase);

@@ -53,6 +53,8 @@
 // convention.
 #include <stdlib.h>
 
+#include <algorithm>
+
 #include "tvg_internal.cuh"
 #include "tvg_ewald_mlp.cuh"
 
@@ -443,7 +445,8 @@ struct GroupParams {
 	float taylor_h;     // groups with a larger half extent take per-target images (with Ewald)
 	float wide_grid;    // node spacings per length of the table for single points
 	float tay_grid;     // Taylor-table node spacings per length (2 (TVG_TAYLOR_NODES - 1) / L)
-	int items;          // items of a split walk (walk_items)
+	int items;          // items of a split walk (walk_items), 0: no group is split
+	int wide_items;     // the same for the groups with per-target images (k_ewald_wide)
 	double uniform_g;   // G / L^2: times the total mass, the scale of the uniform-background remainder
 };
 
@@ -1821,9 +1824,10 @@ k_ewald_group(GroupParams p, const int32_t *__restrict__ active, const int32_t *
 // few wide groups: 38 ms of Ewald walk with a warp for each, 1.7 ms so; of 48^3,
 // all wide, monopoles: 1990 and 113 ms (there the smaller records count).
 #define WIDE_ITEMS 4736
-__device__ __forceinline__ int wide_parts(int nwide, int ntop)
+#define WIDE_MAX_PARTS 64
+__device__ __forceinline__ int wide_parts(const GroupParams &p, int nwide)
 {
-	return max(1, min(min(ntop, 64), WIDE_ITEMS / max(nwide, 1)));
+	return max(1, min(min(p.dc->ntop, WIDE_MAX_PARTS), p.wide_items / max(nwide, 1)));
 }
 
 template <int TPL>
@@ -1959,7 +1963,7 @@ k_ewald_wide(GroupParams p, const int32_t *__restrict__ active, const int32_t *_
 	EwaldSmem &S = ((EwaldSmem *) smem_raw)[threadIdx.x >> 5];
 	const int lane = threadIdx.x & 31, nwide = wide[0];
 	if (nwide == 0) return;
-	const int parts = wide_parts(nwide, p.dc->ntop);
+	const int parts = wide_parts(p, nwide);
 	double nev = 0;
 	for (;;) {
 		int item = 0;
@@ -2011,7 +2015,7 @@ __global__ void k_ewald_wide_sum(GroupParams p, const int32_t *__restrict__ acti
                                  const double *__restrict__ part, F *acc0, F *acc1, F *acc2, F *gacc0,
                                  F *gacc1, F *gacc2)
 {
-	const int nwide = wide[0], parts = nwide ? wide_parts(nwide, p.dc->ntop) : 1;
+	const int nwide = wide[0], parts = nwide ? wide_parts(p, nwide) : 1;
 	if (parts <= 1) return;
 	for (int64_t e = blockIdx.x * (int64_t) blockDim.x + threadIdx.x; e < (int64_t) nwide * p.gsize;
 	     e += (int64_t) gridDim.x * blockDim.x) {
@@ -2252,7 +2256,7 @@ static int launch_walk_q(tvg_context *ctx, GroupParams p, const float *mass_f, c
 	return TVG_OK;
 }
 
-// whether the groups may be split: from the number of groups, or, for an active
+// Whether the groups may be split: from the number of groups, or, for an active
 // list, whose length the device knows, always (its kernels then decide). FP64
 // contexts keep a warp per group: they return the FP32 sums at full width, and a
 // split changes the sums' order (1e-7 of the force).
@@ -2340,6 +2344,35 @@ static int launch_pair(tvg_context *ctx, const GroupParams &p, bool ewald, bool 
 	return launch_ewald<TPL, false, F, false>(ctx, p, mass_f, last_f, cnt + 1);
 }
 
+// Memory for the parts' sums of a walk in groups of p.gsize, for the capacity's
+// number of groups: both walks' split groups, and the groups with per-target
+// images (table). 3001 particles in groups of 64 take 3 MB, a box of 32^3 34 MB, a
+// box of 256^3, of which only the latter groups can be split, 7 MB. Without the memory
+// the walk goes on with one part a group. Captured steps hold the pointer: they are
+// dropped when it changes (a walk that is being captured follows a direct one of the
+// same size and finds the memory there).
+static void part_room(tvg_context *ctx, GroupParams &p, bool wide)
+{
+	const int64_t groups = ctx->cap / p.gsize + 1;
+	const int64_t split = may_split(ctx, p) ? std::min<int64_t>(p.items, WALK_MAX_PARTS * groups) : 0;
+	const int64_t images = wide ? std::min<int64_t>(p.wide_items, WIDE_MAX_PARTS * groups) : 0;
+	const size_t need_split = sizeof(PartSum) * (size_t) (split * p.gsize), need_wide = 24 * (size_t) (images * p.gsize);
+	const size_t need = std::max(need_split, need_wide);
+	if (need > ctx->part_bytes && !ctx->capturing) {
+		void *m = nullptr;
+		if (cudaMalloc(&m, need) == cudaSuccess) {
+			tvg_graph_release(ctx);
+			cudaFree(ctx->part_sums);
+			ctx->part_sums = m;
+			ctx->part_bytes = need;
+		} else {
+			cudaGetLastError();
+		}
+	}
+	if (need_split > ctx->part_bytes) p.items = 0;
+	if (need_wide > ctx->part_bytes) p.wide_items = 0;
+}
+
 template <typename F>
 static int walk_group_typed(tvg_context *ctx, int use_bh, uint32_t parts, int ewald_kind)
 {
@@ -2361,18 +2394,10 @@ static int walk_group_typed(tvg_context *ctx, int use_bh, uint32_t parts, int ew
 		                "the table (tvg_ewald_mlp_validate)");
 	cudaStream_t s = ctx->stream;
 	if (!ctx->have_walktree) TVG_CHECK(prepare_typed<F>(ctx));
-	// the parts' sums of both walks, for the largest groups: at most walk_items()
-	// items, and no more than the capacity's groups in 64 parts
-	if (!ctx->part_sums && (sizeof(F) == 4 || (ewald && !mlp))) {
-		const int64_t most = (ctx->cap / 32 + 1) * 64, full = walk_items(ctx->cfg.periodic, false);
-		const int64_t items = most < full ? most : full;
-		TVG_CUDA(ctx, cudaMalloc(&ctx->part_sums, sizeof(PartSum) * 128 * (size_t) items));
-	}
 	if (ewald && !mlp) {
 		if (!ctx->ewald_wide) TVG_CHECK(tvg_impl_ewald_wide(ctx));
 		// the list holds every group (at most one per 32 particles)
-		if (!ctx->wide_list)
-			TVG_CUDA(ctx, cudaMalloc((void **) &ctx->wide_list, 4 * (size_t) (ctx->cap / 32 + 1024)));
+		if (!ctx->wide_list) TVG_CHECK(tvg_alloc(ctx, (void **) &ctx->wide_list, 4 * (size_t) (ctx->cap / 32 + 1024)));
 		TVG_CUDA(ctx, cudaMemsetAsync(ctx->wide_list, 0, 4, s));
 	}
 	if (ewald && !ctx->ewald_taylor) TVG_CHECK(tvg_impl_ewald_taylor(ctx));
@@ -2402,6 +2427,8 @@ static int walk_group_typed(tvg_context *ctx, int use_bh, uint32_t parts, int ew
 	}
 	p.periodic = cf.periodic;
 	p.items = walk_items(cf.periodic, ctx->use_active);
+	p.wide_items = WIDE_ITEMS;
+	part_room(ctx, p, ewald && !mlp);
 	p.use_bh = use_bh;
 	p.open_bundles = (cf.flags & TVG_CFG_OPEN_BUNDLES) ? 1 : 0;
 	p.scale = (float) (cf.periodic ? ctx->dsize / 4294967296.0 : ctx->dsize / 2147483648.0);

@@ -879,7 +879,7 @@ static int walk_typed(tvg_context *ctx, int use_bh, uint32_t parts)
 	c.ew = nullptr;
 	if (parts & TVG_WALK_EWALD) {
 		const int npt = 65 * 65 * 65;
-		if (!ctx->ewald_xyz) TVG_CUDA(ctx, cudaMalloc(&ctx->ewald_xyz, 32 * (size_t) npt));
+		if (!ctx->ewald_xyz) TVG_CHECK(tvg_alloc(ctx, &ctx->ewald_xyz, 32 * (size_t) npt));
 		F *const *f = (F *const *) ctx->ewald_f;
 		k_plain_ewald<<<TVG_CNT(ctx, tvg_blocks(npt, 256)), 256, 0, s>>>(f[0], f[1], f[2], f[3],
 		                                                                 (F *) ctx->ewald_xyz);
