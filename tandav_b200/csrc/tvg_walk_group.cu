@@ -446,6 +446,7 @@ struct GroupParams {
 	float wide_grid;    // node spacings per length of the table for single points
 	float tay_grid;     // Taylor-table node spacings per length (2 (TVG_TAYLOR_NODES - 1) / L)
 	int items;          // items of a split walk (walk_items), 0: no group is split
+	int full_items;     // the same where an active list's groups are at least half full
 	int wide_items;     // the same for the groups with per-target images (k_ewald_wide)
 	double uniform_g;   // G / L^2: times the total mass, the scale of the uniform-background remainder
 };
@@ -1047,19 +1048,32 @@ __device__ void walk_group(const GroupParams &p, SM &S, const tvg_wnode *__restr
 // 1.06 / 1.12 / 1.20, of 72^3 2.9 / 2.9 / 3.1). Those of an isolated halo are
 // lighter: eight (one warp per group / 8, both of 64 particles: box of 32^3 2.40 /
 // 0.36 ms, halo of 3001 0.31 / 0.11, of 100,000 2.6 / 1.9). The groups of an active
-// list may be of any kind, among them light ones, in any number: two (walks of lists,
-// ms with unsplit groups / 2 / 16 a warp: of a clumpy box of 10^6 1000 particles
-// spread 0.10 / 0.10 / 0.25, 100,000 neighbours 0.24 / 0.26 / 0.49; of a 128^3 box
-// 1000 spread 4.7 / 2.3 / 2.2, 20,000 neighbours 5.5 / 1.0 / 1.0; of a halo of 10^6
-// 1000 spread 0.18 / 0.12 / 0.19, 100,000 neighbours 0.35 / 0.30 / 0.42).
+// list may be of any kind, among them light ones, in any number: two, and four in
+// a periodic box where the list fills half of its groups' places (ms with unsplit
+// groups / 2 / 4 / 16 a warp: of a clumpy box of 10^6 1000 particles spread 0.10 / 0.10 /
+// 0.13 / 0.25, 100,000 neighbours 0.24 / 0.26 / 0.30 / 0.49; of a 128^3 box with
+// monopoles 1000 spread 25.6 / 11.7 / 10.9 / 10.4, 300,000 neighbours 64.5 / 64.5 /
+// 55.4 / 54.4; of a halo of 10^6 1000 spread 0.18 / 0.12 / 0.13 / 0.19, 300,000
+// neighbours 0.55 / 0.55 / 0.58 / 0.73).
 #define WALK_WARPS (148 * 16)
 #define WALK_MAX_PARTS 32
-static int walk_items(bool periodic, bool list) { return WALK_WARPS * (list ? 2 : periodic ? 16 : 8); }
 
-__host__ __device__ __forceinline__ int walk_parts(const GroupParams &p, int64_t ngroups)
+__host__ __device__ __forceinline__ int parts_of(int items, int64_t ngroups)
 {
-	const int64_t k = p.items / (ngroups > 0 ? ngroups : 1);
+	const int64_t k = items / (ngroups > 0 ? ngroups : 1);
 	return k < 1 ? 1 : k > WALK_MAX_PARTS ? WALK_MAX_PARTS : (int) k;
+}
+
+static void walk_items(GroupParams &p, bool list)
+{
+	p.items = WALK_WARPS * (list ? 2 : p.periodic ? 16 : 8);
+	p.full_items = WALK_WARPS * (list && p.periodic ? 4 : 0);
+}
+
+__device__ __forceinline__ int walk_parts(const GroupParams &p, int64_t ngroups)
+{
+	const bool full = p.full_items > p.items && 2 * p.dc->n_active >= ngroups * p.gsize;
+	return parts_of(full ? p.full_items : p.items, ngroups);
 }
 
 // The warp's memory. A pop takes at most 1/7 of the stack's free room, so a short
@@ -2262,7 +2276,7 @@ static int launch_walk_q(tvg_context *ctx, GroupParams p, const float *mass_f, c
 // split changes the sums' order (1e-7 of the force).
 static bool may_split(const tvg_context *ctx, const GroupParams &p)
 {
-	return ctx->cfg.float_bytes == 4 && (ctx->use_active || walk_parts(p, (ctx->n + p.gsize - 1) / p.gsize) > 1);
+	return ctx->cfg.float_bytes == 4 && (ctx->use_active || parts_of(p.items, (ctx->n + p.gsize - 1) / p.gsize) > 1);
 }
 
 template <int MODE, int TPL, typename F>
@@ -2354,7 +2368,7 @@ static int launch_pair(tvg_context *ctx, const GroupParams &p, bool ewald, bool 
 static void part_room(tvg_context *ctx, GroupParams &p, bool wide)
 {
 	const int64_t groups = ctx->cap / p.gsize + 1;
-	const int64_t split = may_split(ctx, p) ? std::min<int64_t>(p.items, WALK_MAX_PARTS * groups) : 0;
+	const int64_t split = may_split(ctx, p) ? std::min<int64_t>(std::max(p.items, p.full_items), WALK_MAX_PARTS * groups) : 0;
 	const int64_t images = wide ? std::min<int64_t>(p.wide_items, WIDE_MAX_PARTS * groups) : 0;
 	const size_t need_split = sizeof(PartSum) * (size_t) (split * p.gsize), need_wide = 24 * (size_t) (images * p.gsize);
 	const size_t need = std::max(need_split, need_wide);
@@ -2369,7 +2383,7 @@ static void part_room(tvg_context *ctx, GroupParams &p, bool wide)
 			cudaGetLastError();
 		}
 	}
-	if (need_split > ctx->part_bytes) p.items = 0;
+	if (need_split > ctx->part_bytes) p.items = p.full_items = 0;
 	if (need_wide > ctx->part_bytes) p.wide_items = 0;
 }
 
@@ -2426,7 +2440,7 @@ static int walk_group_typed(tvg_context *ctx, int use_bh, uint32_t parts, int ew
 		TVG_CUDA(ctx, cudaGetLastError());
 	}
 	p.periodic = cf.periodic;
-	p.items = walk_items(cf.periodic, ctx->use_active);
+	walk_items(p, ctx->use_active);
 	p.wide_items = WIDE_ITEMS;
 	part_room(ctx, p, ewald && !mlp);
 	p.use_bh = use_bh;

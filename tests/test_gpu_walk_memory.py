@@ -67,7 +67,7 @@ def test_walk_without_memory_for_the_parts():
     torch.cuda.empty_cache()
     before = free()
     ctx.walk(G.FORM_GROUP, use_bh=False, parts=parts)
-    assert before - free() > 60 * MB
+    assert before - free() > 40 * MB             # more than was left before
     split = ctx.download(fields)
     ctx.close()
     np.testing.assert_array_equal(one["cost"], split["cost"])
