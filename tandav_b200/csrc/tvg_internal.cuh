@@ -195,6 +195,7 @@ struct tvg_context {
 	int32_t *wide_list = nullptr;      // groups that take per-target images (k_ewald_wide)
 	void *part_sums = nullptr;         // sums of the parts of split groups (both group walks)
 	size_t part_bytes = 0;
+	bool tune_all = false;             // tvg_autotune times a sample of all particles
 	float *ewald_taylor = nullptr;     // T and 3 derivatives at TVG_TAYLOR_NODES^3 nodes, 32 floats each
 	// Ewald-walk opening of the group form: the monopole error of the
 	// correction may reach ewald_open_rel |a_old| (relative mode); the limit of
