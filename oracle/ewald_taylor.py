@@ -2,7 +2,8 @@
 (tandav_b200/csrc/tvg_ewald.cu: k_ewald_fine, k_ewald_taylor,
 k_ewald_wide_table; the lookups in tandav_b200/csrc/tvg_walk_group.cu:
 ewald_kjh, ewald_k). `record` takes the derivatives component by component;
-the tables hold its symmetric part (`tensors`, `compact`).
+the tables hold its symmetric part (`tensors`, completed by `lookup`, and
+`compact`).
 
 TEST INFRASTRUCTURE ONLY: it checks the scheme (finite differences on a
 grid of half the node spacing, third-order expansion about the nearest node)
@@ -97,8 +98,9 @@ def evaluate(rec, du):
 
 
 def tensors(rec):
-    """dT, d2T and d3T of a record, each averaged over its index permutations
-    (T is a gradient): what a 32-float record of the table holds."""
+    """T, dT, d2T and d3T of a record, the derivatives averaged over their index
+    permutations (T is a gradient). A 32-float record of the table holds all of
+    dT and d2T and twelve entries of d3T; `lookup` fills in the rest."""
     B, C, D = np.zeros((3, 3)), np.zeros((3, 3, 3)), np.zeros((3, 3, 3, 3))
     t3 = ("xxx", "yyy", "zzz", "xxy", "xxz", "xyy", "yyz", "xzz", "yzz", "xyz")
     for a in range(3):
@@ -116,6 +118,16 @@ def tensors(rec):
         return sum(np.transpose(t, p) for p in perms) / len(perms)
 
     return rec[0::20][:3], mean(B), mean(C), mean(D)
+
+
+def lookup(t):
+    """The tensors with d3T as the 33-node lookup takes it: xyzz, xzzz and yzzz
+    from the zero trace."""
+    T, B, C, D = t[0], t[1], t[2], t[3].copy()
+    for a, b in ((0, 1), (0, 2), (1, 2)):
+        for idx in set(itertools.permutations((a, b, 2, 2))):
+            D[idx] = -D[a, b, 0, 0] - D[a, b, 1, 1]
+    return T, B, C, D
 
 
 def compact(rec, nodes):
