@@ -3,13 +3,16 @@ TVG_CFG_FIX_SMALL_TOPNODES a small top node's particles are taken from its
 Target on, a running node count: with bundles of one particle the nodes
 outnumber the particles and Target passes the last of them. What lies there
 counts as a massless particle at the origin, whatever the capacity and whatever
-an earlier, larger upload left behind."""
+an earlier, larger upload left behind. Where the box side is a float, FP32 bundles
+that reach the half-box plane wrap in float (gravity_run); where it is not, they
+take the general form."""
 import numpy as np
 import pytest
 
 import port
+from pipeline import oracle_ewald_tables, oracle_pipeline
 from tandav_b200 import gravity as G
-from test_gpu_parity import reference_table
+from test_gpu_parity import gpu_pipeline, reference_table, walks
 
 pytestmark = pytest.mark.gpu
 
@@ -82,3 +85,22 @@ def test_small_top_nodes_past_the_last_particle(fsize, use_bh, periodic):
     np.testing.assert_array_equal(out[0]["cost"], cost)
     np.testing.assert_array_equal(out[0]["grav_acc"], acc)
     np.testing.assert_array_equal(out[0]["grav_pot"], pot)
+
+
+@pytest.mark.parametrize("box", [1000.0, 1000.1])
+def test_bundles_across_the_half_box_plane(box):
+    """FP32 boxes whose bundles of up to 64 particles are wide enough for many of
+    them to straddle a target's half-box plane: force and count bit for bit."""
+    rng = np.random.default_rng(8)
+    n = 4003
+    pos = rng.uniform(0.0, 999.9, (3, n)).astype(np.float32)
+    mass = rng.uniform(0.5, 1.5, n)
+    o = oracle_pipeline(pos, mass, np.zeros(3), box, 4, box=box, softening=2.0,
+                        ewald=oracle_ewald_tables(4, box))
+    with G.GravityContext(n, periodic=True, boxsize=box, gravity=43007.1, softening=2.0) as ctx:
+        perm, _, _, _ = gpu_pipeline(ctx, pos, mass, np.zeros(3), box)
+        assert np.array_equal(perm, o["perm"])
+        bh, _, rel = walks(ctx, True, 4)
+    for name, got in (("bh", bh), ("rel", rel)):
+        np.testing.assert_array_equal(got["cost"], o[name + "_cost"])
+        np.testing.assert_array_equal(got["grav_acc"], o[name + "_gacc"])
