@@ -790,7 +790,7 @@ def main():
             "ewald_walk": {"kernel": f"k_ewald_group<{tune_choice}, false, float>",
                            "ms_per_step": round(ew_ms / args.steps, 2),
                            "evaluations_per_group": round(ew_i / args.steps / (n / (32 * tune_choice)), 1),
-                           "evaluation": "Taylor-table K, dK, d2K: 8 float4 loads, ~200 FP32 ops"},
+                           "evaluation": "Taylor-table K, dK, d2K: four 32-byte loads, ~200 FP32 ops"},
             "plain_form": plain,
             "group_form_monopole": monopole,
             "group_form_at_plain_opening": matched,

@@ -152,9 +152,10 @@ __device__ __forceinline__ FineDiff fine_diff(const double *fine, int nodes, int
 //   d3T xxxx yyyy zzzz xxyy xxzz yyzz xxxy xxxz xyyy yyyz xxyz xyyz (xyzz, xzzz and yzzz
 //   from the zero trace), 0.
 // A lookup expands T about the nearest node (|du| <= 1/2 per axis): T to third
-// order, dT to second, d2T to first. With 33 nodes (spacing 1/64) the value is
-// within 4e-7 of |T| and the gradient within 4e-5 rms of direct lattice sums at
-// off-node points across the octant.
+// order, dT to second, d2T to first. With 33 nodes (spacing 1/64), at 400 random
+// points of the octant against direct lattice sums: the value within 4.8e-7 of |T|,
+// the gradient within 4.2e-5 of its largest component (the derivatives component by
+// component, 60 floats: 5.8e-7 and 4.2e-5).
 __global__ void k_ewald_taylor(const double *__restrict__ fine, float *tay)
 {
 	const int idx = blockIdx.x * blockDim.x + threadIdx.x;

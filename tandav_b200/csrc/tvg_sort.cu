@@ -3,7 +3,9 @@
 // Replaces Qsort_Index on the 128-bit keys (sort.c:90-341, cmp_peanoKeys at
 // peano.c:6-12) and reorder_collisionless_particles (peano.c:50-82).
 //  1. LSD radix sort of (key_hi, index) on the 64-bit high key word: 8-bit
-//     digits, one kernel per digit (k_radix_pass). All eight digit histograms are
+//     digits, one kernel per digit (k_radix_pass), the published one-sweep form
+//     (Adinets and Merrill 2022) with decoupled look-back over the tiles' counts
+//     (Merrill and Garland 2016). All eight digit histograms are
 //     counted in one pass over the keys beforehand; a pass takes tiles of 4096 keys
 //     (few keys: 1024) in the order of a device counter, ranks a tile's keys
 //     stably with warp ballots, finds the tile's place among the equal digits of
@@ -14,9 +16,9 @@
 //     the keys through, so the number of passes, and with it the buffer a step
 //     ends in, never depends on the data. Up to one tile of keys is sorted by one
 //     block in shared memory (k_sort_tile).
-//  2. Runs of equal high words are ordered by the low word (insertion sort
-//     per run, one thread per run; runs are rare and short unless positions
-//     coincide).
+//  2. Runs of equal high words are ordered by the low word (k_tie_rank: a thread
+//     per key of a run counts the run's keys that precede it, r loads each in a
+//     run of r; runs are rare and short unless positions coincide).
 //  3. Every particle field is gathered through the permutation in one launch,
 //     four particles per thread with 128-bit stores (and 128-bit loads where
 //     the permutation keeps an aligned run of four in place).
@@ -27,9 +29,10 @@
 // and scatter kernels per digit (three to five launches, 20 B read) took, with
 // the gather of the fields, 4.65 ms for 16.7M particles, 0.47 ms for 400,000,
 // 0.27 ms for 32,768 and 0.28 ms for 3001; this 2.44, 0.20, 0.10 and 0.06 ms. A
-// pass over many keys waits on shared memory (ranking and staging, 16 keys a
-// thread) at the 32 warps an SM holds (4M keys: 61 us, 0.9 TB/s of DRAM traffic,
-// as the L2 holds both buffers).
+// pass over many keys waits on memory (of 15 stall cycles an instruction 4.3 on
+// global loads, keys and look-back, and 2.1 on shared memory) at 29 of the 32 warps
+// an SM holds (4M keys: 56 us, 0.95 TB/s of DRAM traffic, as the L2 holds much of
+// both buffers).
 #include <mutex>
 
 #include "tvg_internal.cuh"
@@ -500,8 +503,9 @@ int tvg_impl_sort(tvg_context *ctx, uint32_t *perm_out)
 //
 // The array belongs to every GPU that loads this library, for the life of the
 // process (about 6.4 MB). All calls on a device share it and it keeps the
-// last call's contents: a call zeroes the counts and states it starts from. Two calls that overlap on the same GPU (from
-// two host threads, or on two streams) corrupt each other's scratch.
+// last call's contents: a call zeroes the counts and states it starts from. Two
+// calls that overlap on the same GPU (from two host threads, or on two streams)
+// corrupt each other's scratch.
 // ------------------------------------------------------------------------
 
 #define NOALLOC_TILES (TVG_NOALLOC_MAX_KEYS / RS_TILE)

@@ -1083,7 +1083,7 @@ __device__ __forceinline__ int walk_parts(const GroupParams &p, int64_t ngroups)
 // 148.0 ms with 1024 entries + 256 sources, 146.1 with 1536 + 128 (768 + 128:
 // 184; 1024 + 64: 149.2; 2048 + 128: 145.8, but 12.6 instead of 12.4 ms on the
 // 100^3 box). FP64 contexts keep the flush points of the longer lists, and with
-// them the bits of their sums.
+// them the bits of the gravity walk's sums.
 #define GW_STACK_QUAD 1536
 #define GW_LIST_QUAD 128
 template <typename F, bool QUAD> struct walk_smem_of { typedef WarpSmem type; };
@@ -1935,7 +1935,7 @@ __device__ void ewald_wide_item(const GroupParams &p, EwaldSmem &S, const tvg_wn
 		if (accept) S.list[nl + __popc(bm & lt)] = entry;
 		nl += __popc(bm);               // below 64: fewer than 32 were left
 		push_children(S.stack, sp, open_int, nchild, child);
-			const unsigned bb = __ballot_sync(0xFFFFFFFFu, open_bundle);
+		const unsigned bb = __ballot_sync(0xFFFFFFFFu, open_bundle);
 		if (open_bundle) S.bq[__popc(bb & lt)] = make_int2(child, nchild);
 		__syncwarp();
 		if (nl >= 32) {
@@ -2273,7 +2273,8 @@ static int launch_walk_q(tvg_context *ctx, GroupParams p, const float *mass_f, c
 // Whether the groups may be split: from the number of groups, or, for an active
 // list, whose length the device knows, always (its kernels then decide). FP64
 // contexts keep a warp per group: they return the FP32 sums at full width, and a
-// split changes the sums' order (1e-7 of the force).
+// split changes the sums' order (1e-7 of the force; only the groups with per-target
+// images, k_ewald_wide, are split there).
 static bool may_split(const tvg_context *ctx, const GroupParams &p)
 {
 	return ctx->cfg.float_bytes == 4 && (ctx->use_active || parts_of(p.items, (ctx->n + p.gsize - 1) / p.gsize) > 1);

@@ -23,8 +23,8 @@
 // packed load (position and the rounded G m), a node one record (the left side
 // of its test, its thresholds), a comparison of a float with a double
 // threshold is one of floats (the threshold rounded so that every float
-// compares alike), and the Ewald tables are interleaved so that a corner is
-// one load for the three components.
+// compares alike), and the Ewald tables are interleaved so that one load
+// brings the components of a corner (FP32: of two).
 //
 // A warp's 32 targets walk the tree together: every lane keeps the node it
 // goes to next, the warp visits the smallest of them, and the lanes that are
